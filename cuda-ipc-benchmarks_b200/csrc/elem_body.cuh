@@ -7,6 +7,7 @@
 #include <climits>
 
 #include "elem_math.cuh"
+#include "elem_modal.cuh"
 #include "kernels.cuh"
 
 namespace lulesh {
@@ -80,77 +81,52 @@ __device__ __forceinline__ void elem_nodes(const DomDev &D, int el, int n[8])
     n[7] = n0 + en * en + en;
 }
 
-// CalcVolumeForceForElems_kernel (lulesh.cu:2080-2259) after the node
-// gathers: stress + FB hourglass corner forces of element `elem`, handed
-// to store(k, fx, fy, fz) corner by corner.  The velocities are fetched
-// from `vel` only when HG (hourglass coefficient > 0).
-template <bool HG, class Vel, class Store>
-__device__ __forceinline__ void force_elem_to(const DomDev &D, TimeCtl &T, const Params &P,
-                                              int elem, const double (&xn)[8],
-                                              const double (&yn)[8], const double (&zn)[8],
-                                              const Vel &vel, const Store &store)
+// CalcVolumeForceForElems_kernel (lulesh.cu:2080-2259) after the coordinate
+// gathers, in the element's modes (elem_modal.cuh): stress + FB hourglass
+// corner forces, one component at a time, handed to store(component, f[8]).
+// vel(component, v[8]) gives the corner velocities, asked for only when HG
+// (hourglass coefficient > 0); elem_error() is called when the volume or the
+// centre Jacobian is negative.
+//
+// A component needs the geometry (78 registers of it) and its own eight
+// velocities, nothing of the other components, so the three run one after the
+// other in few registers.
+template <bool HG, class Vel, class Store, class Error>
+__device__ __forceinline__ void force_modal(const double (&xn)[8], const double (&yn)[8],
+                                            const double (&zn)[8], double volo, double v, double p,
+                                            double q, double ss, double mass, double hourg,
+                                            const Vel &vel, const Store &store,
+                                            const Error &elem_error)
 {
-    double dvdxn[8], dvdyn[8], dvdzn[8];
-    double hgfx[8], hgfy[8], hgfz[8];
-    double hourgam[8][4];
-
-    const double volume = D.v[elem];
-    double det = D.volo[elem] * volume;
-    if (volume < 0.) atomicMin(&T.bad_vol, elem);
-    const double ss1 = D.ss[elem];
-    const double mass1 = D.elemMass[elem];
-    const double sigxx = -D.p[elem] - D.q[elem];
-    const double volinv = 1.0 / det;
-
-    const double hourg = P.hgcoef;
-    const double volume13 = cbrt(det);
-    const double coefficient = -hourg * 0.01 * ss1 * mass1 / volume13;
-
-    elem_volume_derivative(dvdxn, dvdyn, dvdzn, xn, yn, zn);
-    hourglass_modes(xn, yn, zn, dvdxn, dvdyn, dvdzn, hourgam, volinv);
-
-    double B[3][8];
-    shape_function_derivatives(xn, yn, zn, B, &det);
-    elem_node_normals(B[0], B[1], B[2], xn, yn, zn);
-    if (det < 0.) atomicMin(&T.bad_vol, elem);
-
+    ElemModes<double> m;
+    elem_modes(xn, yn, zn, m);
+    ForceGeometry<double> g;
+    force_geometry<double, HG>(m, g);
+    const double det = volo * v;
+    if (v < 0. || g.det < 0.) elem_error();
+    const double press = (p + q) * (1.0 / 64.0);
+    const double vol64 = (1.0 / 64.0) / det;
+    const double coef = HG ? -hourg * 0.01 * ss * mass * rcbrt(det) : 0.0;
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        hgfx[i] = -(sigxx * B[0][i]);
-        hgfy[i] = -(sigxx * B[1][i]);
-        hgfz[i] = -(sigxx * B[2][i]);
+    for (int c = 0; c < 3; ++c) {
+        double vc[8], f[8];
+        if (HG) vel(c, vc);
+        force_component<double, HG>(m, g, c, vc, press, vol64, coef, f);
+        store(c, f);
     }
-    if (HG) {
-        double xdn[8], ydn[8], zdn[8];
-        vel.fetch(xdn, ydn, zdn);
-        fb_hourglass_component(xdn, hourgam, coefficient, hgfx);
-        fb_hourglass_component(ydn, hourgam, coefficient, hgfy);
-        fb_hourglass_component(zdn, hourgam, coefficient, hgfz);
-    }
-#pragma unroll
-    for (int k = 0; k < 8; ++k) store(k, hgfx[k], hgfy[k], hgfz[k]);
 }
 
 // the corner arrays at elem + Ep * corner
 struct CornerStore {
-    const DomDev &D;
-    int elem;
-    __device__ __forceinline__ void operator()(int k, double fx, double fy, double fz) const
+    double *fx, *fy, *fz;
+    int elem, Ep;
+    __device__ __forceinline__ void operator()(int c, const double (&f)[8]) const
     {
-        const int c = elem + D.Ep * k;
-        st_corner(D.fx_elem + c, fx);
-        st_corner(D.fy_elem + c, fy);
-        st_corner(D.fz_elem + c, fz);
+        double *p = (c == 0 ? fx : c == 1 ? fy : fz) + elem;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) st_corner(p + Ep * k, f[k]);
     }
 };
-
-template <bool HG, class Vel>
-__device__ __forceinline__ void force_elem(const DomDev &D, TimeCtl &T, const Params &P, int elem,
-                                           const double (&xn)[8], const double (&yn)[8],
-                                           const double (&zn)[8], const Vel &vel)
-{
-    force_elem_to<HG>(D, T, P, elem, xn, yn, zn, vel, CornerStore{D, elem});
-}
 
 // CalcKinematicsAndMonotonicQGradient_kernel (lulesh.cu:3343-3507) after
 // the node gathers, for element k.

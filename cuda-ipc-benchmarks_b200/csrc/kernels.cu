@@ -129,37 +129,51 @@ __device__ __constant__ int kCZ[8] = {0, 0, 0, 0, 1, 1, 1, 1};
 // ---------------------------------------------------------------------------
 // force: CalcVolumeForceForElems_kernel, lulesh.cu:2080-2259
 
-// one element of the force phase: the node gathers, then force_elem
+// One element of the force phase: the node gathers, then force_modal.
+//
+// Bound by the corner stores (192 B of the 290 B an element moves) and by
+// FP64 issue, about evenly: 70 us at -s 100 (1.0e6 elements) on B200, where
+// the stores and loads take 44 us at the measured copy rate and the ~600
+// operations 32 us at the FP64 peak.  The form that evaluated the reference's
+// expressions corner by corner took 125 us (934 operations, 254 registers,
+// 8 warps per SM).  All 48 gathers go out before any arithmetic: with the
+// velocities gathered component by component, where force_modal asks for
+// them, the kernel fits 128 registers (16 warps) but takes 73 us, and 312
+// against 272 us at -s 160.
 template <bool HG, bool U>
 __device__ __forceinline__ void force_one(const DomDev &D, TimeCtl &T, const Params &P, int elem)
 {
-    // all 48 node gathers are issued before any arithmetic: the velocity
-    // loads then overlap the coordinate work instead of stalling the
-    // hourglass step (measured on B200 at -s 100: 150 -> 136 us)
     int n[8];
     elem_nodes<U>(D, elem, n);
 #pragma unroll
     for (int i = 0; i < 8; ++i) n[i] = chk_index(n[i], D.numNode, &T, kChkNode);
-    double xn[8], yn[8], zn[8];
-    double xdn[8], ydn[8], zdn[8];
+    double vn[3][8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
         if (HG) {
-            xdn[i] = D.xd[n[i]];
-            ydn[i] = D.yd[n[i]];
-            zdn[i] = D.zd[n[i]];
+            vn[0][i] = D.xd[n[i]];
+            vn[1][i] = D.yd[n[i]];
+            vn[2][i] = D.zd[n[i]];
         } else {
-            xdn[i] = ydn[i] = zdn[i] = 0.0;
+            vn[0][i] = vn[1][i] = vn[2][i] = 0.0;
         }
     }
-    const VelRegs vel{xdn, ydn, zdn};
+    double xn[8], yn[8], zn[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) xn[i] = D.x[n[i]];
 #pragma unroll
     for (int i = 0; i < 8; ++i) yn[i] = D.y[n[i]];
 #pragma unroll
     for (int i = 0; i < 8; ++i) zn[i] = D.z[n[i]];
-    force_elem<HG>(D, T, P, elem, xn, yn, zn, vel);
+    force_modal<HG>(
+        xn, yn, zn, D.volo[elem], D.v[elem], D.p[elem], D.q[elem], D.ss[elem], D.elemMass[elem],
+        P.hgcoef,
+        [&](int c, double (&v)[8]) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) v[i] = vn[c][i];
+        },
+        CornerStore{D.fx_elem, D.fy_elem, D.fz_elem, elem, D.Ep},
+        [&] { atomicMin(&T.bad_vol, elem); });
 }
 
 template <bool HG, int BS, bool U>

@@ -21,7 +21,7 @@
 #include <mutex>
 #include <string>
 
-#include "elem_math.cuh"
+#include "elem_body.cuh"
 #include "lulesh_b200.h"
 #include "set.hpp"
 
@@ -60,51 +60,25 @@ __global__ void __launch_bounds__(kBlock)
     const int n[8] = {n0, n0 + 1, n0 + en + 1, n0 + en, n0 + en * en, n0 + en * en + 1,
                       n0 + en * en + en + 1, n0 + en * en + en};
 
-    double xn[8], yn[8], zn[8], dvdxn[8], dvdyn[8], dvdzn[8];
-    double hgfx[8], hgfy[8], hgfz[8], hourgam[8][4], B[3][8];
-    const double volume = v[elem];
-    double det = volo[elem] * volume;
-    if (volume < 0.) atomicMin(flag, elem);
-    const double ss1 = ss[elem], mass1 = elemMass[elem];
-    const double sigxx = -p[elem] - q[elem];
-    const double volinv = 1.0 / det;
+    double xn[8], yn[8], zn[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
         xn[i] = x[n[i]];
         yn[i] = y[n[i]];
         zn[i] = z[n[i]];
     }
-    const double volume13 = cbrt(det);
-    const double coefficient = -hourg * 0.01 * ss1 * mass1 / volume13;
-    lulesh::elem_volume_derivative(dvdxn, dvdyn, dvdzn, xn, yn, zn);
-    lulesh::hourglass_modes(xn, yn, zn, dvdxn, dvdyn, dvdzn, hourgam, volinv);
-    lulesh::shape_function_derivatives(xn, yn, zn, B, &det);
-    lulesh::elem_node_normals(B[0], B[1], B[2], xn, yn, zn);
-    if (det < 0.) atomicMin(flag, elem);
+    lulesh::force_modal<HG>(
+        xn, yn, zn, volo[elem], v[elem], p[elem], q[elem], ss[elem], elemMass[elem], hourg,
+        [&](int c, double (&vel)[8]) {
+            const double *a = c == 0 ? xd : c == 1 ? yd : zd;
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        hgfx[i] = -(sigxx * B[0][i]);
-        hgfy[i] = -(sigxx * B[1][i]);
-        hgfz[i] = -(sigxx * B[2][i]);
-    }
-    if (HG) {
-        double vel[8];
+            for (int i = 0; i < 8; ++i) vel[i] = a[n[i]];
+        },
+        [&](int c, const double (&f)[8]) {
 #pragma unroll
-        for (int i = 0; i < 8; ++i) vel[i] = xd[n[i]];
-        lulesh::fb_hourglass_component(vel, hourgam, coefficient, hgfx);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) vel[i] = yd[n[i]];
-        lulesh::fb_hourglass_component(vel, hourgam, coefficient, hgfy);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) vel[i] = zd[n[i]];
-        lulesh::fb_hourglass_component(vel, hourgam, coefficient, hgfz);
-    }
-#pragma unroll
-    for (int k = 0; k < 8; ++k) {
-        corners[(0 * 8 + k) * Ep + elem] = hgfx[k];
-        corners[(1 * 8 + k) * Ep + elem] = hgfy[k];
-        corners[(2 * 8 + k) * Ep + elem] = hgfz[k];
-    }
+            for (int k = 0; k < 8; ++k) corners[(c * 8 + k) * Ep + elem] = f[k];
+        },
+        [&] { atomicMin(flag, elem); });
 }
 
 // per-node sum of the surrounding corners in corner order 0..7 (the
