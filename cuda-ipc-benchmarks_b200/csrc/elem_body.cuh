@@ -37,23 +37,6 @@ __device__ __forceinline__ double ld_corner(const double *p)
 #endif
 }
 
-// Velocities gathered into registers at kernel start, handed to the body
-// where its arithmetic first needs them.
-struct VelRegs {
-    const double (&xd)[8];
-    const double (&yd)[8];
-    const double (&zd)[8];
-    __device__ __forceinline__ void fetch(double (&x)[8], double (&y)[8], double (&z)[8]) const
-    {
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            x[i] = xd[i];
-            y[i] = yd[i];
-            z[i] = zd[i];
-        }
-    }
-};
-
 // The eight node indices of element el on the structured mesh, in the
 // nodelist order of BuildMesh (lulesh.cu:730-737): corner j sits at lattice
 // offset (x: bits 0x66, y: 0xCC, z: 0xF0 of j) from corner 0.
@@ -129,54 +112,46 @@ struct CornerStore {
 };
 
 // CalcKinematicsAndMonotonicQGradient_kernel (lulesh.cu:3343-3507) after
-// the node gathers, for element k.
+// the coordinate gathers, for element k, in the element's modes.  The
+// velocities enter through their A, B, C modes only; vel(component, v[8])
+// gives the corner values.  The monotonic-Q gradients are those of the
+// coordinates themselves (the reference shifts them by half a step and back).
 template <class Vel>
-__device__ __forceinline__ void kin_elem(const DomDev &D, TimeCtl &T, int k, double (&x_local)[8],
-                                         double (&y_local)[8], double (&z_local)[8],
-                                         const Vel &vel)
+__device__ __forceinline__ void kin_modal(const DomDev &D, TimeCtl &T, int k,
+                                          const double (&xn)[8], const double (&yn)[8],
+                                          const double (&zn)[8], const Vel &vel)
 {
-    double B[3][8];
-    double Dv[3];
-    const double volume = elem_volume(x_local, y_local, z_local);
+    ElemModes<double> m;
+    elem_modes(xn, yn, zn, m);
+    FaceCrosses<double> c;
+    face_crosses(m, c);
+    const double volume = modal_volume(m, c);
     const double relativeVolume = volume / D.volo[k];
     D.vnew[k] = relativeVolume;
     D.delv[k] = relativeVolume - D.v[k];
-    D.arealg[k] = elem_characteristic_length(x_local, y_local, z_local, volume);
-
-    double xd_local[8], yd_local[8], zd_local[8];
-    vel.fetch(xd_local, yd_local, zd_local);
-    const double dt2 = 0.5 * T.deltatime;
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-        x_local[j] -= dt2 * xd_local[j];
-        y_local[j] -= dt2 * yd_local[j];
-        z_local[j] -= dt2 * zd_local[j];
-    }
-    double detJ;
-    shape_function_derivatives(x_local, y_local, z_local, B, &detJ);
-    elem_velocity_divergence(xd_local, yd_local, zd_local, B, detJ, Dv);
-    const double vdovNew = Dv[0] + Dv[1] + Dv[2];
-    D.vdov[k] = vdovNew;
-
-    const double vol = D.volo[k] * relativeVolume;
-    // undo the half-step shift exactly as the reference does (the restored
-    // coordinates can differ from the originals in the last bit)
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-        x_local[j] += dt2 * xd_local[j];
-        y_local[j] += dt2 * yd_local[j];
-        z_local[j] += dt2 * zd_local[j];
-    }
-    double dxz, dvz, dxx, dvx, dxe, dve;
-    mono_gradient(x_local, y_local, z_local, xd_local, yd_local, zd_local, vol, &dxz, &dvz,
-                  &dxx, &dvx, &dxe, &dve);
-    D.delx_zeta[k] = dxz;
-    D.delv_zeta[k] = dvz;
-    D.delx_xi[k] = dxx;
-    D.delv_xi[k] = dvx;
-    D.delx_eta[k] = dxe;
-    D.delv_eta[k] = dve;
     if (relativeVolume < 0) atomicMin(&T.bad_vol, k);
+    D.arealg[k] = modal_length(m, c, volume);
+
+    double va[3], vb[3], vc[3];
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        double v[8], vg;
+        vel(i, v);
+        odd_modes(v, va[i], vb[i], vc[i], vg);
+    }
+    D.vdov[k] = modal_divergence(m, va, vb, vc, 0.5 * T.deltatime);
+
+    const double norm = 1.0 / (volume + 1.e-36);
+    double delx, delv;
+    modal_mono(c.ab, vc, volume, norm, &delx, &delv);
+    D.delx_zeta[k] = delx;
+    D.delv_zeta[k] = delv;
+    modal_mono(c.bc, va, volume, norm, &delx, &delv);
+    D.delx_xi[k] = delx;
+    D.delv_xi[k] = delv;
+    modal_mono(c.ca, vb, volume, norm, &delx, &delv);
+    D.delx_eta[k] = delx;
+    D.delv_eta[k] = delv;
 }
 
 }  // namespace lulesh

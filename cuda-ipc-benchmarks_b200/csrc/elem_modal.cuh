@@ -24,13 +24,23 @@
 // Coordinates enter through differences of corners only (diagonals for A, B,
 // C, G; edges for D, E, F), so no sum of coordinates near 1 is rounded.
 // Every product that feeds a sum is an explicit fma: the bits do not depend
-// on the kernel the functions are inlined into.
+// on the kernel the functions are inlined into.  The modes, the crosses and
+// the kinematics' cancelling sums give the same bits with x and y (and xi and
+// eta) exchanged, as the problem does: the symmetry check of a run compares
+// elements across that diagonal, and its largest relative difference at
+// -s 100 after 505 cycles is 5e-14 this way and 8e-12 with dot3 throughout,
+// for 0 of 225 us a cycle.
 #pragma once
 
 namespace lulesh {
 
 __device__ __forceinline__ double fma_t(double a, double b, double c) { return fma(a, b, c); }
 __device__ __forceinline__ float fma_t(float a, float b, float c) { return fmaf(a, b, c); }
+// a sum and a product that no compiler joins into one fma
+__device__ __forceinline__ double sum_rn(double a, double b) { return __dadd_rn(a, b); }
+__device__ __forceinline__ float sum_rn(float a, float b) { return __fadd_rn(a, b); }
+__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
 __device__ __forceinline__ double rsqrt_t(double a) { return rsqrt(a); }
 __device__ __forceinline__ float rsqrt_t(float a) { return rsqrtf(a); }
 __device__ __forceinline__ double rcbrt_t(double a) { return rcbrt(a); }
@@ -65,17 +75,24 @@ __device__ __forceinline__ T dot3(const T a[3], const T b[3])
     return fma_t(a[0], b[0], fma_t(a[1], b[1], a[2] * b[2]));
 }
 
+// a . b, the same bits with x and y exchanged
+template <typename T>
+__device__ __forceinline__ T dot3_sym(const T a[3], const T b[3])
+{
+    return fma_t(a[2], b[2], sum_rn(mul_rn(a[0], b[0]), mul_rn(a[1], b[1])));
+}
+
 // A, B, C and G of one component from its diagonals (n6-n0, n7-n1, n4-n2,
 // n5-n3)
 template <typename T>
 __device__ __forceinline__ void odd_modes(const T v[8], T &a, T &b, T &c, T &g)
 {
     const T u0 = v[6] - v[0], u1 = v[7] - v[1], u2 = v[4] - v[2], u3 = v[5] - v[3];
-    const T s = u0 + u3, t = u1 + u2, p = u0 - u3, q = u1 - u2;
-    a = s - t;  // u0 - u1 - u2 + u3
+    const T p = u0 - u2, q = u1 - u3, s = u0 + u2, t = u1 + u3;
+    a = p - q;
+    b = p + q;
     c = s + t;
-    b = p + q;  // u0 + u1 - u2 - u3
-    g = p - q;  // u0 - u1 + u2 - u3
+    g = s - t;
 }
 
 // D, E, F of one component from its edges
@@ -87,7 +104,7 @@ __device__ __forceinline__ void even_modes(const T v[8], T &d, T &e, T &f)
     d = s + t;
     f = s - t;
     const T p0 = v[1] - v[0], p1 = v[2] - v[3], p2 = v[5] - v[4], p3 = v[6] - v[7];
-    e = (p2 - p0) + (p3 - p1);
+    e = (p3 - p0) + (p2 - p1);
 }
 
 // Modes of one element's coordinates, [component] each.
@@ -236,8 +253,8 @@ __device__ __forceinline__ void force_component(const ElemModes<T> &m, const For
 template <typename T>
 __device__ __forceinline__ T modal_volume(const ElemModes<T> &m, const FaceCrosses<T> &c)
 {
-    const T h = dot3(m.A, c.fe) + (dot3(m.B, c.df) + dot3(m.C, c.ed));
-    return T(1.0 / 64.0) * fma_t(T(1.0) / T(3.0), h, dot3(m.A, c.bc));
+    const T h = (dot3_sym(m.A, c.fe) + dot3_sym(m.B, c.df)) + dot3_sym(m.C, c.ed);
+    return T(1.0 / 64.0) * fma_t(T(1.0) / T(3.0), h, dot3_sym(m.C, c.ab));
 }
 
 // The larger |N + M|^2, |N - M|^2 of a pair of opposite faces
@@ -260,7 +277,7 @@ __device__ __forceinline__ T modal_length(const ElemModes<T> &m, const FaceCross
 {
     T ma[3], mb[3], mc[3];
     cross2(m.B, m.E, m.F, m.C, ma);
-    cross2(m.C, m.F, m.D, m.A, mb);
+    cross2(m.D, m.A, m.C, m.F, mb);
 #pragma unroll
     for (int i = 0; i < 3; ++i) mc[i] = -(ma[i] + mb[i]);
     T area = fmax_t(larger_face(c.bc, c.fe, ma), T(0.0));
@@ -286,7 +303,7 @@ __device__ __forceinline__ T modal_divergence(const ElemModes<T> &m, const T va[
     cross(b, c, bc);
     cross(c, a, ca);
     cross(a, b, ab);
-    return (dot3(bc, va) + dot3(ca, vb) + dot3(ab, vc)) / dot3(a, bc);
+    return ((dot3_sym(bc, va) + dot3_sym(ca, vb)) + dot3_sym(ab, vc)) / dot3_sym(c, ab);
 }
 
 // One direction of CalcMonoGradient (lulesh.cu:3251-3334): n the cross of
@@ -297,7 +314,7 @@ __device__ __forceinline__ void modal_mono(const T n[3], const T v[3], T volume,
 {
     const T ptiny = T(1.e-36);
     *delx = (T(16.0) * volume) * rsqrt_t(dot3(n, n) + T(256.0) * ptiny);
-    *delv = (T(1.0 / 64.0) * norm) * dot3(n, v);
+    *delv = (T(1.0 / 64.0) * norm) * dot3_sym(n, v);
 }
 
 }  // namespace lulesh

@@ -487,6 +487,14 @@ void launch_nodal_update(const SetArgs &a, int nblocks, Params P, cudaStream_t s
 // ---------------------------------------------------------------------------
 // kinematics: CalcKinematicsAndMonotonicQGradient_kernel, lulesh.cu:3343-3507
 
+// Bound by latency and FP64 issue at 20 warps per SM: 51.6 us at -s 100
+// (1.0e6 elements) on B200, against 22 us for its 144 B per element at the
+// measured copy rate and 19 us for its ~360 operations; 80 us with the
+// reference's corner-by-corner expressions (649 operations, 168 registers).
+// The velocities are gathered where kin_modal asks for them, after the volume
+// and length stores, at 96 registers (5 blocks); 57.8 us at 4 blocks.  Up
+// front took 8 us more at 3 blocks, and between the coordinates and the volume
+// 2 us more at 4 blocks and 4 at 5 (with spills).
 template <int BS, bool U = false>
 __global__ void __launch_bounds__(BS, min_blocks(kKinMinBlocks, BS)) k_kinematics(SetArgs a)
 {
@@ -498,27 +506,22 @@ __global__ void __launch_bounds__(BS, min_blocks(kKinMinBlocks, BS)) k_kinematic
     const int k = blk.y + threadIdx.x;
     if (k >= D.numElem) return;
 
-    // all node gathers first (measured on B200 at -s 100: 92 -> 84 us)
-    int nodes[8];
-    elem_nodes<U>(D, k, nodes);
+    int n[8];
+    elem_nodes<U>(D, k, n);
 #pragma unroll
-    for (int l = 0; l < 8; ++l) nodes[l] = chk_index(nodes[l], D.numNode, &T, kChkNode);
-    double x_local[8], y_local[8], z_local[8];
-    double xd_local[8], yd_local[8], zd_local[8];
+    for (int l = 0; l < 8; ++l) n[l] = chk_index(n[l], D.numNode, &T, kChkNode);
+    double xn[8], yn[8], zn[8];
 #pragma unroll
-    for (int l = 0; l < 8; ++l) {
-        xd_local[l] = D.xd[nodes[l]];
-        yd_local[l] = D.yd[nodes[l]];
-        zd_local[l] = D.zd[nodes[l]];
-    }
-    const VelRegs vel{xd_local, yd_local, zd_local};
+    for (int l = 0; l < 8; ++l) xn[l] = D.x[n[l]];
 #pragma unroll
-    for (int l = 0; l < 8; ++l) x_local[l] = D.x[nodes[l]];
+    for (int l = 0; l < 8; ++l) yn[l] = D.y[n[l]];
 #pragma unroll
-    for (int l = 0; l < 8; ++l) y_local[l] = D.y[nodes[l]];
+    for (int l = 0; l < 8; ++l) zn[l] = D.z[n[l]];
+    kin_modal(D, T, k, xn, yn, zn, [&](int c, double (&v)[8]) {
+        const double *a = c == 0 ? D.xd : c == 1 ? D.yd : D.zd;
 #pragma unroll
-    for (int l = 0; l < 8; ++l) z_local[l] = D.z[nodes[l]];
-    kin_elem(D, T, k, x_local, y_local, z_local, vel);
+        for (int l = 0; l < 8; ++l) v[l] = a[n[l]];
+    });
 }
 
 void launch_kinematics(const SetArgs &a, int nblocks, Params P, cudaStream_t s, int bs, bool u)

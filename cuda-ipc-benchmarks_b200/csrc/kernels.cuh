@@ -27,14 +27,14 @@ constexpr int kNodeBlock = 128;  // threads per block, node kernels
 
 // Resident blocks per SM asked of the compiler (the register budget of the
 // element kernels), chosen by measurement on B200 at -s 100: force 3 (164
-// registers, 69.8 us; 86 us at 4 blocks with spills, 88 at 5), kinematics 3
-// (<= 170 registers, 118 -> 92 us), EOS 12 (40 registers with small spills;
+// registers, 69.8 us; 86 us at 4 blocks with spills, 88 at 5), kinematics 5
+// (96 registers, 51.6 us; 57.8 at 4, and 2 us more at 6 with spills), EOS 12 (40 registers with small spills;
 // 134 us unbounded, 97 us at 8 blocks, 86 us at 12, 88 us at 16).
 #ifndef LULESH_FORCE_MINB
 #define LULESH_FORCE_MINB 3
 #endif
 #ifndef LULESH_KIN_MINB
-#define LULESH_KIN_MINB 3
+#define LULESH_KIN_MINB 5
 #endif
 #ifndef LULESH_EOS_MINB
 #define LULESH_EOS_MINB 12
