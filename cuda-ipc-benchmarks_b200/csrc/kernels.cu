@@ -27,6 +27,7 @@
 // computing them from the element index, and k_nodal_u for the nodal step.
 #include <climits>
 #include <cstdint>
+#include <type_traits>
 
 #include "elem_body.cuh"
 #include "elem_math.cuh"
@@ -132,15 +133,15 @@ __device__ __constant__ int kCZ[8] = {0, 0, 0, 0, 1, 1, 1, 1};
 // One element of the force phase: the node gathers, then force_modal.
 //
 // Bound by the corner stores (192 B of the 290 B an element moves) and by
-// FP64 issue, about evenly: 70 us at -s 100 (1.0e6 elements) on B200, where
-// the stores and loads take 44 us at the measured copy rate and the ~600
-// operations 32 us at the FP64 peak.  The form that evaluated the reference's
+// FP64 issue, about evenly: 63 us at -s 100 (1.0e6 elements) on B200, where
+// the stores and loads take 44 us at the measured copy rate and the 588
+// operations 32 us at the FP64 peak (70 us with the records read from memory).  The form that evaluated the reference's
 // expressions corner by corner took 125 us (934 operations, 254 registers,
 // 8 warps per SM).  All 48 gathers go out before any arithmetic: with the
 // velocities gathered component by component, where force_modal asks for
-// them, the kernel fits 128 registers (16 warps) but takes 73 us, and 312
-// against 272 us at -s 160.
-template <bool HG, bool U>
+// them, the kernel fits 128 registers (16 warps) but took 73 against 70 us,
+// and 312 against 272 us at -s 160.
+template <bool HG, bool U, bool TABLE>
 __device__ __forceinline__ void force_one(const DomDev &D, TimeCtl &T, const Params &P, int elem)
 {
     int n[8];
@@ -165,6 +166,7 @@ __device__ __forceinline__ void force_one(const DomDev &D, TimeCtl &T, const Par
     for (int i = 0; i < 8; ++i) yn[i] = D.y[n[i]];
 #pragma unroll
     for (int i = 0; i < 8; ++i) zn[i] = D.z[n[i]];
+    if (!TABLE && !T.active) return;
     force_modal<HG>(
         xn, yn, zn, D.volo[elem], D.v[elem], D.p[elem], D.q[elem], D.ss[elem], D.elemMass[elem],
         P.hgcoef,
@@ -176,32 +178,41 @@ __device__ __forceinline__ void force_one(const DomDev &D, TimeCtl &T, const Par
         [&] { atomicMin(&T.bad_vol, elem); });
 }
 
-template <bool HG, int BS, bool U>
-__global__ void __launch_bounds__(BS, min_blocks(kForceMinBlocks, BS)) k_force(SetArgs a, Params P)
+template <bool HG, int BS, bool U, class W>
+__global__ void __launch_bounds__(BS, min_blocks(kForceMinBlocks, BS))
+    k_force(const __grid_constant__ W w, Params P)
 {
     pdl_enter();
-    const int2 blk = a.blocks[LULESH_FORCE_REVERSE ? gridDim.x - 1 - blockIdx.x : blockIdx.x];
-    const DomDev &D = a.doms[blk.x];
-    TimeCtl &T = a.tcs[D.tc];
-    if (!T.active) return;
+    const int2 blk = w.template block<BS, LULESH_FORCE_REVERSE>();
+    const DomDev &D = w.domain(blk.x);
+    TimeCtl &T = w.time(D);
+    if (W::kTable && !T.active) return;
     const int elem = blk.y + threadIdx.x;
     if (elem >= D.numElem) return;
-    force_one<HG, U>(D, T, P, elem);
+    force_one<HG, U, W::kTable>(D, T, P, elem);
 }
 
-template <int BS, bool U = false>
-static void launch_force_bs(const SetArgs &a, int nblocks, Params P, cudaStream_t s)
+template <int BS, bool U, class W>
+static void launch_force_w(const W &w, bool pdl, int nblocks, Params P, cudaStream_t s)
 {
     if (P.hgcoef > 0.0)
-        launch_k(k_force<true, BS, U>, nblocks, BS, s, a.pdl != 0, a, P);
+        launch_k(k_force<true, BS, U, W>, nblocks, BS, s, pdl, w, P);
     else
-        launch_k(k_force<false, BS, U>, nblocks, BS, s, a.pdl != 0, a, P);
+        launch_k(k_force<false, BS, U, W>, nblocks, BS, s, pdl, w, P);
+}
+
+template <int BS>
+static void launch_force_bs(const SetArgs &a, int nblocks, Params P, cudaStream_t s)
+{
+    launch_where<true, BS == kElemBlock>(a, nblocks, [&](const auto &w) {
+        launch_force_w<BS, false>(w, a.pdl != 0, nblocks, P, s);
+    });
 }
 
 void launch_force(const SetArgs &a, int nblocks, Params P, cudaStream_t s, int bs, bool u)
 {
-    if (u) {
-        launch_force_bs<kElemBlock, true>(a, nblocks, P, s);
+    if (u) {  // an lmesh set is one domain
+        launch_force_w<kElemBlock, true>(by_value<1>(a, nblocks), a.pdl != 0, nblocks, P, s);
         return;
     }
     switch (bs) {
@@ -219,13 +230,15 @@ void launch_force(const SetArgs &a, int nblocks, Params P, cudaStream_t s, int b
 // (lulesh.cu:1082-1091).  A corner whose element lies in a neighbouring
 // subdomain is read from that subdomain's corner array: the result equals
 // the undecomposed mesh's sum bit for bit.
+// NEIGHBOURS false: this domain's own corners only.
+template <bool NEIGHBOURS>
 __device__ __forceinline__ void gather_corners(const DomDev *doms, const DomDev &D, int px,
                                                int py, int pz, double &fx, double &fy,
                                                double &fz, TimeCtl *T)
 {
     const int nx = D.nx;
     fx = fy = fz = 0.0;
-    if (D.tp > 1) {
+    if (NEIGHBOURS && D.tp > 1) {
         // subdomains: the source domain of each corner first (this one or
         // a neighbour), then one load path that the warp shares
 #pragma unroll
@@ -316,14 +329,15 @@ __device__ __forceinline__ void advance_node(const DomDev &D, const TimeCtl &T, 
 // MODE 1: AddNodeForcesFromElems over this domain's own corners only,
 //         writing fx/fy/fz (the partial sums the reference exchanges).
 // MODE 2: the node update from fx/fy/fz (after CommSBN added neighbours).
-template <int MODE, int BS>
-__global__ void __launch_bounds__(BS, min_blocks(kNodalMinBlocks, BS)) k_nodal(SetArgs a, Params P)
+template <int MODE, int BS, class W>
+__global__ void __launch_bounds__(BS, min_blocks(kNodalMinBlocks, BS))
+    k_nodal(const __grid_constant__ W w, Params P)
 {
     pdl_enter();
-    const int2 blk = a.blocks[blockIdx.x];
-    const DomDev &D = a.doms[blk.x];
-    const TimeCtl &T = a.tcs[D.tc];
-    if (!T.active) return;
+    const int2 blk = w.template block<BS, LULESH_NODAL_REVERSE && !W::kTable>();
+    const DomDev &D = w.domain(blk.x);
+    TimeCtl &T = w.time(D);
+    if (W::kTable && !T.active) return;
     const int i = blk.y + threadIdx.x;
     if (i >= D.numNode) return;
     const int en = D.en;
@@ -334,11 +348,9 @@ __global__ void __launch_bounds__(BS, min_blocks(kNodalMinBlocks, BS)) k_nodal(S
 
     double fx, fy, fz;
     if (MODE == 0) {
-        gather_corners(a.doms, D, px, py, pz, fx, fy, fz, &a.tcs[D.tc]);
+        gather_corners<!std::is_same_v<W, OneDomain>>(w.doms(), D, px, py, pz, fx, fy, fz, &T);
     } else if (MODE == 1) {
-        DomDev L = D;
-        L.tp = 1;  // own corners only
-        gather_corners(a.doms, L, px, py, pz, fx, fy, fz, &a.tcs[D.tc]);
+        gather_corners<false>(w.doms(), D, px, py, pz, fx, fy, fz, &T);  // own corners only
         D.fx[i] = fx;
         D.fy[i] = fy;
         D.fz[i] = fz;
@@ -353,7 +365,8 @@ __global__ void __launch_bounds__(BS, min_blocks(kNodalMinBlocks, BS)) k_nodal(S
     // px/py/pz == 0 node sets of the domains at the mesh origin faces
     const int bc = (D.col == 0 && px == 0 ? 1 : 0) | (D.row == 0 && py == 0 ? 2 : 0) |
                    (D.plane == 0 && pz == 0 ? 4 : 0);
-    advance_node(D, T, P, i, bc, fx, fy, fz, a.materialize, MODE == 0);
+    if (!W::kTable && !T.active) return;
+    advance_node(D, T, P, i, bc, fx, fy, fz, w.materialize(), MODE == 0);
 }
 
 // Unstructured meshes: AddNodeForcesFromElems (lulesh.cu:1715-1751) over
@@ -364,13 +377,14 @@ __global__ void __launch_bounds__(BS, min_blocks(kNodalMinBlocks, BS)) k_nodal(S
 // 8-int stride: one sector per thread per load), and the corner loads go
 // out four corners at a time.
 template <int BS>
-__global__ void __launch_bounds__(BS, min_blocks(kNodalUMinBlocks, BS)) k_nodal_u(SetArgs a, Params P)
+__global__ void __launch_bounds__(BS, min_blocks(kNodalUMinBlocks, BS))
+    k_nodal_u(const __grid_constant__ OneDomain w, Params P)
 {
     pdl_enter();
     __shared__ int s_list[8 * BS];
-    const int2 blk = a.blocks[blockIdx.x];
-    const DomDev &D = a.doms[blk.x];
-    const TimeCtl &T = a.tcs[D.tc];
+    const int2 blk = w.template block<BS, LULESH_NODAL_REVERSE>();
+    const DomDev &D = w.D[0];
+    const TimeCtl &T = *w.tc;
     if (!T.active) return;  // the whole block
     const int first = blk.y;
     const int last = min(first + BS, D.numNode) - 1;
@@ -406,7 +420,7 @@ __global__ void __launch_bounds__(BS, min_blocks(kNodalUMinBlocks, BS)) k_nodal_
                     fz += vz[q];
                 }
         }
-        advance_node(D, T, P, i, D.nodeBC[i], fx, fy, fz, a.materialize, true);
+        advance_node(D, T, P, i, D.nodeBC[i], fx, fy, fz, w.mat, true);
         return;
     }
     const long long list_len = 8LL * D.numElem;  // corner-list entries
@@ -458,51 +472,61 @@ __global__ void __launch_bounds__(BS, min_blocks(kNodalUMinBlocks, BS)) k_nodal_
         fz += ld_corner(D.fz_elem + k);
     }
     // symmetry nodes of the mesh's X/Y/Z sets: nodeBC bits 0/1/2
-    advance_node(D, T, P, i, D.nodeBC[i], fx, fy, fz, a.materialize, true);
+    advance_node(D, T, P, i, D.nodeBC[i], fx, fy, fz, w.mat, true);
+}
+
+template <int BS>
+static void launch_nodal_bs(const SetArgs &a, int nblocks, Params P, cudaStream_t s)
+{
+    launch_where<true, BS == kNodeBlock>(a, nblocks, [&](const auto &w) {
+        launch_k(k_nodal<0, BS, std::decay_t<decltype(w)>>, nblocks, BS, s, a.pdl != 0, w, P);
+    });
 }
 
 void launch_nodal(const SetArgs &a, int nblocks, Params P, cudaStream_t s, int bs, bool u)
 {
     if (u) {
-        launch_k(k_nodal_u<kNodeBlock>, nblocks, kNodeBlock, s, a.pdl != 0, a, P);
+        launch_k(k_nodal_u<kNodeBlock>, nblocks, kNodeBlock, s, a.pdl != 0,
+                 by_value<1>(a, nblocks), P);
         return;
     }
     switch (bs) {
-        case 256: launch_k(k_nodal<0, 256>, nblocks, 256, s, a.pdl != 0, a, P); break;
-        case 512: launch_k(k_nodal<0, 512>, nblocks, 512, s, a.pdl != 0, a, P); break;
-        default: launch_k(k_nodal<0, kNodeBlock>, nblocks, kNodeBlock, s, a.pdl != 0, a, P); break;
+        case 256: launch_nodal_bs<256>(a, nblocks, P, s); break;
+        case 512: launch_nodal_bs<512>(a, nblocks, P, s); break;
+        default: launch_nodal_bs<kNodeBlock>(a, nblocks, P, s); break;
     }
 }
 
 void launch_nodal_gather_local(const SetArgs &a, int nblocks, cudaStream_t s)
 {
-    k_nodal<1, kNodeBlock><<<nblocks, kNodeBlock, 0, s>>>(a, Params{});
+    k_nodal<1, kNodeBlock, ManyDomains><<<nblocks, kNodeBlock, 0, s>>>(ManyDomains{a}, Params{});
 }
 
 void launch_nodal_update(const SetArgs &a, int nblocks, Params P, cudaStream_t s)
 {
-    k_nodal<2, kNodeBlock><<<nblocks, kNodeBlock, 0, s>>>(a, P);
+    k_nodal<2, kNodeBlock, ManyDomains><<<nblocks, kNodeBlock, 0, s>>>(ManyDomains{a}, P);
 }
 
 // ---------------------------------------------------------------------------
 // kinematics: CalcKinematicsAndMonotonicQGradient_kernel, lulesh.cu:3343-3507
 
-// Bound by latency and FP64 issue at 20 warps per SM: 51.6 us at -s 100
+// Bound by latency and FP64 issue at 20 warps per SM: 43 us at -s 100
 // (1.0e6 elements) on B200, against 22 us for its 144 B per element at the
-// measured copy rate and 19 us for its ~360 operations; 80 us with the
-// reference's corner-by-corner expressions (649 operations, 168 registers).
+// measured copy rate and 20 us for its 367 operations (51.6 us with the
+// records read from memory); 80 us with the reference's corner-by-corner expressions (649 operations, 168 registers).
 // The velocities are gathered where kin_modal asks for them, after the volume
-// and length stores, at 96 registers (5 blocks); 57.8 us at 4 blocks.  Up
+// and length stores, at 96 registers (5 blocks); 6 us more at 4 blocks.  Up
 // front took 8 us more at 3 blocks, and between the coordinates and the volume
 // 2 us more at 4 blocks and 4 at 5 (with spills).
-template <int BS, bool U = false>
-__global__ void __launch_bounds__(BS, min_blocks(kKinMinBlocks, BS)) k_kinematics(SetArgs a)
+template <int BS, bool U, class W>
+__global__ void __launch_bounds__(BS, min_blocks(kKinMinBlocks, BS))
+    k_kinematics(const __grid_constant__ W w)
 {
     pdl_enter();
-    const int2 blk = a.blocks[LULESH_KIN_REVERSE ? gridDim.x - 1 - blockIdx.x : blockIdx.x];
-    const DomDev &D = a.doms[blk.x];
-    TimeCtl &T = a.tcs[D.tc];
-    if (!T.active) return;
+    const int2 blk = w.template block<BS, LULESH_KIN_REVERSE>();
+    const DomDev &D = w.domain(blk.x);
+    TimeCtl &T = w.time(D);
+    if (W::kTable && !T.active) return;
     const int k = blk.y + threadIdx.x;
     if (k >= D.numElem) return;
 
@@ -517,6 +541,7 @@ __global__ void __launch_bounds__(BS, min_blocks(kKinMinBlocks, BS)) k_kinematic
     for (int l = 0; l < 8; ++l) yn[l] = D.y[n[l]];
 #pragma unroll
     for (int l = 0; l < 8; ++l) zn[l] = D.z[n[l]];
+    if (!W::kTable && !T.active) return;
     kin_modal(D, T, k, xn, yn, zn, [&](int c, double (&v)[8]) {
         const double *a = c == 0 ? D.xd : c == 1 ? D.yd : D.zd;
 #pragma unroll
@@ -524,17 +549,27 @@ __global__ void __launch_bounds__(BS, min_blocks(kKinMinBlocks, BS)) k_kinematic
     });
 }
 
+template <int BS>
+static void launch_kinematics_bs(const SetArgs &a, int nblocks, cudaStream_t s)
+{
+    launch_where<true, BS == kElemBlock>(a, nblocks, [&](const auto &w) {
+        launch_k(k_kinematics<BS, false, std::decay_t<decltype(w)>>, nblocks, BS, s, a.pdl != 0,
+                 w);
+    });
+}
+
 void launch_kinematics(const SetArgs &a, int nblocks, Params P, cudaStream_t s, int bs, bool u)
 {
     (void)P;
     if (u) {
-        launch_k(k_kinematics<kElemBlock, true>, nblocks, kElemBlock, s, a.pdl != 0, a);
+        launch_k(k_kinematics<kElemBlock, true, OneDomain>, nblocks, kElemBlock, s, a.pdl != 0,
+                 by_value<1>(a, nblocks));
         return;
     }
     switch (bs) {
-        case 64: launch_k(k_kinematics<64>, nblocks, 64, s, a.pdl != 0, a); break;
-        case 256: launch_k(k_kinematics<256>, nblocks, 256, s, a.pdl != 0, a); break;
-        default: launch_k(k_kinematics<kElemBlock>, nblocks, kElemBlock, s, a.pdl != 0, a); break;
+        case 64: launch_kinematics_bs<64>(a, nblocks, s); break;
+        case 256: launch_kinematics_bs<256>(a, nblocks, s); break;
+        default: launch_kinematics_bs<kElemBlock>(a, nblocks, s); break;
     }
 }
 
@@ -793,13 +828,14 @@ __device__ __forceinline__ double warp_min(double v)
 
 // SUB: a subdomain set's fused cycle, which reads a comm face's neighbour
 // element in the neighbouring subdomain (no MonoQ ghost copy)
-template <int BS, bool U = false, bool SUB = false>
-__global__ void __launch_bounds__(BS, min_blocks(kEosMinBlocks, BS)) k_eos(SetArgs a, Params P)
+template <int BS, bool U, bool SUB, class W>
+__global__ void __launch_bounds__(BS, min_blocks(kEosMinBlocks, BS))
+    k_eos(const __grid_constant__ W w, Params P)
 {
     pdl_enter();
-    const int2 blk = a.blocks[LULESH_EOS_REVERSE ? gridDim.x - 1 - blockIdx.x : blockIdx.x];
-    const DomDev &D = a.doms[blk.x];
-    TimeCtl &T = a.tcs[D.tc];
+    const int2 blk = w.template block<BS, LULESH_EOS_REVERSE>();
+    const DomDev &D = w.domain(blk.x);
+    TimeCtl &T = w.time(D);
     if (!T.active) return;  // uniform per block
     const int i = blk.y + threadIdx.x;
     double dtc = 1.0e+20, dth = 1.0e+20;
@@ -838,27 +874,27 @@ __global__ void __launch_bounds__(BS, min_blocks(kEosMinBlocks, BS)) k_eos(SetAr
             const int ix = zidx % nx, t = zidx / nx, iy = t % nx, iz = t / nx;
             const DomDev *sxm = &D, *sxp = &D, *sem = &D, *sep = &D, *szm = &D, *szp = &D;
             if (bcMask & XI_M_COMM) {
-                sxm = &a.doms[D.nbr[0 + 3 + 9]];
+                sxm = &w.doms()[D.nbr[0 + 3 + 9]];
                 lxm = (iz * nx + iy) * nx + (nx - 1);
             }
             if (bcMask & XI_P_COMM) {
-                sxp = &a.doms[D.nbr[2 + 3 + 9]];
+                sxp = &w.doms()[D.nbr[2 + 3 + 9]];
                 lxp = (iz * nx + iy) * nx;
             }
             if (bcMask & ETA_M_COMM) {
-                sem = &a.doms[D.nbr[1 + 0 + 9]];
+                sem = &w.doms()[D.nbr[1 + 0 + 9]];
                 lem = (iz * nx + (nx - 1)) * nx + ix;
             }
             if (bcMask & ETA_P_COMM) {
-                sep = &a.doms[D.nbr[1 + 6 + 9]];
+                sep = &w.doms()[D.nbr[1 + 6 + 9]];
                 lep = (iz * nx) * nx + ix;
             }
             if (bcMask & ZETA_M_COMM) {
-                szm = &a.doms[D.nbr[1 + 3 + 0]];
+                szm = &w.doms()[D.nbr[1 + 3 + 0]];
                 lzm = ((nx - 1) * nx + iy) * nx + ix;
             }
             if (bcMask & ZETA_P_COMM) {
-                szp = &a.doms[D.nbr[1 + 3 + 18]];
+                szp = &w.doms()[D.nbr[1 + 3 + 18]];
                 lzp = iy * nx + ix;
             }
             phixi = mono_limiter_split(D.delv_xi, sxm->delv_xi, sxp->delv_xi, zidx, bcMask, XI_M,
@@ -906,7 +942,7 @@ __global__ void __launch_bounds__(BS, min_blocks(kEosMinBlocks, BS)) k_eos(SetAr
         }
         const double q_old_z = D.q[zidx];
         if (q_old_z > P.qstop) atomicMin(&T.bad_q, zidx);
-        if (a.materialize) {
+        if (w.materialize()) {
             D.qq[zidx] = qquad;
             D.ql[zidx] = qlin;
         }
@@ -996,21 +1032,31 @@ __global__ void __launch_bounds__(BS, min_blocks(kEosMinBlocks, BS)) k_eos(SetAr
     }
 }
 
+template <int BS, bool SUB>
+static void launch_eos_bs(const SetArgs &a, int nblocks, Params P, cudaStream_t s)
+{
+    launch_where<!SUB, SUB>(a, nblocks, [&](const auto &w) {
+        launch_k(k_eos<BS, false, SUB, std::decay_t<decltype(w)>>, nblocks, BS, s, a.pdl != 0, w,
+                 P);
+    });
+}
+
 void launch_eos(const SetArgs &a, int nblocks, Params P, cudaStream_t s, int bs, bool u,
                 bool sub)
 {
     if (u) {
-        launch_k(k_eos<kElemBlock, true>, nblocks, kElemBlock, s, a.pdl != 0, a, P);
+        launch_k(k_eos<kElemBlock, true, false, OneDomain>, nblocks, kElemBlock, s, a.pdl != 0,
+                 by_value<1>(a, nblocks), P);
         return;
     }
     if (sub) {  // subdomain sets take 128-element blocks only
-        launch_k(k_eos<kElemBlock, false, true>, nblocks, kElemBlock, s, a.pdl != 0, a, P);
+        launch_eos_bs<kElemBlock, true>(a, nblocks, P, s);
         return;
     }
     switch (bs) {
-        case 64: launch_k(k_eos<64>, nblocks, 64, s, a.pdl != 0, a, P); break;
-        case 256: launch_k(k_eos<256>, nblocks, 256, s, a.pdl != 0, a, P); break;
-        default: launch_k(k_eos<kElemBlock>, nblocks, kElemBlock, s, a.pdl != 0, a, P); break;
+        case 64: launch_eos_bs<64, false>(a, nblocks, P, s); break;
+        case 256: launch_eos_bs<256, false>(a, nblocks, P, s); break;
+        default: launch_eos_bs<kElemBlock, false>(a, nblocks, P, s); break;
     }
 }
 

@@ -11,13 +11,6 @@
 #include "lulesh_b200.h"
 #include "lulesh_dev.h"
 
-// Node blocks last to first: the nodal kernel follows the force kernel,
-// whose last-written corner forces are the ones still in L2 (measured on
-// B200 at -s 100: nodal 53.7 -> 48.9 us, the same results).
-#ifndef LULESH_NODAL_REVERSE
-#define LULESH_NODAL_REVERSE 1
-#endif
-
 // The EOS of a subdomain set's fused cycle, and of a part of a multi-GPU
 // problem, reads a comm face's neighbour element in the neighbouring
 // subdomain or its proxy (k_eos<..., SUB>): the value k_monoq_ghost would
@@ -137,6 +130,11 @@ struct lulesh_set {
         a.blocks = blocks;
         a.materialize = (flags & LULESH_FLAG_MATERIALIZE) ? 1 : 0;
         a.pdl = pdl ? 1 : 0;
+        // not for parts: their records are followed by proxies
+        a.ndom = ndom;
+        a.records = nparts == 1 && njobs == 1 && (ndom == 1 || ndom == lulesh::kFewDomains)
+                        ? hdoms.data()
+                        : nullptr;
         return a;
     }
 };
