@@ -623,65 +623,14 @@ __device__ __forceinline__ void elem_face_links(const DomDev &D, int z, int &bc,
     }
 }
 
-// one direction of the monotonic limiter, lulesh.cu:3595-3624
-__device__ __forceinline__ double mono_limiter(const double *delv, int i, int bc, int mmask,
-                                               int msymm, int mfree, int pmask, int psymm,
-                                               int pfree, int lm, int lp, double mult,
-                                               double maxslope, double ptiny, int nlinks,
-                                               TimeCtl *T)
+// One direction of the monotonic limiter, lulesh.cu:3595-3624, from the
+// element's gradient d and those of its minus and plus neighbours (the
+// element's own at a symmetry plane, 0 at a free surface).
+__device__ __forceinline__ double mono_limiter(double d, double delvm, double delvp, double mult,
+                                               double maxslope)
 {
-    const double norm = 1. / (delv[i] + ptiny);
-    double delvm, delvp;
-    const int mb = bc & mmask, pb = bc & pmask;
-    if (mb == msymm)
-        delvm = delv[i];
-    else if (mb == mfree)
-        delvm = 0.0;
-    else  // 0 or *_COMM: neighbour or ghost element
-        delvm = delv[chk_index(lm, nlinks, T, kChkLink)];
-    if (pb == psymm)
-        delvp = delv[i];
-    else if (pb == pfree)
-        delvp = 0.0;
-    else
-        delvp = delv[chk_index(lp, nlinks, T, kChkLink)];
-    delvm = delvm * norm;
-    delvp = delvp * norm;
-    double phi = .5 * (delvm + delvp);
-    delvm *= mult;
-    delvp *= mult;
-    if (delvm < phi) phi = delvm;
-    if (delvp < phi) phi = delvp;
-    if (phi < 0.) phi = 0.;
-    if (phi > maxslope) phi = maxslope;
-    return phi;
-}
-
-// mono_limiter with the minus and plus neighbours read from their own
-// arrays (dm[lm], dp[lp]): a comm face's neighbour element is then read in
-// the neighbouring subdomain instead of from this subdomain's ghost copy.
-__device__ __forceinline__ double mono_limiter_split(const double *delv, const double *dm,
-                                                     const double *dp, int i, int bc,
-                                                     int mmask, int msymm, int mfree,
-                                                     int pmask, int psymm, int pfree, int lm,
-                                                     int lp, double mult, double maxslope,
-                                                     double ptiny, int nm, int np, TimeCtl *T)
-{
-    const double norm = 1. / (delv[i] + ptiny);
-    double delvm, delvp;
-    const int mb = bc & mmask, pb = bc & pmask;
-    if (mb == msymm)
-        delvm = delv[i];
-    else if (mb == mfree)
-        delvm = 0.0;
-    else
-        delvm = dm[chk_index(lm, nm, T, kChkLink)];
-    if (pb == psymm)
-        delvp = delv[i];
-    else if (pb == pfree)
-        delvp = 0.0;
-    else
-        delvp = dp[chk_index(lp, np, T, kChkLink)];
+    const double ptiny = 1.e-36;
+    const double norm = 1. / (d + ptiny);
     delvm = delvm * norm;
     delvp = delvp * norm;
     double phi = .5 * (delvm + delvp);
@@ -819,6 +768,13 @@ __device__ __forceinline__ void eos_reps(int rep, double e_temp, double p_temp, 
     }
 }
 
+__device__ __forceinline__ double warp_max(double v)
+{
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
+    return v;
+}
+
 __device__ __forceinline__ double warp_min(double v)
 {
 #pragma unroll
@@ -826,8 +782,35 @@ __device__ __forceinline__ double warp_min(double v)
     return v;
 }
 
+// Block b's turn among a domain's EOS blocks.  The slots are grouped by rep
+// class, the costliest first; walked in that order, the first third of the
+// kernel computes and the rest waits for memory.  One block in kEosMix is
+// therefore a costly one until those run out (a permutation of the blocks; the
+// blocks' own order where the costly class is more than 1/kEosMix of them).
+// EOS on B200, us, class order -> 2, 3, 4 of a kind: -s 100 55.9 -> 52.1 (3 and
+// 4), -s 133 with 20 regions and cost 4 135.8 -> 127.4 (3), 129.4 (4).
+constexpr int kEosMix = 3;
+template <int BS>
+__device__ __forceinline__ int eos_block(const DomDev &D, int b)
+{
+    const int heavy = D.eosClassEnd[0] / BS;
+    if (heavy * kEosMix > (D.numElem + BS - 1) / BS || b >= heavy * kEosMix) return b;
+    return b % kEosMix == 0 ? b / kEosMix : heavy + b - b / kEosMix - 1;
+}
+
 // SUB: a subdomain set's fused cycle, which reads a comm face's neighbour
 // element in the neighbouring subdomain (no MonoQ ghost copy)
+//
+// Bound by the latency of its 22 loads an element and their scattered sectors
+// (487 B of L2 traffic for 196 B of data), not by the reps: 52 us at -s 100
+// (1.0e6 elements) on B200, against 30 us for the 196 B at the measured copy
+// rate; 40 more reps for the costliest class add 8 us.  With each load beside
+// its use, between branches, atomics and stores that no load can pass, it took
+// 70.5 us at 40 registers and 12 blocks per SM.  All loads first want 64
+// registers: 8 blocks 55.9 us, 6 64.4, 7 59.8, 10 59.9 (spills), 12 72.5.
+// Elements in natural order instead of class order: 57.8 us at 8 blocks,
+// 53.7 at 9, but 150 against 136 us at -s 133 with cost 4, where every warp
+// runs its costliest element's reps.
 template <int BS, bool U, bool SUB, class W>
 __global__ void __launch_bounds__(BS, min_blocks(kEosMinBlocks, BS))
     k_eos(const __grid_constant__ W w, Params P)
@@ -837,8 +820,8 @@ __global__ void __launch_bounds__(BS, min_blocks(kEosMinBlocks, BS))
     const DomDev &D = w.domain(blk.x);
     TimeCtl &T = w.time(D);
     if (!T.active) return;  // uniform per block
-    const int i = blk.y + threadIdx.x;
-    double dtc = 1.0e+20, dth = 1.0e+20;
+    const int i = eos_block<BS>(D, blk.y / BS) * BS + threadIdx.x;
+    double dtc = 1.0e+20, vmax = 0.0;
     if (i < D.numElem) {
         // The element of this slot and its rep count.  The reference visits
         // regElemlist and finds the rep by region (giveMyRegion,
@@ -851,87 +834,102 @@ __global__ void __launch_bounds__(BS, min_blocks(kEosMinBlocks, BS))
         while (cls < D.eosNumClass - 1 && i >= D.eosClassEnd[cls]) ++cls;
         const int rep = D.eosClassRep[cls];
 
-        // ---- CalcMonotonicQRegionForElems_kernel, lulesh.cu:3586-3724
-        const double ptiny = 1.e-36;
-        int bcMask, lxm, lxp, lem, lep, lzm, lzp;
+        // Every array the element needs, before any arithmetic, branch or
+        // store.  A face on the mesh boundary reads the element itself: its
+        // neighbour's value is then the element's own (symmetry plane) or
+        // replaced by 0 (free surface).
+        int bcMask, lm[3], lp[3];
         if (U) {  // the mesh's own links and boundary mask
             bcMask = D.elemBC[zidx];
-            lxm = D.lxim[zidx];
-            lxp = D.lxip[zidx];
-            lem = D.letam[zidx];
-            lep = D.letap[zidx];
-            lzm = D.lzetam[zidx];
-            lzp = D.lzetap[zidx];
+            lm[0] = D.lxim[zidx];
+            lp[0] = D.lxip[zidx];
+            lm[1] = D.letam[zidx];
+            lp[1] = D.letap[zidx];
+            lm[2] = D.lzetam[zidx];
+            lp[2] = D.lzetap[zidx];
         } else {
-            elem_face_links(D, zidx, bcMask, lxm, lxp, lem, lep, lzm, lzp);
+            elem_face_links(D, zidx, bcMask, lm[0], lp[0], lm[1], lp[1], lm[2], lp[2]);
         }
-        const double mult = P.monoq_limiter_mult, maxs = P.monoq_max_slope;
-        double phixi, phieta, phizeta;
+        const auto is = [&](int mask, int symm, int free) {
+            return (bcMask & mask) == symm || (bcMask & mask) == free;
+        };
+        if (is(XI_M, XI_M_SYMM, XI_M_FREE)) lm[0] = zidx;
+        if (is(XI_P, XI_P_SYMM, XI_P_FREE)) lp[0] = zidx;
+        if (is(ETA_M, ETA_M_SYMM, ETA_M_FREE)) lm[1] = zidx;
+        if (is(ETA_P, ETA_P_SYMM, ETA_P_FREE)) lp[1] = zidx;
+        if (is(ZETA_M, ZETA_M_SYMM, ZETA_M_FREE)) lm[2] = zidx;
+        if (is(ZETA_P, ZETA_P_SYMM, ZETA_P_FREE)) lp[2] = zidx;
+        const DomDev *sm[3] = {&D, &D, &D}, *sp[3] = {&D, &D, &D};
         if (SUB) {
             // comm faces: the mirrored element of the neighbour's opposite
             // face layer, where k_monoq_ghost would copy it from
             const int nx = D.nx;
             const int ix = zidx % nx, t = zidx / nx, iy = t % nx, iz = t / nx;
-            const DomDev *sxm = &D, *sxp = &D, *sem = &D, *sep = &D, *szm = &D, *szp = &D;
             if (bcMask & XI_M_COMM) {
-                sxm = &w.doms()[D.nbr[0 + 3 + 9]];
-                lxm = (iz * nx + iy) * nx + (nx - 1);
+                sm[0] = &w.doms()[D.nbr[0 + 3 + 9]];
+                lm[0] = (iz * nx + iy) * nx + (nx - 1);
             }
             if (bcMask & XI_P_COMM) {
-                sxp = &w.doms()[D.nbr[2 + 3 + 9]];
-                lxp = (iz * nx + iy) * nx;
+                sp[0] = &w.doms()[D.nbr[2 + 3 + 9]];
+                lp[0] = (iz * nx + iy) * nx;
             }
             if (bcMask & ETA_M_COMM) {
-                sem = &w.doms()[D.nbr[1 + 0 + 9]];
-                lem = (iz * nx + (nx - 1)) * nx + ix;
+                sm[1] = &w.doms()[D.nbr[1 + 0 + 9]];
+                lm[1] = (iz * nx + (nx - 1)) * nx + ix;
             }
             if (bcMask & ETA_P_COMM) {
-                sep = &w.doms()[D.nbr[1 + 6 + 9]];
-                lep = (iz * nx) * nx + ix;
+                sp[1] = &w.doms()[D.nbr[1 + 6 + 9]];
+                lp[1] = (iz * nx) * nx + ix;
             }
             if (bcMask & ZETA_M_COMM) {
-                szm = &w.doms()[D.nbr[1 + 3 + 0]];
-                lzm = ((nx - 1) * nx + iy) * nx + ix;
+                sm[2] = &w.doms()[D.nbr[1 + 3 + 0]];
+                lm[2] = ((nx - 1) * nx + iy) * nx + ix;
             }
             if (bcMask & ZETA_P_COMM) {
-                szp = &w.doms()[D.nbr[1 + 3 + 18]];
-                lzp = iy * nx + ix;
+                sp[2] = &w.doms()[D.nbr[1 + 3 + 18]];
+                lp[2] = iy * nx + ix;
             }
-            phixi = mono_limiter_split(D.delv_xi, sxm->delv_xi, sxp->delv_xi, zidx, bcMask, XI_M,
-                                       XI_M_SYMM, XI_M_FREE, XI_P, XI_P_SYMM, XI_P_FREE, lxm, lxp,
-                                       mult, maxs, ptiny, sxm->allElem, sxp->allElem, &T);
-            phieta = mono_limiter_split(D.delv_eta, sem->delv_eta, sep->delv_eta, zidx, bcMask,
-                                        ETA_M, ETA_M_SYMM, ETA_M_FREE, ETA_P, ETA_P_SYMM,
-                                        ETA_P_FREE, lem, lep, mult, maxs, ptiny, sem->allElem,
-                                        sep->allElem, &T);
-            phizeta = mono_limiter_split(D.delv_zeta, szm->delv_zeta, szp->delv_zeta, zidx,
-                                         bcMask, ZETA_M, ZETA_M_SYMM, ZETA_M_FREE, ZETA_P,
-                                         ZETA_P_SYMM, ZETA_P_FREE, lzm, lzp, mult, maxs, ptiny,
-                                         szm->allElem, szp->allElem, &T);
-        } else {
-            phixi = mono_limiter(D.delv_xi, zidx, bcMask, XI_M, XI_M_SYMM, XI_M_FREE, XI_P,
-                                 XI_P_SYMM, XI_P_FREE, lxm, lxp, mult, maxs, ptiny, D.allElem, &T);
-            phieta = mono_limiter(D.delv_eta, zidx, bcMask, ETA_M, ETA_M_SYMM, ETA_M_FREE, ETA_P,
-                                  ETA_P_SYMM, ETA_P_FREE, lem, lep, mult, maxs, ptiny, D.allElem,
-                                  &T);
-            phizeta = mono_limiter(D.delv_zeta, zidx, bcMask, ZETA_M, ZETA_M_SYMM, ZETA_M_FREE,
-                                   ZETA_P, ZETA_P_SYMM, ZETA_P_FREE, lzm, lzp, mult, maxs, ptiny,
-                                   D.allElem, &T);
         }
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            lm[c] = chk_index(lm[c], SUB ? sm[c]->allElem : D.allElem, &T, kChkLink);
+            lp[c] = chk_index(lp[c], SUB ? sp[c]->allElem : D.allElem, &T, kChkLink);
+        }
+        const double dxi = D.delv_xi[zidx], deta = D.delv_eta[zidx], dzeta = D.delv_zeta[zidx];
+        double xim = sm[0]->delv_xi[lm[0]], xip = sp[0]->delv_xi[lp[0]];
+        double etam = sm[1]->delv_eta[lm[1]], etap = sp[1]->delv_eta[lp[1]];
+        double zetam = sm[2]->delv_zeta[lm[2]], zetap = sp[2]->delv_zeta[lp[2]];
         const double vdov_z = D.vdov[zidx];
         const double vnew_z = D.vnew[zidx];
+        const double xxi = D.delx_xi[zidx], xeta = D.delx_eta[zidx], xzeta = D.delx_zeta[zidx];
+        const double mass_z = D.elemMass[zidx], volo_z = D.volo[zidx];
+        const double q_old_z = D.q[zidx], v_z = D.v[zidx];
+        const double e_temp = D.e[zidx], p_temp = D.p[zidx], delvc_temp = D.delv[zidx];
+        const double area_tmp = D.arealg[zidx];
+
+        // ---- CalcMonotonicQRegionForElems_kernel, lulesh.cu:3586-3724
+        if ((bcMask & XI_M) == XI_M_FREE) xim = 0.0;
+        if ((bcMask & XI_P) == XI_P_FREE) xip = 0.0;
+        if ((bcMask & ETA_M) == ETA_M_FREE) etam = 0.0;
+        if ((bcMask & ETA_P) == ETA_P_FREE) etap = 0.0;
+        if ((bcMask & ZETA_M) == ZETA_M_FREE) zetam = 0.0;
+        if ((bcMask & ZETA_P) == ZETA_P_FREE) zetap = 0.0;
+        const double mult = P.monoq_limiter_mult, maxs = P.monoq_max_slope;
+        const double phixi = mono_limiter(dxi, xim, xip, mult, maxs);
+        const double phieta = mono_limiter(deta, etam, etap, mult, maxs);
+        const double phizeta = mono_limiter(dzeta, zetam, zetap, mult, maxs);
         double qlin, qquad;
         if (vdov_z > 0.) {
             qlin = 0.;
             qquad = 0.;
         } else {
-            double delvxxi = D.delv_xi[zidx] * D.delx_xi[zidx];
-            double delvxeta = D.delv_eta[zidx] * D.delx_eta[zidx];
-            double delvxzeta = D.delv_zeta[zidx] * D.delx_zeta[zidx];
+            double delvxxi = dxi * xxi;
+            double delvxeta = deta * xeta;
+            double delvxzeta = dzeta * xzeta;
             if (delvxxi > 0.) delvxxi = 0.;
             if (delvxeta > 0.) delvxeta = 0.;
             if (delvxzeta > 0.) delvxzeta = 0.;
-            const double rho = D.elemMass[zidx] / (D.volo[zidx] * vnew_z);
+            const double rho = mass_z / (volo_z * vnew_z);
             qlin = -P.qlc_monoq * rho *
                    (delvxxi * (1. - phixi) + delvxeta * (1. - phieta) +
                     delvxzeta * (1. - phizeta));
@@ -940,7 +938,6 @@ __global__ void __launch_bounds__(BS, min_blocks(kEosMinBlocks, BS))
                      delvxeta * delvxeta * (1. - phieta * phieta) +
                      delvxzeta * delvxzeta * (1. - phizeta * phizeta));
         }
-        const double q_old_z = D.q[zidx];
         if (q_old_z > P.qstop) atomicMin(&T.bad_q, zidx);
         if (w.materialize()) {
             D.qq[zidx] = qquad;
@@ -956,7 +953,7 @@ __global__ void __launch_bounds__(BS, min_blocks(kEosMinBlocks, BS))
         if (eosvmax != 0.) {
             if (vnewc > eosvmax) vnewc = eosvmax;
         }
-        double vc = D.v[zidx];
+        double vc = v_z;
         if (eosvmin != 0.) {
             if (vc < eosvmin) vc = eosvmin;
         }
@@ -966,9 +963,6 @@ __global__ void __launch_bounds__(BS, min_blocks(kEosMinBlocks, BS))
         if (vc <= 0.) atomicMin(&T.bad_vol, zidx);
 
         double p_new = 0., e_new = 0., q_new = 0., bvc = 0., pbvc = 0.;
-        const double e_temp = D.e[zidx];
-        const double p_temp = D.p[zidx];
-        const double delvc_temp = D.delv[zidx];
         const double rho0 = P.refdens;
         // the reference density is 1.0 in every sedov problem (uniform branch)
         const bool rho1 = rho0 == 1.0;
@@ -999,36 +993,38 @@ __global__ void __launch_bounds__(BS, min_blocks(kEosMinBlocks, BS))
         // CalcTimeConstraintsForElems_kernel body, lulesh.cu:4246-4279
         const double qqc2 = 64.0 * P.qqc * P.qqc;
         const double vdov_tmp = vdov_z;
-        if (vdov_tmp != 0.) {
-            const double dtdvov = P.dvovmax / (fabs(vdov_tmp) + 1.e-20);
-            if (dth > dtdvov) dth = dtdvov;
-        }
+        vmax = fabs(vdov_tmp);
         const double ss_tmp = ssTmp;
-        const double area_tmp = D.arealg[zidx];
         double dtf = ss_tmp * ss_tmp;
         dtf += ((vdov_tmp < 0.) ? qqc2 * area_tmp * area_tmp * vdov_tmp * vdov_tmp : 0.);
-        dtf = area_tmp / sqrt(dtf);
+        dtf = area_tmp * rsqrt(dtf);
         if (vdov_tmp != 0. && dtf < dtc) dtc = dtf;
     }
-    // block minimum (exact, order-free), one atomic per block
-    __shared__ double s_c[BS / 32], s_h[BS / 32];
+    // block minimum (exact, order-free), one atomic per block.  The hydro
+    // limit dvovmax / (|vdov| + tiny) falls as |vdov| grows, also after
+    // rounding, so its minimum is that of the block's largest |vdov|: one
+    // division per block.
+    __shared__ double s_c[BS / 32], s_v[BS / 32];
     dtc = warp_min(dtc);
-    dth = warp_min(dth);
+    vmax = warp_max(vmax);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (lane == 0) {
         s_c[warp] = dtc;
-        s_h[warp] = dth;
+        s_v[warp] = vmax;
     }
     __syncthreads();
     if (threadIdx.x == 0) {
-        double c = s_c[0], h = s_h[0];
+        double c = s_c[0], v = s_v[0];
 #pragma unroll
-        for (int w = 1; w < BS / 32; ++w) {
-            c = fmin(c, s_c[w]);
-            h = fmin(h, s_h[w]);
+        for (int k = 1; k < BS / 32; ++k) {
+            c = fmin(c, s_c[k]);
+            v = fmax(v, s_v[k]);
         }
         if (c < 1.0e+20) atomicMin(&T.min_courant, dbits(c));
-        if (h < 1.0e+20) atomicMin(&T.min_hydro, dbits(h));
+        if (v != 0.) {
+            const double h = P.dvovmax / (v + 1.e-20);
+            if (h < 1.0e+20) atomicMin(&T.min_hydro, dbits(h));
+        }
     }
 }
 

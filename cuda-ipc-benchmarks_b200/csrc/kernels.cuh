@@ -35,8 +35,8 @@ constexpr int kNodeBlock = 128;  // threads per block, node kernels
 // Resident blocks per SM asked of the compiler (the register budget of the
 // element kernels), chosen by measurement on B200 at -s 100: force 3 (164
 // registers, 69.8 us; 86 us at 4 blocks with spills, 88 at 5), kinematics 5
-// (96 registers, 51.6 us; 57.8 at 4, and 2 us more at 6 with spills), EOS 12 (40 registers with small spills;
-// 134 us unbounded, 97 us at 8 blocks, 86 us at 12, 88 us at 16).
+// (96 registers, 51.6 us; 57.8 at 4, and 2 us more at 6 with spills), EOS 8
+// (64 registers, 55.9 us; 59.8 at 7 and at 10, 64.4 at 6, 72.5 at 12).
 #ifndef LULESH_FORCE_MINB
 #define LULESH_FORCE_MINB 3
 #endif
@@ -44,7 +44,7 @@ constexpr int kNodeBlock = 128;  // threads per block, node kernels
 #define LULESH_KIN_MINB 5
 #endif
 #ifndef LULESH_EOS_MINB
-#define LULESH_EOS_MINB 12
+#define LULESH_EOS_MINB 8
 #endif
 // nodal: 16 blocks (32 registers, every warp slot of the SM) for the
 // streaming corner gather, 60.2 -> 56.7 us
