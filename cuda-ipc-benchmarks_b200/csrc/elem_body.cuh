@@ -6,7 +6,6 @@
 
 #include <climits>
 
-#include "elem_math.cuh"
 #include "elem_modal.cuh"
 #include "kernels.cuh"
 
@@ -89,7 +88,7 @@ __device__ __forceinline__ void force_modal(const double (&xn)[8], const double 
     if (v < 0. || g.det < 0.) elem_error();
     const double press = (p + q) * (1.0 / 64.0);
     const double vol64 = (1.0 / 64.0) / det;
-    const double coef = HG ? -hourg * 0.01 * ss * mass * rcbrt(det) : 0.0;
+    const double coef = HG ? over_cbrt(-hourg * 0.01 * ss * mass, det) : 0.0;
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
         double vc[8], f[8];

@@ -30,7 +30,6 @@
 #include <type_traits>
 
 #include "elem_body.cuh"
-#include "elem_math.cuh"
 #include "kernels.cuh"
 #include "lulesh_b200.h"
 

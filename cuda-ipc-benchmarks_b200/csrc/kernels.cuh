@@ -87,6 +87,7 @@ struct SetArgs {
     // which the kernels then take by value (OneDomain, FewDomains)
     const DomDev *records = nullptr;
     int ndom = 0;
+    const CornerF32 *corner32 = nullptr;  // a mixed set's first domain (host side only)
 };
 
 // Where a block of a cycle kernel works: its domain's record, the time state

@@ -3,11 +3,12 @@
 //
 // FP32: the element-local stress / FB-hourglass arithmetic of
 //   CalcVolumeForceForElems_kernel (lulesh.cu:2080-2259) and the
-//   characteristic length, velocity gradient and monotonic-Q gradients of
-//   CalcKinematicsAndMonotonicQGradient_kernel (lulesh.cu:3343-3507).
-//   Every one of these is a function of coordinate DIFFERENCES, so the
-//   kernels form x[k] - x[0] in FP64 and hand FP32 only the small,
-//   well-conditioned differences; velocities go to FP32 directly.
+//   characteristic length, velocity divergence and monotonic-Q gradients of
+//   CalcKinematicsAndMonotonicQGradient_kernel (lulesh.cu:3343-3507), in the
+//   element's modes (elem_modal.cuh).  Every one of these is a function of
+//   coordinate and velocity DIFFERENCES, so the kernels form x[k] - x[0] and
+//   xd[k] - xd[0] in FP64 and hand FP32 only those: a velocity gradient then
+//   keeps FP32's digits where the flow is fast and its differences small.
 // FP32 storage, compensated sum: corner forces are stored as FP32 and each
 //   node adds its eight corners with Neumaier's compensated summation, then
 //   converts (sum + compensation) to FP64.
@@ -16,21 +17,25 @@
 //   digits), the node update, the EOS, and the dt reduction.
 #include <climits>
 
+#include <type_traits>
+
 #include "elem_math.cuh"
+#include "elem_modal.cuh"
 #include "kernels.cuh"
 
 namespace lulesh {
 
-// Resident blocks per SM asked of the compiler for the mixed kernels:
-// 4 (128 registers, no spills) measured best on B200 at -s 120, two
-// alternating runs each, identical results: force 137 us against 181 at 5
-// blocks (96 registers, spills), 147 at 3 and 311 at 6; kinematics 114.8 us
-// against 115.7 at 5 and 125.9 at 3; the cycle 498 us against 545 at 5.
+// Resident blocks per SM asked of the compiler for the mixed kernels, measured
+// on B200 at -s 120 (1.7e6 elements), identical results: force 5 (96
+// registers) 87 us, 94 at 3 and 4; kinematics 5 (94 registers) 78 us, the
+// same at 4 and 6.  The corner-by-corner forms took 131 us and 113 us at 128
+// registers.  What is left in both is the 48 gathers and their conversions to
+// FP32, and in the kinematics the FP64 volume.
 #ifndef LULESH_MIXED_FORCE_MINB
-#define LULESH_MIXED_FORCE_MINB 4
+#define LULESH_MIXED_FORCE_MINB 5
 #endif
 #ifndef LULESH_MIXED_KIN_MINB
-#define LULESH_MIXED_KIN_MINB 4
+#define LULESH_MIXED_KIN_MINB 5
 #endif
 
 __device__ __forceinline__ void elem_nodes_m(const DomDev &D, int el, int n[8])
@@ -48,18 +53,27 @@ __device__ __forceinline__ void elem_nodes_m(const DomDev &D, int el, int n[8])
     n[7] = n0 + en * en + en;
 }
 
-template <bool HG>
+// The FP32 corner arrays of a domain: by value with the domain's record, from
+// the device table otherwise.
+template <class W>
+__device__ __forceinline__ CornerF32 corner_arrays(const W &, const CornerF32 *table,
+                                                   const CornerF32 &one, int d)
+{
+    return W::kTable ? table[d] : one;
+}
+
+template <bool HG, class W>
 __global__ void __launch_bounds__(kElemBlock, LULESH_MIXED_FORCE_MINB)
-    k_force_mixed(SetArgs a, Params P, const CornerF32 *cfs)
+    k_force_mixed(const __grid_constant__ W w, Params P, const CornerF32 *cfs, CornerF32 cf1)
 {
     pdl_enter();
-    const int2 blk = a.blocks[blockIdx.x];
-    const DomDev &D = a.doms[blk.x];
-    TimeCtl &T = a.tcs[D.tc];
-    if (!T.active) return;
+    const int2 blk = w.template block<kElemBlock, false>();
+    const DomDev &D = w.domain(blk.x);
+    TimeCtl &T = w.time(D);
+    if (W::kTable && !T.active) return;
     const int elem = blk.y + threadIdx.x;
     if (elem >= D.numElem) return;
-    const CornerF32 cf = cfs[blk.x];
+    const CornerF32 cf = corner_arrays(w, cfs, cf1, blk.x);
 
     int n[8];
     elem_nodes_m(D, elem, n);
@@ -67,13 +81,14 @@ __global__ void __launch_bounds__(kElemBlock, LULESH_MIXED_FORCE_MINB)
     for (int i = 0; i < 8; ++i) n[i] = chk_index(n[i], D.numNode, &T, kChkNode);
     // all node gathers first: the velocities arrive while the coordinate
     // arithmetic runs
-    float vx[8], vy[8], vz[8];
+    float v[3][8];
+    if (HG) {
+        const double u0 = D.xd[n[0]], v0 = D.yd[n[0]], w0 = D.zd[n[0]];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        if (HG) {
-            vx[i] = (float)D.xd[n[i]];
-            vy[i] = (float)D.yd[n[i]];
-            vz[i] = (float)D.zd[n[i]];
+        for (int i = 0; i < 8; ++i) {
+            v[0][i] = (float)(D.xd[n[i]] - u0);
+            v[1][i] = (float)(D.yd[n[i]] - v0);
+            v[2][i] = (float)(D.zd[n[i]] - w0);
         }
     }
     const double x0 = D.x[n[0]], y0 = D.y[n[0]], z0 = D.z[n[0]];
@@ -85,50 +100,49 @@ __global__ void __launch_bounds__(kElemBlock, LULESH_MIXED_FORCE_MINB)
         zn[i] = (float)(D.z[n[i]] - z0);
     }
     const double volume = D.v[elem];
-    const double detd = D.volo[elem] * volume;
-    if (volume < 0.) atomicMin(&T.bad_vol, elem);
-    float det = (float)detd;
-    const float volinv = 1.0f / det;
-    const float coefficient =
-        (float)(-P.hgcoef * 0.01 * D.ss[elem] * D.elemMass[elem]) / cbrtf(det);
-    const float sigxx = (float)(-D.p[elem] - D.q[elem]);
+    const float det = (float)(D.volo[elem] * volume);
+    const float coef =
+        over_cbrt((float)(-P.hgcoef * 0.01 * D.ss[elem] * D.elemMass[elem]), det);
+    const float press = (float)(D.p[elem] + D.q[elem]) * (1.0f / 64.0f);
+    const float vol64 = (1.0f / 64.0f) / det;
+    if (!W::kTable && !T.active) return;
 
-    float dvdxn[8], dvdyn[8], dvdzn[8], hourgam[8][4];
-    elem_volume_derivative(dvdxn, dvdyn, dvdzn, xn, yn, zn);
-    hourglass_modes(xn, yn, zn, dvdxn, dvdyn, dvdzn, hourgam, volinv);
-    float B[3][8];
-    shape_function_derivatives(xn, yn, zn, B, &det);
-    elem_node_normals(B[0], B[1], B[2], xn, yn, zn);
-    if (det < 0.f) atomicMin(&T.bad_vol, elem);
-    float hgfx[8], hgfy[8], hgfz[8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        hgfx[i] = -(sigxx * B[0][i]);
-        hgfy[i] = -(sigxx * B[1][i]);
-        hgfz[i] = -(sigxx * B[2][i]);
-    }
-    if (HG) {
-        fb_hourglass_component(vx, hourgam, coefficient, hgfx);
-        fb_hourglass_component(vy, hourgam, coefficient, hgfy);
-        fb_hourglass_component(vz, hourgam, coefficient, hgfz);
-    }
+    ElemModes<float> m;
+    elem_modes(xn, yn, zn, m);
+    ForceGeometry<float> g;
+    force_geometry<float, HG>(m, g);
+    if (volume < 0. || g.det < 0.f) atomicMin(&T.bad_vol, elem);
     // written once, read once by the nodal gather: evict-first
     const int Ep = D.Ep;
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
-        __stcs(cf.fx + elem + Ep * k, hgfx[k]);
-        __stcs(cf.fy + elem + Ep * k, hgfy[k]);
-        __stcs(cf.fz + elem + Ep * k, hgfz[k]);
+    for (int c = 0; c < 3; ++c) {
+        float f[8];
+        force_component<float, HG>(m, g, c, v[c], press, vol64, coef, f);
+        float *to = (c == 0 ? cf.fx : c == 1 ? cf.fy : cf.fz) + elem;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) __stcs(to + Ep * k, f[k]);
     }
+}
+
+// launch(where, the only domain's corner arrays)
+template <class Launch>
+static void launch_mixed(const SetArgs &a, int nblocks, const Launch &launch)
+{
+    launch_where<true, false>(a, nblocks, [&](const auto &w) {
+        launch(w, a.corner32 ? *a.corner32 : CornerF32{});
+    });
 }
 
 void launch_force_mixed(const SetArgs &a, int nblocks, Params P, const CornerF32 *cf,
                         cudaStream_t s)
 {
-    if (P.hgcoef > 0.0)
-        launch_k(k_force_mixed<true>, nblocks, kElemBlock, s, a.pdl != 0, a, P, cf);
-    else
-        launch_k(k_force_mixed<false>, nblocks, kElemBlock, s, a.pdl != 0, a, P, cf);
+    launch_mixed(a, nblocks, [&](const auto &w, const CornerF32 &one) {
+        using W = std::decay_t<decltype(w)>;
+        if (P.hgcoef > 0.0)
+            launch_k(k_force_mixed<true, W>, nblocks, kElemBlock, s, a.pdl != 0, w, P, cf, one);
+        else
+            launch_k(k_force_mixed<false, W>, nblocks, kElemBlock, s, a.pdl != 0, w, P, cf, one);
+    });
 }
 
 // Neumaier's compensated addition: s + c carries the sum of all terms
@@ -150,17 +164,18 @@ __device__ __forceinline__ void comp_add(float &s, float &c, float v)
 #define LULESH_MIXED_NODAL_MINB 10
 #endif
 
+template <class W>
 __global__ void __launch_bounds__(kNodeBlock, min_blocks(LULESH_MIXED_NODAL_MINB, kNodeBlock))
-    k_nodal_mixed(SetArgs a, Params P, const CornerF32 *cfs)
+    k_nodal_mixed(const __grid_constant__ W w, Params P, const CornerF32 *cfs, CornerF32 cf1)
 {
     pdl_enter();
-    const int2 blk = a.blocks[blockIdx.x];
-    const DomDev &D = a.doms[blk.x];
-    const TimeCtl &T = a.tcs[D.tc];
-    if (!T.active) return;
+    const int2 blk = w.template block<kNodeBlock, LULESH_NODAL_REVERSE && !W::kTable>();
+    const DomDev &D = w.domain(blk.x);
+    TimeCtl &T = w.time(D);
+    if (W::kTable && !T.active) return;
     const int i = blk.y + threadIdx.x;
     if (i >= D.numNode) return;
-    const CornerF32 cf = cfs[blk.x];
+    const CornerF32 cf = corner_arrays(w, cfs, cf1, blk.x);
     const int en = D.en, nx = D.nx;
     const int px = i % en, t = i / en, py = t % en, pz = t / en;
     float sx = 0.f, sy = 0.f, sz = 0.f, cx = 0.f, cy = 0.f, cz = 0.f;
@@ -177,7 +192,7 @@ __global__ void __launch_bounds__(kNodeBlock, min_blocks(LULESH_MIXED_NODAL_MINB
         vx[j] = vy[j] = vz[j] = 0.f;
         if (in[j]) {
             const int idx = chk_index(j * D.Ep + (ez * nx + ey) * nx + ex, 8LL * D.Ep,
-                                      &a.tcs[D.tc], kChkCorner);
+                                      &T, kChkCorner);
             vx[j] = __ldcs(cf.fx + idx);
             vy[j] = __ldcs(cf.fy + idx);
             vz[j] = __ldcs(cf.fz + idx);
@@ -194,6 +209,7 @@ __global__ void __launch_bounds__(kNodeBlock, min_blocks(LULESH_MIXED_NODAL_MINB
     const double fx = (double)sx + (double)cx;
     const double fy = (double)sy + (double)cy;
     const double fz = (double)sz + (double)cz;
+    if (!W::kTable && !T.active) return;
     const double one_over_nMass = 1. / D.nodalMass[i];
     double xdd = fx * one_over_nMass, ydd = fy * one_over_nMass, zdd = fz * one_over_nMass;
     if (D.col == 0 && px == 0) xdd = 0.0;
@@ -212,7 +228,7 @@ __global__ void __launch_bounds__(kNodeBlock, min_blocks(LULESH_MIXED_NODAL_MINB
     D.xd[i] = xdtmp;
     D.yd[i] = ydtmp;
     D.zd[i] = zdtmp;
-    if (a.materialize) {
+    if (w.materialize()) {
         D.fx[i] = fx;
         D.fy[i] = fy;
         D.fz[i] = fz;
@@ -225,79 +241,87 @@ __global__ void __launch_bounds__(kNodeBlock, min_blocks(LULESH_MIXED_NODAL_MINB
 void launch_nodal_mixed(const SetArgs &a, int nblocks, Params P, const CornerF32 *cf,
                         cudaStream_t s)
 {
-    launch_k(k_nodal_mixed, nblocks, kNodeBlock, s, a.pdl != 0, a, P, cf);
+    launch_mixed(a, nblocks, [&](const auto &w, const CornerF32 &one) {
+        launch_k(k_nodal_mixed<std::decay_t<decltype(w)>>, nblocks, kNodeBlock, s, a.pdl != 0, w,
+                 P, cf, one);
+    });
 }
 
+template <class W>
 __global__ void __launch_bounds__(kElemBlock, LULESH_MIXED_KIN_MINB)
-    k_kinematics_mixed(SetArgs a, Params P)
+    k_kinematics_mixed(const __grid_constant__ W w)
 {
     pdl_enter();
-    const int2 blk = a.blocks[LULESH_KIN_REVERSE ? gridDim.x - 1 - blockIdx.x : blockIdx.x];
-    const DomDev &D = a.doms[blk.x];
-    TimeCtl &T = a.tcs[D.tc];
-    if (!T.active) return;
+    const int2 blk = w.template block<kElemBlock, LULESH_KIN_REVERSE>();
+    const DomDev &D = w.domain(blk.x);
+    TimeCtl &T = w.time(D);
+    if (W::kTable && !T.active) return;
     const int k = blk.y + threadIdx.x;
     if (k >= D.numElem) return;
-    int nodes[8];
-    elem_nodes_m(D, k, nodes);
+    int n[8];
+    elem_nodes_m(D, k, n);
 #pragma unroll
-    for (int l = 0; l < 8; ++l) nodes[l] = chk_index(nodes[l], D.numNode, &T, kChkNode);
-    // velocities gathered first (used after the FP64 volume)
-    float xv[8], yv[8], zv[8];
-#pragma unroll
-    for (int l = 0; l < 8; ++l) {
-        xv[l] = (float)D.xd[nodes[l]];
-        yv[l] = (float)D.yd[nodes[l]];
-        zv[l] = (float)D.zd[nodes[l]];
-    }
+    for (int l = 0; l < 8; ++l) n[l] = chk_index(n[l], D.numNode, &T, kChkNode);
     // FP64: volume and relative volume (they feed delv)
-    double xd64[8], yd64[8], zd64[8];
+    double x64[8], y64[8], z64[8];
 #pragma unroll
     for (int l = 0; l < 8; ++l) {
-        xd64[l] = D.x[nodes[l]];
-        yd64[l] = D.y[nodes[l]];
-        zd64[l] = D.z[nodes[l]];
+        x64[l] = D.x[n[l]];
+        y64[l] = D.y[n[l]];
+        z64[l] = D.z[n[l]];
     }
-    const double volume = elem_volume(xd64, yd64, zd64);
+    if (!W::kTable && !T.active) return;
+    const double volume = elem_volume(x64, y64, z64);
     const double relativeVolume = volume / D.volo[k];
     D.vnew[k] = relativeVolume;
     D.delv[k] = relativeVolume - D.v[k];
+    if (relativeVolume < 0) atomicMin(&T.bad_vol, k);
     // FP32: everything else, on coordinates relative to corner 0
     float xl[8], yl[8], zl[8];
 #pragma unroll
     for (int l = 0; l < 8; ++l) {
-        xl[l] = (float)(xd64[l] - xd64[0]);
-        yl[l] = (float)(yd64[l] - yd64[0]);
-        zl[l] = (float)(zd64[l] - zd64[0]);
+        xl[l] = (float)(x64[l] - x64[0]);
+        yl[l] = (float)(y64[l] - y64[0]);
+        zl[l] = (float)(z64[l] - z64[0]);
     }
-    D.arealg[k] = (double)elem_characteristic_length(xl, yl, zl, (float)volume);
-    const float dt2 = (float)(0.5 * T.deltatime);
-    float xh[8], yh[8], zh[8];
+    const float vol = (float)volume;
+    ElemModes<float> m;
+    elem_modes(xl, yl, zl, m);
+    FaceCrosses<float> c;
+    face_crosses(m, c);
+    D.arealg[k] = (double)modal_length(m, c, vol);
+    // the velocities' A, B, C modes are all the step needs
+    float va[3], vb[3], vc[3];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-        xh[j] = xl[j] - dt2 * xv[j];
-        yh[j] = yl[j] - dt2 * yv[j];
-        zh[j] = zl[j] - dt2 * zv[j];
+    for (int c = 0; c < 3; ++c) {
+        const double *from = c == 0 ? D.xd : c == 1 ? D.yd : D.zd;
+        const double v0 = from[n[0]];
+        float v[8], vg;
+#pragma unroll
+        for (int l = 0; l < 8; ++l) v[l] = (float)(from[n[l]] - v0);
+        odd_modes(v, va[c], vb[c], vc[c], vg);
     }
-    float B[3][8], detJ, Dv[3];
-    shape_function_derivatives(xh, yh, zh, B, &detJ);
-    elem_velocity_divergence(xv, yv, zv, B, detJ, Dv);
-    D.vdov[k] = (double)(Dv[0] + Dv[1] + Dv[2]);
-    const float vol = (float)(D.volo[k] * relativeVolume);
-    float dxz, dvz, dxx, dvx, dxe, dve;
-    mono_gradient(xl, yl, zl, xv, yv, zv, vol, &dxz, &dvz, &dxx, &dvx, &dxe, &dve);
-    D.delx_zeta[k] = dxz;
-    D.delv_zeta[k] = dvz;
-    D.delx_xi[k] = dxx;
-    D.delv_xi[k] = dvx;
-    D.delx_eta[k] = dxe;
-    D.delv_eta[k] = dve;
-    if (relativeVolume < 0) atomicMin(&T.bad_vol, k);
+    D.vdov[k] = (double)modal_divergence(m, va, vb, vc, (float)(0.5 * T.deltatime));
+    const float norm = 1.0f / (vol + 1.e-36f);
+    float delx, delv;
+    modal_mono(c.ab, vc, vol, norm, &delx, &delv);
+    D.delx_zeta[k] = delx;
+    D.delv_zeta[k] = delv;
+    modal_mono(c.bc, va, vol, norm, &delx, &delv);
+    D.delx_xi[k] = delx;
+    D.delv_xi[k] = delv;
+    modal_mono(c.ca, vb, vol, norm, &delx, &delv);
+    D.delx_eta[k] = delx;
+    D.delv_eta[k] = delv;
 }
 
 void launch_kinematics_mixed(const SetArgs &a, int nblocks, Params P, cudaStream_t s)
 {
-    launch_k(k_kinematics_mixed, nblocks, kElemBlock, s, a.pdl != 0, a, P);
+    (void)P;
+    launch_where<true, false>(a, nblocks, [&](const auto &w) {
+        launch_k(k_kinematics_mixed<std::decay_t<decltype(w)>>, nblocks, kElemBlock, s,
+                 a.pdl != 0, w);
+    });
 }
 
 }  // namespace lulesh

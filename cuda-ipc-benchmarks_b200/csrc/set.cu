@@ -268,6 +268,7 @@ static int create_common(lulesh_set *s, const std::vector<DomPlace> &place, int 
     if (mixed)
         LCHECK(cudaMemcpyAsync(s->dcorner32, hc32.data(), sizeof(CornerF32) * s->ndom,
                                cudaMemcpyHostToDevice, s->stream));
+    if (mixed) s->hcorner32 = hc32;
 
     // time control blocks
     std::vector<TimeCtl> tc(s->njobs);

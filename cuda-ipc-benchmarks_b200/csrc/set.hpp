@@ -65,6 +65,7 @@ struct lulesh_set {
 
     // mixed precision corner buffers
     lulesh::CornerF32 *dcorner32 = nullptr;
+    std::vector<lulesh::CornerF32> hcorner32;  // host copy
 
     // L2 access-policy window set on `stream` (single domains)
     bool l2_window = false;
@@ -135,6 +136,7 @@ struct lulesh_set {
         a.records = nparts == 1 && njobs == 1 && (ndom == 1 || ndom == lulesh::kFewDomains)
                         ? hdoms.data()
                         : nullptr;
+        a.corner32 = hcorner32.empty() ? nullptr : hcorner32.data();
         return a;
     }
 };

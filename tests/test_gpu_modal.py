@@ -44,3 +44,17 @@ def test_distorted_elements_match_the_oracle(lulesh, oracle_mod, nx, warp):
             diff, scale = np.max(np.abs(g[:m] - o[:m])), np.max(np.abs(o[:m]))
             assert diff <= RTOL * scale, (f, diff, scale)
     orc.close()
+
+
+@pytest.mark.parametrize("sizes", [(1, 7), (5, 13), (32, 2)])
+def test_mixed_records_by_value_and_by_table(lulesh, sizes):
+    """A mixed single domain takes its record by value, a mixed batch from the
+    table: the same kernels' arithmetic, the same bits."""
+    jobs = [lulesh.JobSpec(nx, its=15) for nx in sizes]
+    with lulesh.LuleshSet.batch(jobs, flags=lulesh.FLAG_MIXED) as b:
+        assert b.run() == lulesh.OK
+        for j, spec in enumerate(jobs):
+            with lulesh.LuleshSet(nx=spec.nx, its=15, flags=lulesh.FLAG_MIXED) as s:
+                assert s.run() == lulesh.OK
+                for f in ("e", "p", "q", "v", "ss", "x", "y", "z", "xd", "yd", "zd"):
+                    assert np.array_equal(b.field(f, j), s.field(f)), (spec.nx, f)
