@@ -43,12 +43,8 @@ __device__ __forceinline__ unsigned long long dbits(double v)
     return (unsigned long long)__double_as_longlong(v);
 }
 
-__global__ void k_time_increment(TimeCtl *tcs, int ntc, Params P)
+__device__ __forceinline__ void time_increment(TimeCtl &T, const Params &P)
 {
-    pdl_enter();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= ntc) return;
-    TimeCtl &T = tcs[i];
     T.active = 0;
     if (T.done) return;
     // checkErrors (lulesh.cu:2879-2892): a cycle that raised an error ends
@@ -111,6 +107,13 @@ __global__ void k_time_increment(TimeCtl *tcs, int ntc, Params P)
     T.active = 1;
 }
 
+__global__ void k_time_increment(TimeCtl *tcs, int ntc, Params P)
+{
+    pdl_enter();
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < ntc) time_increment(tcs[i], P);
+}
+
 void launch_time_increment(TimeCtl *tcs, int ntc, Params P, cudaStream_t s, bool pdl)
 {
     const int b = 128;
@@ -127,6 +130,61 @@ __device__ __constant__ int kCY[8] = {0, 0, 1, 1, 0, 0, 1, 1};
 __device__ __constant__ int kCZ[8] = {0, 0, 0, 0, 1, 1, 1, 1};
 
 // ---------------------------------------------------------------------------
+// scattered meshes
+
+// 32 bytes in one access (32-byte aligned); the volatile form keeps its place
+// after griddepcontrol.wait
+__device__ __forceinline__ void ld4(const double *p, double &a, double &b, double &c, double &d)
+{
+    asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];"
+                 : "=d"(a), "=d"(b), "=d"(c), "=d"(d)
+                 : "l"(p));
+}
+
+__device__ __forceinline__ void st4(double *p, double a, double b, double c, double d)
+{
+    asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(a), "d"(b), "d"(c),
+                 "d"(d)
+                 : "memory");
+}
+
+__device__ __forceinline__ void load_node(const DomDev &D, int n, double &x, double &y, double &z,
+                                          double &xd, double &yd, double &zd)
+{
+    const double *p = D.nodePack + 8 * (size_t)n;
+    ld4(p, x, y, z, xd);
+    const double2 t = *reinterpret_cast<const double2 *>(p + 4);
+    yd = t.x;
+    zd = t.y;
+}
+
+__device__ __forceinline__ void store_node(const DomDev &D, int n, double x, double y, double z,
+                                           double xd, double yd, double zd)
+{
+    double *p = D.nodePack + 8 * (size_t)n;
+    st4(p, x, y, z, xd);
+    *reinterpret_cast<double2 *>(p + 4) = make_double2(yd, zd);
+}
+
+// Start of a scattered mesh's cycle: the time increment, and every node's six
+// values side by side.  Packed anew each cycle, so what the caller wrote to
+// the node arrays between cycles counts.
+__global__ void __launch_bounds__(kNodeBlock)
+    k_begin_packed(const __grid_constant__ OneDomain w, Params P)
+{
+    pdl_enter();
+    const DomDev &D = w.D[0];
+    const int i = blockIdx.x * kNodeBlock + threadIdx.x;
+    if (i == 0) time_increment(*w.tc, P);
+    if (i < D.numNode) store_node(D, i, D.x[i], D.y[i], D.z[i], D.xd[i], D.yd[i], D.zd[i]);
+}
+
+void launch_begin_packed(const SetArgs &a, int nblocks, Params P, cudaStream_t s)
+{
+    launch_k(k_begin_packed, nblocks, kNodeBlock, s, a.pdl != 0, by_value<1>(a, nblocks), P);
+}
+
+// ---------------------------------------------------------------------------
 // force: CalcVolumeForceForElems_kernel, lulesh.cu:2080-2259
 
 // One element of the force phase: the node gathers, then force_modal.
@@ -140,32 +198,38 @@ __device__ __constant__ int kCZ[8] = {0, 0, 0, 0, 1, 1, 1, 1};
 // velocities gathered component by component, where force_modal asks for
 // them, the kernel fits 128 registers (16 warps) but took 73 against 70 us,
 // and 312 against 272 us at -s 160.
-template <bool HG, bool U, bool TABLE>
+template <bool HG, Mesh M, bool TABLE>
 __device__ __forceinline__ void force_one(const DomDev &D, TimeCtl &T, const Params &P, int elem)
 {
     int n[8];
-    elem_nodes<U>(D, elem, n);
+    elem_nodes<M != Mesh::kBox>(D, elem, n);
 #pragma unroll
     for (int i = 0; i < 8; ++i) n[i] = chk_index(n[i], D.numNode, &T, kChkNode);
-    double vn[3][8];
+    double vn[3][8], xn[8], yn[8], zn[8];
+    if constexpr (M == Mesh::kPacked) {
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        if (HG) {
-            vn[0][i] = D.xd[n[i]];
-            vn[1][i] = D.yd[n[i]];
-            vn[2][i] = D.zd[n[i]];
-        } else {
-            vn[0][i] = vn[1][i] = vn[2][i] = 0.0;
+        for (int i = 0; i < 8; ++i)
+            load_node(D, n[i], xn[i], yn[i], zn[i], vn[0][i], vn[1][i], vn[2][i]);
+    } else {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            if (HG) {
+                vn[0][i] = D.xd[n[i]];
+                vn[1][i] = D.yd[n[i]];
+                vn[2][i] = D.zd[n[i]];
+            } else {
+                vn[0][i] = vn[1][i] = vn[2][i] = 0.0;
+            }
         }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) xn[i] = D.x[n[i]];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) yn[i] = D.y[n[i]];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) zn[i] = D.z[n[i]];
     }
-    double xn[8], yn[8], zn[8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) xn[i] = D.x[n[i]];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) yn[i] = D.y[n[i]];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) zn[i] = D.z[n[i]];
     if (!TABLE && !T.active) return;
+    double fx[8], fy[8];  // held for cornerPack, whose corners take all three
     force_modal<HG>(
         xn, yn, zn, D.volo[elem], D.v[elem], D.p[elem], D.q[elem], D.ss[elem], D.elemMass[elem],
         P.hgcoef,
@@ -173,11 +237,23 @@ __device__ __forceinline__ void force_one(const DomDev &D, TimeCtl &T, const Par
 #pragma unroll
             for (int i = 0; i < 8; ++i) v[i] = vn[c][i];
         },
-        CornerStore{D.fx_elem, D.fy_elem, D.fz_elem, elem, D.Ep},
+        [&](int c, const double (&f)[8]) {
+            if constexpr (M == Mesh::kPacked) {
+                double *p = D.cornerPack + 32 * (size_t)elem;
+#pragma unroll
+                for (int k = 0; k < 8; ++k) {
+                    if (c == 0) fx[k] = f[k];
+                    if (c == 1) fy[k] = f[k];
+                    if (c == 2) st4(p + 4 * k, fx[k], fy[k], f[k], 0.0);
+                }
+            } else {
+                CornerStore{D.fx_elem, D.fy_elem, D.fz_elem, elem, D.Ep}(c, f);
+            }
+        },
         [&] { atomicMin(&T.bad_vol, elem); });
 }
 
-template <bool HG, int BS, bool U, class W>
+template <bool HG, int BS, Mesh M, class W>
 __global__ void __launch_bounds__(BS, min_blocks(kForceMinBlocks, BS))
     k_force(const __grid_constant__ W w, Params P)
 {
@@ -188,30 +264,34 @@ __global__ void __launch_bounds__(BS, min_blocks(kForceMinBlocks, BS))
     if (W::kTable && !T.active) return;
     const int elem = blk.y + threadIdx.x;
     if (elem >= D.numElem) return;
-    force_one<HG, U, W::kTable>(D, T, P, elem);
+    force_one<HG, M, W::kTable>(D, T, P, elem);
 }
 
-template <int BS, bool U, class W>
+template <int BS, Mesh M, class W>
 static void launch_force_w(const W &w, bool pdl, int nblocks, Params P, cudaStream_t s)
 {
     if (P.hgcoef > 0.0)
-        launch_k(k_force<true, BS, U, W>, nblocks, BS, s, pdl, w, P);
+        launch_k(k_force<true, BS, M, W>, nblocks, BS, s, pdl, w, P);
     else
-        launch_k(k_force<false, BS, U, W>, nblocks, BS, s, pdl, w, P);
+        launch_k(k_force<false, BS, M, W>, nblocks, BS, s, pdl, w, P);
 }
 
 template <int BS>
 static void launch_force_bs(const SetArgs &a, int nblocks, Params P, cudaStream_t s)
 {
     launch_where<true, BS == kElemBlock>(a, nblocks, [&](const auto &w) {
-        launch_force_w<BS, false>(w, a.pdl != 0, nblocks, P, s);
+        launch_force_w<BS, Mesh::kBox>(w, a.pdl != 0, nblocks, P, s);
     });
 }
 
 void launch_force(const SetArgs &a, int nblocks, Params P, cudaStream_t s, int bs, bool u)
 {
     if (u) {  // an lmesh set is one domain
-        launch_force_w<kElemBlock, true>(by_value<1>(a, nblocks), a.pdl != 0, nblocks, P, s);
+        const OneDomain w = by_value<1>(a, nblocks);
+        if (w.D[0].nodePack)
+            launch_force_w<kElemBlock, Mesh::kPacked>(w, a.pdl != 0, nblocks, P, s);
+        else
+            launch_force_w<kElemBlock, Mesh::kLists>(w, a.pdl != 0, nblocks, P, s);
         return;
     }
     switch (bs) {
@@ -287,7 +367,7 @@ __device__ __forceinline__ void gather_corners(const DomDev *doms, const DomDev 
 // 2999-3028) for node i with the summed force (fx, fy, fz)
 __device__ __forceinline__ void advance_node(const DomDev &D, const TimeCtl &T, const Params &P,
                                              int i, int bc, double fx, double fy, double fz,
-                                             int materialize, bool write_f)
+                                             int materialize, bool write_f, bool pack = false)
 {
     const double one_over_nMass = 1. / D.nodalMass[i];
     double xdd = fx * one_over_nMass;
@@ -305,12 +385,16 @@ __device__ __forceinline__ void advance_node(const DomDev &D, const TimeCtl &T, 
     if (fabs(xdtmp) < u_cut) xdtmp = 0.0;
     if (fabs(ydtmp) < u_cut) ydtmp = 0.0;
     if (fabs(zdtmp) < u_cut) zdtmp = 0.0;
-    D.x[i] += xdtmp * dt;
-    D.y[i] += ydtmp * dt;
-    D.z[i] += zdtmp * dt;
+    const double x = D.x[i] + xdtmp * dt;
+    const double y = D.y[i] + ydtmp * dt;
+    const double z = D.z[i] + zdtmp * dt;
+    D.x[i] = x;
+    D.y[i] = y;
+    D.z[i] = z;
     D.xd[i] = xdtmp;
     D.yd[i] = ydtmp;
     D.zd[i] = zdtmp;
+    if (pack) store_node(D, i, x, y, z, xdtmp, ydtmp, zdtmp);
     if (materialize) {
         if (write_f) {
             D.fx[i] = fx;
@@ -366,6 +450,40 @@ __global__ void __launch_bounds__(BS, min_blocks(kNodalMinBlocks, BS))
                    (D.plane == 0 && pz == 0 ? 4 : 0);
     if (!W::kTable && !T.active) return;
     advance_node(D, T, P, i, bc, fx, fy, fz, w.materialize(), MODE == 0);
+}
+
+// Scattered meshes: the corner forces of a node, one sector each, summed in
+// run order, then the node update.
+__global__ void __launch_bounds__(kNodeBlock)
+    k_nodal_packed(const __grid_constant__ OneDomain w, Params P)
+{
+    pdl_enter();
+    const DomDev &D = w.D[0];
+    TimeCtl &T = *w.tc;
+    const int i = blockIdx.x * kNodeBlock + threadIdx.x;
+    if (i >= D.numNode) return;
+    int k[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) k[j] = D.packedCornerEll[(size_t)j * D.numNode + i];
+    double vx[8], vy[8], vz[8], pad;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        vx[j] = vy[j] = vz[j] = 0.0;
+        if (k[j] >= 0)
+            ld4(D.cornerPack + 4 * (size_t)chk_index(k[j], 8LL * D.Ep, &T, kChkCorner), vx[j],
+                vy[j], vz[j], pad);
+    }
+    if (!T.active) return;
+    double fx = 0.0, fy = 0.0, fz = 0.0;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        if (k[j] >= 0) {  // a run is a prefix of the slots
+            fx += vx[j];
+            fy += vy[j];
+            fz += vz[j];
+        }
+    }
+    advance_node(D, T, P, i, D.nodeBC[i], fx, fy, fz, w.mat, true, /*pack=*/true);
 }
 
 // Unstructured meshes: AddNodeForcesFromElems (lulesh.cu:1715-1751) over
@@ -485,8 +603,9 @@ static void launch_nodal_bs(const SetArgs &a, int nblocks, Params P, cudaStream_
 void launch_nodal(const SetArgs &a, int nblocks, Params P, cudaStream_t s, int bs, bool u)
 {
     if (u) {
-        launch_k(k_nodal_u<kNodeBlock>, nblocks, kNodeBlock, s, a.pdl != 0,
-                 by_value<1>(a, nblocks), P);
+        const OneDomain w = by_value<1>(a, nblocks);
+        launch_k(w.D[0].nodePack ? k_nodal_packed : k_nodal_u<kNodeBlock>, nblocks, kNodeBlock, s,
+                 a.pdl != 0, w, P);
         return;
     }
     switch (bs) {
@@ -517,8 +636,9 @@ void launch_nodal_update(const SetArgs &a, int nblocks, Params P, cudaStream_t s
 // and length stores, at 96 registers (5 blocks); 6 us more at 4 blocks.  Up
 // front took 8 us more at 3 blocks, and between the coordinates and the volume
 // 2 us more at 4 blocks and 4 at 5 (with spills).
-template <int BS, bool U, class W>
-__global__ void __launch_bounds__(BS, min_blocks(kKinMinBlocks, BS))
+template <int BS, Mesh M, class W>
+__global__ void __launch_bounds__(BS, min_blocks(M == Mesh::kPacked ? kKinPackedMinBlocks
+                                                                    : kKinMinBlocks, BS))
     k_kinematics(const __grid_constant__ W w)
 {
     pdl_enter();
@@ -530,29 +650,42 @@ __global__ void __launch_bounds__(BS, min_blocks(kKinMinBlocks, BS))
     if (k >= D.numElem) return;
 
     int n[8];
-    elem_nodes<U>(D, k, n);
+    elem_nodes<M != Mesh::kBox>(D, k, n);
 #pragma unroll
     for (int l = 0; l < 8; ++l) n[l] = chk_index(n[l], D.numNode, &T, kChkNode);
     double xn[8], yn[8], zn[8];
+    if constexpr (M == Mesh::kPacked) {
+        double vn[3][8];
 #pragma unroll
-    for (int l = 0; l < 8; ++l) xn[l] = D.x[n[l]];
+        for (int l = 0; l < 8; ++l)
+            load_node(D, n[l], xn[l], yn[l], zn[l], vn[0][l], vn[1][l], vn[2][l]);
+        if (!W::kTable && !T.active) return;
+        kin_modal(D, T, k, xn, yn, zn, [&](int c, double (&v)[8]) {
 #pragma unroll
-    for (int l = 0; l < 8; ++l) yn[l] = D.y[n[l]];
+            for (int l = 0; l < 8; ++l) v[l] = vn[c][l];
+        });
+        return;
+    } else {
 #pragma unroll
-    for (int l = 0; l < 8; ++l) zn[l] = D.z[n[l]];
-    if (!W::kTable && !T.active) return;
-    kin_modal(D, T, k, xn, yn, zn, [&](int c, double (&v)[8]) {
-        const double *a = c == 0 ? D.xd : c == 1 ? D.yd : D.zd;
+        for (int l = 0; l < 8; ++l) xn[l] = D.x[n[l]];
 #pragma unroll
-        for (int l = 0; l < 8; ++l) v[l] = a[n[l]];
-    });
+        for (int l = 0; l < 8; ++l) yn[l] = D.y[n[l]];
+#pragma unroll
+        for (int l = 0; l < 8; ++l) zn[l] = D.z[n[l]];
+        if (!W::kTable && !T.active) return;
+        kin_modal(D, T, k, xn, yn, zn, [&](int c, double (&v)[8]) {
+            const double *a = c == 0 ? D.xd : c == 1 ? D.yd : D.zd;
+#pragma unroll
+            for (int l = 0; l < 8; ++l) v[l] = a[n[l]];
+        });
+    }
 }
 
 template <int BS>
 static void launch_kinematics_bs(const SetArgs &a, int nblocks, cudaStream_t s)
 {
     launch_where<true, BS == kElemBlock>(a, nblocks, [&](const auto &w) {
-        launch_k(k_kinematics<BS, false, std::decay_t<decltype(w)>>, nblocks, BS, s, a.pdl != 0,
+        launch_k(k_kinematics<BS, Mesh::kBox, std::decay_t<decltype(w)>>, nblocks, BS, s, a.pdl != 0,
                  w);
     });
 }
@@ -561,8 +694,10 @@ void launch_kinematics(const SetArgs &a, int nblocks, Params P, cudaStream_t s, 
 {
     (void)P;
     if (u) {
-        launch_k(k_kinematics<kElemBlock, true, OneDomain>, nblocks, kElemBlock, s, a.pdl != 0,
-                 by_value<1>(a, nblocks));
+        const OneDomain w = by_value<1>(a, nblocks);
+        launch_k(w.D[0].nodePack ? k_kinematics<kElemBlock, Mesh::kPacked, OneDomain>
+                                 : k_kinematics<kElemBlock, Mesh::kLists, OneDomain>,
+                 nblocks, kElemBlock, s, a.pdl != 0, w);
         return;
     }
     switch (bs) {

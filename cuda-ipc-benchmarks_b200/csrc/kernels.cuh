@@ -59,6 +59,11 @@ constexpr int kNodalMinBlocks = LULESH_NODAL_MINB;
 constexpr int kNodalUMinBlocks = LULESH_NODAL_U_MINB;
 constexpr int kForceMinBlocks = LULESH_FORCE_MINB;
 constexpr int kKinMinBlocks = LULESH_KIN_MINB;
+// packed meshes: 128 registers, 12.6 us at -s 40; 14.8 at 3 and 5 blocks
+#ifndef LULESH_KIN_PACKED_MINB
+#define LULESH_KIN_PACKED_MINB 4
+#endif
+constexpr int kKinPackedMinBlocks = LULESH_KIN_PACKED_MINB;
 constexpr int kEosMinBlocks = LULESH_EOS_MINB;
 
 // Minimum resident blocks of a kernel launched with BS threads per block
@@ -72,6 +77,11 @@ constexpr int min_blocks(int minb, int bs)
 // nodal kernel are compiled for; a set's block tables use one of each.
 constexpr bool valid_elem_block(int bs) { return bs == 64 || bs == 128 || bs == 256; }
 constexpr bool valid_node_block(int bs) { return bs == 128 || bs == 256 || bs == 512; }
+
+// What the element kernels read the mesh from: the element's position in a
+// structured box, an unstructured mesh's lists, or those lists and the packed
+// nodes and corners of a scattered mesh.
+enum class Mesh { kBox, kLists, kPacked };
 
 // A kernel launch over all domains of a set: block b works on domain
 // blocks[b].x starting at item blocks[b].y (element, node or region slot).
@@ -233,6 +243,8 @@ inline void launch_k(void (*kernel)(KArgs...), int grid, int block, cudaStream_t
     cudaLaunchKernelEx(&cfg, kernel, args...);  // errors: cudaGetLastError
 }
 
+// start of a scattered mesh's cycle: time increment and node packing (node blocks)
+void launch_begin_packed(const SetArgs &a, int nblocks, Params P, cudaStream_t s);
 void launch_time_increment(TimeCtl *tcs, int ntc, Params P, cudaStream_t s, bool pdl = false);
 // u: the set's domains are unstructured (lmesh): 128-wide blocks, mesh
 // arrays read instead of structured indexing

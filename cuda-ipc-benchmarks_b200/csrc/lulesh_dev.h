@@ -93,6 +93,13 @@ struct DomDev {
     // null when some node has more than 8 corners (the kernel then reads the
     // run from nodeElemCornerList)
     int *nodeCornerEll;
+    // scattered unstructured meshes (pack_scattered_mesh, set.cu), else null:
+    // node i's x, y, z, xd, yd, zd at nodePack + 8*i (two 32-byte sectors),
+    // packed at the start of every cycle; corner k of element e's force at
+    // cornerPack + 4*(8*e + k) (one sector); packedCornerEll is nodeCornerEll
+    // with 8*e + k in place of e + Ep*k
+    double *nodePack, *cornerPack;
+    int *packedCornerEll;
 };
 
 // Mixed-precision corner forces, FP32, layout of fx_elem ([8][Ep]).

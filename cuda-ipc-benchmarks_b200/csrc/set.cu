@@ -131,6 +131,62 @@ struct DomPlace {
     int job, tp, col, row, plane, rank;
 };
 
+// Distinct 32-byte sectors a warp's gather of one corner of 32 elements
+// touches in a node array, on average: 9 in a box's own numbering, 32 when
+// neighbouring elements' nodes lie anywhere.
+static double gather_sectors(const HostDomain &h)
+{
+    long long sectors = 0, gathers = 0;
+    for (int k = 0; k < 8; ++k)
+        for (int e = 0; e < h.numElem; e += 32) {
+            int seen[32], n = 0;
+            for (int i = e; i < std::min(e + 32, h.numElem); ++i) {
+                const int s = h.nodelist[(size_t)k * h.Ep + i] / 4;
+                if (std::find(seen, seen + n, s) == seen + n) seen[n++] = s;
+            }
+            sectors += n;
+            ++gathers;
+        }
+    return gathers ? (double)sectors / (double)gathers : 0.0;
+}
+
+// A mesh whose gathers are scattered moves a 32-byte sector for every 8-byte
+// node or corner value; packed (DomDev::nodePack), two sectors hold a node's
+// six values and one a corner's three.  The line lies at 28 sectors a gather,
+// measured on B200 (us per cycle, lists against packed):
+//    9 sectors, a box's own order        -s 40 30.8 / 36.9   -s 64 63.6 / 96.3
+//   25, nodes shuffled in runs of 256    -s 40 39.2 / 39.1   -s 64 82.0 / 106.5
+//   30, all shuffled in runs of 1024     -s 40 56.6 / 41.2   -s 64 128 / 113
+//   32, random nodes                     -s 40 59.5 / 39.1   -s 64 152 / 107
+//   32, random nodes and elements        -s 40 74.0 / 42.9   -s 64 192 / 116
+// (near neighbours still meet in L1, so few shuffled meshes gain below it).
+#ifndef LULESH_PACK_SECTORS
+#define LULESH_PACK_SECTORS 28.0
+#endif
+static int pack_scattered_mesh(lulesh_set *s, const HostDomain &h, DomDev &D)
+{
+    if (!D.nodeCornerEll || (s->flags & LULESH_FLAG_MATERIALIZE) ||
+        gather_sectors(h) < LULESH_PACK_SECTORS)
+        return LULESH_OK;
+    const size_t N = D.numNode, nodes = 8 * N, corners = 32 * (size_t)D.Ep;  // doubles
+    if (cudaMalloc(&s->pack, sizeof(double) * (nodes + corners) + sizeof(int) * 8 * N) !=
+        cudaSuccess) {
+        (void)cudaGetLastError();  // not enough memory for both: run from the lists
+        s->pack = nullptr;
+        return LULESH_OK;
+    }
+    D.nodePack = static_cast<double *>(s->pack);
+    D.cornerPack = D.nodePack + nodes;
+    D.packedCornerEll = reinterpret_cast<int *>(D.cornerPack + corners);
+    std::vector<int> at(h.nodeCornerEll);
+    for (int &c : at)
+        if (c >= 0) c = 8 * (c % D.Ep) + c / D.Ep;
+    LCHECK(cudaMemcpyAsync(D.packedCornerEll, at.data(), sizeof(int) * at.size(),
+                           cudaMemcpyHostToDevice, s->stream));
+    LCHECK(cudaStreamSynchronize(s->stream));
+    return LULESH_OK;
+}
+
 static int create_common(lulesh_set *s, const std::vector<DomPlace> &place, int device)
 {
     if (device >= 0) LCHECK(cudaSetDevice(device));
@@ -217,6 +273,7 @@ static int create_common(lulesh_set *s, const std::vector<DomPlace> &place, int 
         int su = upload_domain(h, pl.job, commd[d], mixed, cv, s->stream, &D, &hc32[d],
                                node_region ? &ncv : nullptr);
         if (su != LULESH_OK) return su;
+        if (s->unstructured && (su = pack_scattered_mesh(s, h, D)) != LULESH_OK) return su;
         s->hdoms[d] = D;
         s->dom_rank[d] = pl.rank;
         s->dom_job[d] = pl.job;
@@ -293,6 +350,14 @@ static int create_common(lulesh_set *s, const std::vector<DomPlace> &place, int 
     return LULESH_OK;
 }
 
+void launch_begin(lulesh_set *s, cudaStream_t st)
+{
+    if (s->pack)
+        launch_begin_packed(s->args(s->node_blocks), s->n_node_blocks, s->P, st);
+    else
+        launch_time_increment(s->dtc, s->njobs, s->P, st, s->pdl);
+}
+
 void launch_force_fp64(lulesh_set *s, cudaStream_t st)
 {
     launch_force(s->args(s->elem_blocks), s->n_elem_blocks, s->P, st, s->eb, s->unstructured);
@@ -303,7 +368,7 @@ int enqueue_cycle(lulesh_set *s)
     if (s->flags & LULESH_FLAG_COMM_STAGED) return enqueue_cycle_staged(s);
     cudaStream_t st = s->stream;
     const bool mixed = (s->flags & LULESH_FLAG_MIXED) != 0;
-    launch_time_increment(s->dtc, s->njobs, s->P, st, s->pdl);
+    launch_begin(s, st);
     if (mixed)
         launch_force_mixed(s->args(s->elem_blocks), s->n_elem_blocks, s->P, s->dcorner32, st);
     else
@@ -801,6 +866,7 @@ int lulesh_destroy(lulesh_set *s)
     if (s->htc_pinned) cudaFreeHost(s->htc_pinned);
     if (s->dcorner32) cudaFree(s->dcorner32);
     if (s->run_ctl) cudaFree(s->run_ctl);
+    if (s->pack) cudaFree(s->pack);
     if (s->arena) cudaFree(s->arena);
     if (s->own_stream && s->stream) cudaStreamDestroy(s->stream);
     delete s;
@@ -950,7 +1016,7 @@ int lulesh_profile_phases(lulesh_set *s, int ncycles, double *ms_out, int *nphas
     const bool mixed = (s->flags & LULESH_FLAG_MIXED) != 0;
     for (int c = 0; c < ncycles; ++c) {
         LCHECK(cudaEventRecord(ev[0], st));
-        launch_time_increment(s->dtc, s->njobs, s->P, st, s->pdl);
+        launch_begin(s, st);
         LCHECK(cudaEventRecord(ev[1], st));
         if (mixed)
             launch_force_mixed(s->args(s->elem_blocks), s->n_elem_blocks, s->P, s->dcorner32, st);

@@ -76,6 +76,7 @@ struct lulesh_set {
     // domain's x..zd, node_region_bytes), single domains carve in place
     void *arena = nullptr;
     size_t arena_bytes = 0;
+    void *pack = nullptr;  // nodePack and cornerPack of a scattered mesh
     size_t node_region_bytes = 0;
 
     // captured cycle, and a graph of graph_cycles consecutive cycles
@@ -146,6 +147,8 @@ void set_error(const std::string &msg);
 int cuda_status(cudaError_t e, const char *what);
 // enqueue one cycle (no graph)
 int enqueue_cycle(lulesh_set *s);
+// the start of a cycle: the time increment (and a scattered mesh's packing)
+void launch_begin(lulesh_set *s, cudaStream_t st);
 // the FP64 force phase of every domain of the set
 void launch_force_fp64(lulesh_set *s, cudaStream_t st);
 // staged comm path of one cycle (comm.cu)
