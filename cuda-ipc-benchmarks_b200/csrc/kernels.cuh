@@ -220,10 +220,15 @@ __device__ __forceinline__ int chk_index(long long i, long long n, TimeCtl *T, i
 // writes are visible, before touching any memory, then lets its own
 // dependents be scheduled.  Without the attribute both pass at once.
 
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger()
+{
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
 __device__ __forceinline__ void pdl_enter()
 {
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    pdl_wait();
+    pdl_trigger();
 }
 
 template <typename... KArgs, typename... Args>

@@ -12,7 +12,10 @@
 // long as the library is loaded.
 //
 // The corner forces of up to kNoAllocMaxElems elements live in that array;
-// its last 256 bytes hold the volume-error flag.  Host code never uses the
+// its last 256 bytes hold the volume-error flag, which is 0 between calls (and
+// in a newly loaded module): the gather kernel, which reports it, puts it
+// back.  So a call is two launches, the second scheduled while the first
+// drains.  Host code never uses the
 // array's name as an address: the device address comes from
 // cudaGetSymbolAddress, looked up with the device current on every call made
 // outside stream capture (a device reset or a caller-created context moves
@@ -32,13 +35,12 @@ constexpr int kCornerDoubles = 3 * 8 * kNoAllocMaxElems;
 constexpr int kBlock = 128;
 
 // corner forces [component][corner][element] followed by a 256-byte tail
-// whose first int is the smallest element with a negative volume
+// whose first int is INT_MAX - (the smallest element with a negative volume),
+// 0 for none
 static __device__ __align__(256) double g_noalloc_scratch[kCornerDoubles + 32];
 
 std::mutex g_mu;
 void *g_addr[64];  // last looked-up address of g_noalloc_scratch, per device ordinal
-
-__global__ void k_flag_reset(int *flag) { *flag = INT_MAX; }
 
 template <bool HG>
 __global__ void __launch_bounds__(kBlock)
@@ -50,6 +52,7 @@ __global__ void __launch_bounds__(kBlock)
                     const double *__restrict__ ss, const double *__restrict__ elemMass,
                     double hourg, double *__restrict__ corners, int *flag)
 {
+    lulesh::pdl_trigger();  // the gather may be scheduled; it waits for this grid
     const int numElem = nx * nx * nx;
     const int elem = blockIdx.x * blockDim.x + threadIdx.x;
     if (elem >= numElem) return;
@@ -78,20 +81,25 @@ __global__ void __launch_bounds__(kBlock)
 #pragma unroll
             for (int k = 0; k < 8; ++k) corners[(c * 8 + k) * Ep + elem] = f[k];
         },
-        [&] { atomicMin(flag, elem); });
+        [&] { atomicMax(flag, INT_MAX - elem); });
 }
 
 // per-node sum of the surrounding corners in corner order 0..7 (the
 // nodeElemCornerList order of a structured mesh)
 __global__ void __launch_bounds__(kBlock)
-    k_gather_noalloc(int nx, const double *__restrict__ corners, const int *flag,
+    k_gather_noalloc(int nx, const double *corners, int *flag,
                      double *__restrict__ fx, double *__restrict__ fy, double *__restrict__ fz,
                      int *bad_elem)
 {
     const int en = nx + 1, numNode = en * en * en;
     const int numElem = nx * nx * nx, Ep = ((numElem + 31) / 32) * 32;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i == 0 && bad_elem) *bad_elem = (*flag == INT_MAX) ? -1 : *flag;
+    lulesh::pdl_wait();  // the force kernel's corners and flag
+    if (i == 0) {
+        const int bad = *flag;
+        if (bad_elem) *bad_elem = bad == 0 ? -1 : INT_MAX - bad;
+        *flag = 0;
+    }
     if (i >= numNode) return;
     const int px = i % en, t = i / en, py = t % en, pz = t / en;
     const int cx[8] = {0, 1, 1, 0, 0, 1, 1, 0}, cy[8] = {0, 0, 1, 1, 0, 0, 1, 1},
@@ -173,14 +181,13 @@ extern "C" int lulesh_volume_force_noalloc(int nx, const double *x, const double
     double *corners = static_cast<double *>(base);
     int *flag = reinterpret_cast<int *>(corners + kCornerDoubles);
     const int numElem = nx * nx * nx, numNode = (nx + 1) * (nx + 1) * (nx + 1);
-    k_flag_reset<<<1, 1, 0, s>>>(flag);
     if (hgcoef > 0.0)
         k_force_noalloc<true><<<(numElem + kBlock - 1) / kBlock, kBlock, 0, s>>>(
             nx, x, y, z, xd, yd, zd, volo, v, p, q, ss, elemMass, hgcoef, corners, flag);
     else
         k_force_noalloc<false><<<(numElem + kBlock - 1) / kBlock, kBlock, 0, s>>>(
             nx, x, y, z, xd, yd, zd, volo, v, p, q, ss, elemMass, hgcoef, corners, flag);
-    k_gather_noalloc<<<(numNode + kBlock - 1) / kBlock, kBlock, 0, s>>>(nx, corners, flag, fx,
-                                                                        fy, fz, bad_elem);
+    lulesh::launch_k(k_gather_noalloc, (numNode + kBlock - 1) / kBlock, kBlock, s, /*pdl=*/true, nx,
+                     corners, flag, fx, fy, fz, bad_elem);
     return (cudaGetLastError() == cudaSuccess) ? LULESH_OK : LULESH_CUDA_ERROR;
 }
