@@ -116,7 +116,7 @@ struct CornerStore {
 // gives the corner values.  The monotonic-Q gradients are those of the
 // coordinates themselves (the reference shifts them by half a step and back).
 template <class Vel>
-__device__ __forceinline__ void kin_modal(const DomDev &D, TimeCtl &T, int k,
+__device__ __forceinline__ void kin_modal(const DomDev &D, TimeCtl &T, double dt, int k,
                                           const double (&xn)[8], const double (&yn)[8],
                                           const double (&zn)[8], const Vel &vel)
 {
@@ -138,7 +138,7 @@ __device__ __forceinline__ void kin_modal(const DomDev &D, TimeCtl &T, int k,
         vel(i, v);
         odd_modes(v, va[i], vb[i], vc[i], vg);
     }
-    D.vdov[k] = modal_divergence(m, va, vb, vc, 0.5 * T.deltatime);
+    D.vdov[k] = modal_divergence(m, va, vb, vc, 0.5 * dt);
 
     const double norm = 1.0 / (volume + 1.e-36);
     double delx, delv;

@@ -107,6 +107,63 @@ __device__ __forceinline__ void time_increment(TimeCtl &T, const Params &P)
     T.active = 1;
 }
 
+// The time increment inside the cycle's own kernels (SetArgs::next), for sets
+// small enough that a launch more is felt.  T, the job's time state, stands
+// still while force and nodal run; N is scratch between cycles.
+//   force       runs where the increment will find the job due; its errors go
+//               to N, so that no block sees another's and stops
+//   nodal       one extra warp a block makes the increment from T, for the
+//               block's own use; the job's first block leaves it in N
+//   kinematics  works from N; the job's first block copies N to T and adds
+//               force's errors
+//   EOS         as after a k_time_increment launch
+// Measured on B200 in graphs of 4 cycles, us per cycle with a launch -> inside:
+// -s 10 17.5 -> 16.7, -s 30 20.1 -> 18.6, -s 45 28.5 -> 26.7, -s 64 55.3 -> 54.7,
+// 2x2x2 of -s 12 23.1 -> 21.6; past one wave of the node update it costs more
+// than the launch (-s 100 188.8 -> 192.6, a 24-job batch 187 -> 196).
+__device__ __forceinline__ bool increment_due(const TimeCtl &T, const Params &P)
+{
+#if LULESH_CHECKED
+    if (T.chk != 0) return false;
+#endif
+    return !T.done && T.bad_vol == INT_MAX && T.bad_q == INT_MAX && T.time < P.stoptime &&
+           !(T.its_cap > 0 && T.cycle >= T.its_cap);
+}
+
+// what time_increment sets, from one record to the other
+__device__ __forceinline__ void copy_increment(TimeCtl &to, const TimeCtl &from)
+{
+    to.time = from.time;
+    to.deltatime = from.deltatime;
+    to.dtcourant = from.dtcourant;
+    to.dthydro = from.dthydro;
+    to.min_courant = from.min_courant;
+    to.min_hydro = from.min_hydro;
+    to.cycle = from.cycle;
+    to.active = from.active;
+    to.done = from.done;
+    to.status = from.status;
+}
+
+__device__ __forceinline__ void commit_increment(TimeCtl &T, TimeCtl &N)
+{
+    copy_increment(T, N);
+    if (N.bad_vol != INT_MAX) {
+        atomicMin(&T.bad_vol, N.bad_vol);
+        N.bad_vol = INT_MAX;
+    }
+    if (N.chk != 0) {
+        atomicCAS(&T.chk, 0, N.chk);
+        N.chk = 0;
+    }
+}
+
+// the block that speaks for its job: the first items of its first domain
+__device__ __forceinline__ bool first_of_job(const DomDev &D, int first)
+{
+    return first == 0 && (D.col | D.row | D.plane) == 0;
+}
+
 __global__ void k_time_increment(TimeCtl *tcs, int ntc, Params P)
 {
     pdl_enter();
@@ -199,12 +256,13 @@ void launch_begin_packed(const SetArgs &a, int nblocks, Params P, cudaStream_t s
 // them, the kernel fits 128 registers (16 warps) but took 73 against 70 us,
 // and 312 against 272 us at -s 160.
 template <bool HG, Mesh M, bool TABLE>
-__device__ __forceinline__ void force_one(const DomDev &D, TimeCtl &T, const Params &P, int elem)
+__device__ __forceinline__ void force_one(const DomDev &D, bool active, TimeCtl &E, const Params &P,
+                                          int elem)
 {
     int n[8];
     elem_nodes<M != Mesh::kBox>(D, elem, n);
 #pragma unroll
-    for (int i = 0; i < 8; ++i) n[i] = chk_index(n[i], D.numNode, &T, kChkNode);
+    for (int i = 0; i < 8; ++i) n[i] = chk_index(n[i], D.numNode, &E, kChkNode);
     double vn[3][8], xn[8], yn[8], zn[8];
     if constexpr (M == Mesh::kPacked) {
 #pragma unroll
@@ -228,7 +286,7 @@ __device__ __forceinline__ void force_one(const DomDev &D, TimeCtl &T, const Par
 #pragma unroll
         for (int i = 0; i < 8; ++i) zn[i] = D.z[n[i]];
     }
-    if (!TABLE && !T.active) return;
+    if (!TABLE && !active) return;
     double fx[8], fy[8];  // held for cornerPack, whose corners take all three
     force_modal<HG>(
         xn, yn, zn, D.volo[elem], D.v[elem], D.p[elem], D.q[elem], D.ss[elem], D.elemMass[elem],
@@ -250,7 +308,7 @@ __device__ __forceinline__ void force_one(const DomDev &D, TimeCtl &T, const Par
                 CornerStore{D.fx_elem, D.fy_elem, D.fz_elem, elem, D.Ep}(c, f);
             }
         },
-        [&] { atomicMin(&T.bad_vol, elem); });
+        [&] { atomicMin(&E.bad_vol, elem); });
 }
 
 template <bool HG, int BS, Mesh M, class W>
@@ -260,11 +318,12 @@ __global__ void __launch_bounds__(BS, min_blocks(kForceMinBlocks, BS))
     pdl_enter();
     const int2 blk = w.template block<BS, LULESH_FORCE_REVERSE>();
     const DomDev &D = w.domain(blk.x);
-    TimeCtl &T = w.time(D);
-    if (W::kTable && !T.active) return;
+    const TimeCtl &T = w.time(D);
+    const bool active = w.increments() ? increment_due(T, P) : T.active != 0;
+    if (W::kTable && !active) return;
     const int elem = blk.y + threadIdx.x;
     if (elem >= D.numElem) return;
-    force_one<HG, M, W::kTable>(D, T, P, elem);
+    force_one<HG, M, W::kTable>(D, active, w.next(D), P, elem);
 }
 
 template <int BS, Mesh M, class W>
@@ -365,8 +424,8 @@ __device__ __forceinline__ void gather_corners(const DomDev *doms, const DomDev 
 // of ApplyAccelerationBoundaryConditionsForNodes (bc bits 0/1/2 zero the
 // x/y/z acceleration) and CalcPositionAndVelocityForNodes (lulesh.cu:
 // 2999-3028) for node i with the summed force (fx, fy, fz)
-__device__ __forceinline__ void advance_node(const DomDev &D, const TimeCtl &T, const Params &P,
-                                             int i, int bc, double fx, double fy, double fz,
+__device__ __forceinline__ void advance_node(const DomDev &D, double dt, const Params &P, int i,
+                                             int bc, double fx, double fy, double fz,
                                              int materialize, bool write_f, bool pack = false)
 {
     const double one_over_nMass = 1. / D.nodalMass[i];
@@ -377,7 +436,6 @@ __device__ __forceinline__ void advance_node(const DomDev &D, const TimeCtl &T, 
     if (bc & 2) ydd = 0.0;
     if (bc & 4) zdd = 0.0;
 
-    const double dt = T.deltatime;
     const double u_cut = P.u_cut;
     double xdtmp = D.xd[i] + xdd * dt;
     double ydtmp = D.yd[i] + ydd * dt;
@@ -412,16 +470,46 @@ __device__ __forceinline__ void advance_node(const DomDev &D, const TimeCtl &T, 
 // MODE 1: AddNodeForcesFromElems over this domain's own corners only,
 //         writing fx/fy/fz (the partial sums the reference exchanges).
 // MODE 2: the node update from fx/fy/fz (after CommSBN added neighbours).
-template <int MODE, int BS, class W>
-__global__ void __launch_bounds__(BS, min_blocks(kNodalMinBlocks, BS))
+// INCR (MODE 0): a warp more than BS threads makes the time increment while
+// the others gather.
+template <int MODE, int BS, class W, bool INCR = false>
+__global__ void __launch_bounds__(INCR ? BS + 32 : BS,
+                                  min_blocks(INCR ? kNodalIncrMinBlocks : kNodalMinBlocks, BS))
     k_nodal(const __grid_constant__ W w, Params P)
 {
     pdl_enter();
     const int2 blk = w.template block<BS, LULESH_NODAL_REVERSE && !W::kTable>();
     const DomDev &D = w.domain(blk.x);
     TimeCtl &T = w.time(D);
-    if (W::kTable && !T.active) return;
     const int i = blk.y + threadIdx.x;
+    if constexpr (INCR) {
+        __shared__ double s_dt;
+        __shared__ int s_active;
+        const bool speaks = first_of_job(D, blk.y);
+        if (W::kTable && !speaks && !increment_due(T, P)) return;
+        const bool mine = threadIdx.x < BS && i < D.numNode;
+        const int en = D.en, px = i % en, t = i / en, py = t % en, pz = t / en;
+        double fx, fy, fz;
+        if (threadIdx.x >= BS) {
+            TimeCtl n = T;
+            time_increment(n, P);
+            if (threadIdx.x == BS) {
+                s_dt = n.deltatime;
+                s_active = n.active;
+                if (speaks) copy_increment(w.next(D), n);
+            }
+        } else if (mine) {
+            gather_corners<!std::is_same_v<W, OneDomain>>(w.doms(), D, px, py, pz, fx, fy, fz,
+                                                          &w.next(D));
+        }
+        __syncthreads();
+        if (!mine || !s_active) return;
+        const int bc = (D.col == 0 && px == 0 ? 1 : 0) | (D.row == 0 && py == 0 ? 2 : 0) |
+                       (D.plane == 0 && pz == 0 ? 4 : 0);
+        advance_node(D, s_dt, P, i, bc, fx, fy, fz, w.materialize(), true);
+        return;
+    }
+    if (W::kTable && !T.active) return;
     if (i >= D.numNode) return;
     const int en = D.en;
     const int px = i % en;
@@ -449,7 +537,7 @@ __global__ void __launch_bounds__(BS, min_blocks(kNodalMinBlocks, BS))
     const int bc = (D.col == 0 && px == 0 ? 1 : 0) | (D.row == 0 && py == 0 ? 2 : 0) |
                    (D.plane == 0 && pz == 0 ? 4 : 0);
     if (!W::kTable && !T.active) return;
-    advance_node(D, T, P, i, bc, fx, fy, fz, w.materialize(), MODE == 0);
+    advance_node(D, T.deltatime, P, i, bc, fx, fy, fz, w.materialize(), MODE == 0);
 }
 
 // Scattered meshes: the corner forces of a node, one sector each, summed in
@@ -483,7 +571,7 @@ __global__ void __launch_bounds__(kNodeBlock)
             fz += vz[j];
         }
     }
-    advance_node(D, T, P, i, D.nodeBC[i], fx, fy, fz, w.mat, true, /*pack=*/true);
+    advance_node(D, T.deltatime, P, i, D.nodeBC[i], fx, fy, fz, w.mat, true, /*pack=*/true);
 }
 
 // Unstructured meshes: AddNodeForcesFromElems (lulesh.cu:1715-1751) over
@@ -537,7 +625,7 @@ __global__ void __launch_bounds__(BS, min_blocks(kNodalUMinBlocks, BS))
                     fz += vz[q];
                 }
         }
-        advance_node(D, T, P, i, D.nodeBC[i], fx, fy, fz, w.mat, true);
+        advance_node(D, T.deltatime, P, i, D.nodeBC[i], fx, fy, fz, w.mat, true);
         return;
     }
     const long long list_len = 8LL * D.numElem;  // corner-list entries
@@ -589,14 +677,18 @@ __global__ void __launch_bounds__(BS, min_blocks(kNodalUMinBlocks, BS))
         fz += ld_corner(D.fz_elem + k);
     }
     // symmetry nodes of the mesh's X/Y/Z sets: nodeBC bits 0/1/2
-    advance_node(D, T, P, i, D.nodeBC[i], fx, fy, fz, w.mat, true);
+    advance_node(D, T.deltatime, P, i, D.nodeBC[i], fx, fy, fz, w.mat, true);
 }
 
 template <int BS>
 static void launch_nodal_bs(const SetArgs &a, int nblocks, Params P, cudaStream_t s)
 {
     launch_where<true, BS == kNodeBlock>(a, nblocks, [&](const auto &w) {
-        launch_k(k_nodal<0, BS, std::decay_t<decltype(w)>>, nblocks, BS, s, a.pdl != 0, w, P);
+        using W = std::decay_t<decltype(w)>;
+        if (a.next)
+            launch_k(k_nodal<0, BS, W, true>, nblocks, BS + 32, s, a.pdl != 0, w, P);
+        else
+            launch_k(k_nodal<0, BS, W>, nblocks, BS, s, a.pdl != 0, w, P);
     });
 }
 
@@ -644,8 +736,9 @@ __global__ void __launch_bounds__(BS, min_blocks(M == Mesh::kPacked ? kKinPacked
     pdl_enter();
     const int2 blk = w.template block<BS, LULESH_KIN_REVERSE>();
     const DomDev &D = w.domain(blk.x);
-    TimeCtl &T = w.time(D);
-    if (W::kTable && !T.active) return;
+    TimeCtl &T = w.time(D), &N = w.next(D);
+    if (w.increments() && threadIdx.x == 0 && first_of_job(D, blk.y)) commit_increment(T, N);
+    if (W::kTable && !N.active) return;
     const int k = blk.y + threadIdx.x;
     if (k >= D.numElem) return;
 
@@ -659,8 +752,8 @@ __global__ void __launch_bounds__(BS, min_blocks(M == Mesh::kPacked ? kKinPacked
 #pragma unroll
         for (int l = 0; l < 8; ++l)
             load_node(D, n[l], xn[l], yn[l], zn[l], vn[0][l], vn[1][l], vn[2][l]);
-        if (!W::kTable && !T.active) return;
-        kin_modal(D, T, k, xn, yn, zn, [&](int c, double (&v)[8]) {
+        if (!W::kTable && !N.active) return;
+        kin_modal(D, T, N.deltatime, k, xn, yn, zn, [&](int c, double (&v)[8]) {
 #pragma unroll
             for (int l = 0; l < 8; ++l) v[l] = vn[c][l];
         });
@@ -672,8 +765,8 @@ __global__ void __launch_bounds__(BS, min_blocks(M == Mesh::kPacked ? kKinPacked
         for (int l = 0; l < 8; ++l) yn[l] = D.y[n[l]];
 #pragma unroll
         for (int l = 0; l < 8; ++l) zn[l] = D.z[n[l]];
-        if (!W::kTable && !T.active) return;
-        kin_modal(D, T, k, xn, yn, zn, [&](int c, double (&v)[8]) {
+        if (!W::kTable && !N.active) return;
+        kin_modal(D, T, N.deltatime, k, xn, yn, zn, [&](int c, double (&v)[8]) {
             const double *a = c == 0 ? D.xd : c == 1 ? D.yd : D.zd;
 #pragma unroll
             for (int l = 0; l < 8; ++l) v[l] = a[n[l]];

@@ -52,6 +52,12 @@ constexpr int kNodeBlock = 128;  // threads per block, node kernels
 #define LULESH_NODAL_MINB 16
 #endif
 constexpr int kNodalMinBlocks = LULESH_NODAL_MINB;
+// with the time increment's warp (small sets, one wave): registers for all
+// corner loads of a node at once
+#ifndef LULESH_NODAL_INCR_MINB
+#define LULESH_NODAL_INCR_MINB 8
+#endif
+constexpr int kNodalIncrMinBlocks = LULESH_NODAL_INCR_MINB;
 // unstructured nodal kernel: four corners x 3 components in flight
 #ifndef LULESH_NODAL_U_MINB
 #define LULESH_NODAL_U_MINB 12
@@ -72,6 +78,14 @@ constexpr int min_blocks(int minb, int bs)
 {
     return (minb * 128 / bs) > 0 ? (minb * 128 / bs) : 1;
 }
+
+// Largest set (nodes) whose cycle kernels make the time increment: one wave of
+// the node update, 16 blocks of 128 on each of 148 SMs.  Beyond it every later
+// wave would make it again, to save a launch of 1% of the cycle.
+#ifndef LULESH_INLINE_NODES
+#define LULESH_INLINE_NODES (148 * 16 * 128)
+#endif
+constexpr long long kInlineIncrementNodes = LULESH_INLINE_NODES;
 
 // Block shapes the FP64 element kernels (force, kinematics, EOS) and the
 // nodal kernel are compiled for; a set's block tables use one of each.
@@ -97,11 +111,16 @@ struct SetArgs {
     // which the kernels then take by value (OneDomain, FewDomains)
     const DomDev *records = nullptr;
     int ndom = 0;
+    // one record per job beside tcs: the cycle's kernels make the time
+    // increment themselves (inline_increment, set.hpp); null after a
+    // k_time_increment launch
+    TimeCtl *next = nullptr;
     const CornerF32 *corner32 = nullptr;  // a mixed set's first domain (host side only)
 };
 
 // Where a block of a cycle kernel works: its domain's record, the time state
-// and the first item.
+// (time) and the first item.  next is where the cycle's own time state is
+// formed when its kernels increment the time themselves, else time again.
 //
 // ManyDomains reads them from memory: block table -> domain record -> array
 // pointers, three dependent loads before the first gather, and the pointers
@@ -123,6 +142,11 @@ struct ManyDomains {
     }
     __device__ __forceinline__ const DomDev &domain(int d) const { return a.doms[d]; }
     __device__ __forceinline__ TimeCtl &time(const DomDev &D) const { return a.tcs[D.tc]; }
+    __device__ __forceinline__ TimeCtl &next(const DomDev &D) const
+    {
+        return a.next ? a.next[D.tc] : a.tcs[D.tc];
+    }
+    __device__ __forceinline__ bool increments() const { return a.next != nullptr; }
     __device__ __forceinline__ const DomDev *doms() const { return a.doms; }
     __device__ __forceinline__ int materialize() const { return a.materialize; }
     // The node block table is already laid out last to first.  A job that is
@@ -134,7 +158,7 @@ struct ManyDomains {
 template <int N>
 struct ByValue {
     DomDev D[N];
-    TimeCtl *tc;
+    TimeCtl *tc, *tn;
     int mat;
     int per;  // blocks per domain of this launch
     template <int BS, bool REVERSE>
@@ -146,6 +170,8 @@ struct ByValue {
     }
     __device__ __forceinline__ const DomDev &domain(int d) const { return D[N == 1 ? 0 : d]; }
     __device__ __forceinline__ TimeCtl &time(const DomDev &) const { return *tc; }
+    __device__ __forceinline__ TimeCtl &next(const DomDev &) const { return *tn; }
+    __device__ __forceinline__ bool increments() const { return tn != tc; }
     __device__ __forceinline__ const DomDev *doms() const { return D; }
     __device__ __forceinline__ int materialize() const { return mat; }
     // the time state is read beside the gathers, and checked before any store
@@ -161,6 +187,7 @@ inline ByValue<N> by_value(const SetArgs &a, int nblocks)
     ByValue<N> w;
     for (int d = 0; d < N; ++d) w.D[d] = a.records[d];
     w.tc = a.tcs;
+    w.tn = a.next ? a.next : a.tcs;
     w.mat = a.materialize;
     w.per = nblocks / N;
     return w;

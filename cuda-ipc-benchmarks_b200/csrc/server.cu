@@ -101,6 +101,7 @@ struct lulesh_server {
     int2 *node_b = nullptr, *elem_b = nullptr;
     int n_node = 0, n_elem = 0;
     int n_table = 0;  // domains in the launched tables
+    bool inline_increment = false;  // as lulesh_set::inline_increment
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     bool dirty = true;
@@ -115,6 +116,7 @@ struct lulesh_server {
         a.blocks = b;
         a.materialize = 0;
         a.pdl = LULESH_PDL;  // the cycle kernels overlap each other's tails
+        a.next = inline_increment ? dtc + cfg.max_jobs : nullptr;
         return a;
     }
 };
@@ -199,8 +201,17 @@ static int rebuild(lulesh_server *s)
         s->exec = nullptr;
         s->graph = nullptr;
     } else {
+        long long nodes = 0;
+        for (const DomDev &D : hd) nodes += D.numNode;
+        const bool was_inline = s->inline_increment;
+        s->inline_increment = nodes <= kInlineIncrementNodes;
+        if (s->exec && was_inline != s->inline_increment) {  // another kernel sequence
+            cudaGraphExecDestroy(s->exec);
+            s->exec = nullptr;
+        }
         SCHECK(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
-        launch_time_increment(s->dtc, s->cfg.max_jobs, s->P, s->stream, LULESH_PDL != 0);
+        if (!s->inline_increment)
+            launch_time_increment(s->dtc, s->cfg.max_jobs, s->P, s->stream, LULESH_PDL != 0);
         launch_force(s->args(s->elem_b), s->n_elem, s->P, s->stream, kServerElemBlock);
         launch_nodal(s->args(s->node_b), s->n_node, s->P, s->stream);
         launch_kinematics(s->args(s->elem_b), s->n_elem, s->P, s->stream, kServerElemBlock);
@@ -257,7 +268,7 @@ int lulesh_server_create(const lulesh_server_config *cfg, lulesh_server **out)
     unsigned long long keep = ~0ull;  // keep freed job memory cached in the pool
     cudaMemPoolSetAttribute(s->pool, cudaMemPoolAttrReleaseThreshold, &keep);
     const int M = cfg->max_jobs;
-    if ((st = cuda_status(cudaMalloc(&s->dtc, sizeof(TimeCtl) * M), "slots"))) return fail(st);
+    if ((st = cuda_status(cudaMalloc(&s->dtc, sizeof(TimeCtl) * 2 * M), "slots"))) return fail(st);
     if ((st = cuda_status(cudaMallocHost(&s->htc, sizeof(TimeCtl) * M), "slots"))) return fail(st);
     if ((st = cuda_status(cudaMalloc(&s->denergy, sizeof(double) * M), "slots"))) return fail(st);
     if ((st = cuda_status(cudaMallocHost(&s->henergy, sizeof(double) * M), "slots")))
@@ -266,14 +277,14 @@ int lulesh_server_create(const lulesh_server_config *cfg, lulesh_server **out)
     if ((st = cuda_status(cudaEventCreateWithFlags(&s->step_done, cudaEventDisableTiming), "event")))
         return fail(st);
     // every slot starts empty: done, so the time-increment kernel skips it
-    std::vector<TimeCtl> empty(M);
+    // (and a record more each for the cycle's own time state)
+    std::vector<TimeCtl> empty(2 * M, initial_timectl(0.0, 0));
     for (int i = 0; i < M; ++i) {
-        empty[i] = initial_timectl(0.0, 0);
         empty[i].done = 1;
         s->htc[i] = empty[i];
         s->free_slots.push_back(M - 1 - i);
     }
-    if ((st = cuda_status(cudaMemcpy(s->dtc, empty.data(), sizeof(TimeCtl) * M,
+    if ((st = cuda_status(cudaMemcpy(s->dtc, empty.data(), sizeof(TimeCtl) * 2 * M,
                                      cudaMemcpyHostToDevice),
                           "slots")))
         return fail(st);

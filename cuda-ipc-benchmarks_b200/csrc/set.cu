@@ -330,9 +330,10 @@ static int create_common(lulesh_set *s, const std::vector<DomPlace> &place, int 
     // time control blocks
     std::vector<TimeCtl> tc(s->njobs);
     for (int j = 0; j < s->njobs; ++j) tc[j] = initial_timectl(job_dt[j], s->jobs[j].its);
-    LCHECK(cudaMalloc(&s->dtc, sizeof(TimeCtl) * s->njobs));
+    LCHECK(cudaMalloc(&s->dtc, sizeof(TimeCtl) * 2 * s->njobs));
     LCHECK(cudaMallocHost(&s->htc_pinned, sizeof(TimeCtl) * s->njobs));
-    LCHECK(cudaMemcpyAsync(s->dtc, tc.data(), sizeof(TimeCtl) * s->njobs,
+    tc.insert(tc.end(), s->njobs, initial_timectl(0.0, 0));  // SetArgs::next
+    LCHECK(cudaMemcpyAsync(s->dtc, tc.data(), sizeof(TimeCtl) * tc.size(),
                            cudaMemcpyHostToDevice, s->stream));
     int st = build_tables(s);
     if (st != LULESH_OK) return st;
@@ -354,7 +355,7 @@ void launch_begin(lulesh_set *s, cudaStream_t st)
 {
     if (s->pack)
         launch_begin_packed(s->args(s->node_blocks), s->n_node_blocks, s->P, st);
-    else
+    else if (!s->inline_increment())
         launch_time_increment(s->dtc, s->njobs, s->P, st, s->pdl);
 }
 

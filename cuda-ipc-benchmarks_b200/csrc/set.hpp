@@ -55,7 +55,7 @@ struct lulesh_set {
 
     // device tables (elem_blocks is the base of one allocation holding all)
     lulesh::DomDev *ddoms = nullptr;
-    lulesh::TimeCtl *dtc = nullptr;
+    lulesh::TimeCtl *dtc = nullptr;   // njobs records, then njobs more (args().next)
     lulesh::TimeCtl *htc_pinned = nullptr;  // pinned mirror for readback
     int2 *elem_blocks = nullptr, *node_blocks = nullptr, *ghost_blocks = nullptr;
     int n_elem_blocks = 0, n_node_blocks = 0, n_ghost_blocks = 0;
@@ -124,6 +124,17 @@ struct lulesh_set {
     int max_plane = 0, max_edge = 0;
     int posted_msg = 0, posted_fields = 0, posted_do_recv = 1, posted_plane_only = 0;
 
+    // The cycle's kernels make the time increment (kernels.cu) in place of a
+    // launch of its own.
+    bool inline_increment() const
+    {
+        if (nparts > 1 || unstructured || (flags & (LULESH_FLAG_COMM_STAGED | LULESH_FLAG_MIXED)))
+            return false;
+        long long nodes = 0;
+        for (const lulesh::DomDev &D : hdoms) nodes += D.numNode;
+        return nodes <= lulesh::kInlineIncrementNodes;
+    }
+
     lulesh::SetArgs args(const int2 *blocks) const
     {
         lulesh::SetArgs a;
@@ -137,6 +148,7 @@ struct lulesh_set {
         a.records = nparts == 1 && njobs == 1 && (ndom == 1 || ndom == lulesh::kFewDomains)
                         ? hdoms.data()
                         : nullptr;
+        if (inline_increment()) a.next = dtc + njobs;
         a.corner32 = hcorner32.empty() ? nullptr : hcorner32.data();
         return a;
     }
