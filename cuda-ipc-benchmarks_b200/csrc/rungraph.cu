@@ -2,12 +2,12 @@
 //
 // The reference drives its main loop from the host (lulesh.cu:4858-4873):
 // TimeIncrement, LagrangeLeapFrog, and a check of the stop condition every
-// cycle.  Here the loop is a WHILE conditional node: its body is one cycle
+// cycle.  Here the loop is a WHILE conditional node: its body is a few cycles
 // (the same launches lulesh_step captures) followed by k_run_continue,
 // which keeps the loop going while any job of the set is not done.  A batch
 // of jobs, or a single job, then runs to completion in a single launch with
-// no host involvement.  Every iteration is counted and the loop stops at a
-// cap, so it ends even if a job could never reach its stop condition.
+// no host involvement.  Every turn is counted and the loop stops at a cap, so
+// it ends even if a job could never reach its stop condition.
 #include "set.hpp"
 
 namespace lulesh {
@@ -16,7 +16,14 @@ namespace {
 
 constexpr unsigned long long kDefaultRunCap = 1000000ull;
 
-// ctl[0]: cycles run so far, ctl[1]: cap
+// Cycles per turn of the loop.  A turn's end (k_run_continue, then the
+// conditional node's own decision) costs about as much as two kernels of a
+// small mesh; cycles after the last job is done skip their work.  Measured on
+// B200, us per cycle, 1 -> 4 per turn: -s 10 23.6 -> 19.0, -s 30 26.8 -> 21.7, a
+// batch of 24 jobs 194 -> 185.
+constexpr int kCyclesPerTurn = 4;
+
+// ctl[0]: turns so far, ctl[1]: cap
 __global__ void k_run_continue(cudaGraphConditionalHandle h, const TimeCtl *tcs, int ntc,
                                unsigned long long *ctl)
 {
@@ -63,11 +70,8 @@ int ensure_run_graph(lulesh_set *s)
                                                        cudaStreamCaptureModeThreadLocal),
                          "capture loop body");
         if (st == LULESH_OK) {
-            // the loop body keeps plain stream order between its kernels
-            const bool pdl = s->pdl;
-            s->pdl = false;
-            int est = enqueue_cycle(s);
-            s->pdl = pdl;
+            int est = LULESH_OK;
+            for (int c = 0; c < kCyclesPerTurn && est == LULESH_OK; ++c) est = enqueue_cycle(s);
             k_run_continue<<<1, 128, 0, s->stream>>>(h, s->dtc, s->njobs, s->run_ctl);
             cudaGraph_t captured = nullptr;
             const int cst = cuda_status(cudaStreamEndCapture(s->stream, &captured), "end capture");
@@ -93,9 +97,14 @@ extern "C" int lulesh_run_graph(lulesh_set *s, long long max_cycles)
     if (!s) return LULESH_INVALID_ARG;
     int st = ensure_run_graph(s);
     if (st != LULESH_OK) return st;
-    const unsigned long long ctl[2] = {
-        0ull, max_cycles > 0 ? (unsigned long long)max_cycles : kDefaultRunCap};
-    RCHECK(cudaMemcpyAsync(s->run_ctl, ctl, sizeof ctl, cudaMemcpyHostToDevice, s->stream));
-    RCHECK(cudaGraphLaunch(s->exec_run, s->stream));
+    const unsigned long long cap = max_cycles > 0 ? (unsigned long long)max_cycles : kDefaultRunCap;
+    const unsigned long long ctl[2] = {0ull, cap / kCyclesPerTurn};
+    if (ctl[1] > 0) {
+        RCHECK(cudaMemcpyAsync(s->run_ctl, ctl, sizeof ctl, cudaMemcpyHostToDevice, s->stream));
+        RCHECK(cudaGraphLaunch(s->exec_run, s->stream));
+    }
+    // the cap's last cycles, fewer than a turn (no work where all jobs are done)
+    for (unsigned long long c = 0; c < cap % kCyclesPerTurn; ++c)
+        if ((st = enqueue_cycle(s)) != LULESH_OK) return st;
     return run_status(s);  // synchronises the stream
 }

@@ -531,14 +531,31 @@ static int ensure_graph(lulesh_set *s)
     return LULESH_OK;
 }
 
-// graph of graph_cycles consecutive cycles (one launch for many cycles)
-static int ensure_graph_k(lulesh_set *s)
+// Cycles per graph launch of a step of n.  A set that leaves graph_cycles at 1
+// gets graphs of kStepCycles once it has run kStepAfter cycles one by one:
+// launches of one-cycle graphs leave gaps (on B200 a cycle ends on a grid of
+// 2 us: -s 30 22.6 -> 20.1 us per cycle in fours, -s 45 30.0 -> 28.5, -s 100
+// 188.8 -> 184.6; eights gain no more), but the longer graph takes about as
+// long to capture and instantiate as it saves in 100 cycles, which a short run
+// does not get back.
+constexpr int kStepCycles = 4;
+constexpr long long kStepAfter = 256;
+static int cycles_per_launch(lulesh_set *s, int n)
 {
-    if (s->graph_k_ready || s->graph_cycles <= 1) return LULESH_OK;
+    if (s->graph_cycles > 1) return s->graph_cycles;
+    const bool lived = s->cycles_run >= kStepAfter;
+    if (!lived) s->cycles_run += n;
+    return lived ? kStepCycles : 1;
+}
+
+// graph of k consecutive cycles (one launch for many cycles)
+static int ensure_graph_k(lulesh_set *s, int k)
+{
+    if (s->graph_k_ready) return LULESH_OK;
     int st = ensure_graph(s);  // prepares comm tables when staged
     if (st != LULESH_OK) return st;
     LCHECK(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
-    for (int c = 0; c < s->graph_cycles && st == LULESH_OK; ++c) st = enqueue_cycle(s);
+    for (int c = 0; c < k && st == LULESH_OK; ++c) st = enqueue_cycle(s);
     cudaGraph_t g = nullptr;
     cudaError_t e = cudaStreamEndCapture(s->stream, &g);
     if (st != LULESH_OK) {
@@ -918,10 +935,10 @@ int lulesh_step(lulesh_set *s, int ncycles)
     }
     int st = ensure_graph(s);
     if (st != LULESH_OK) return st;
-    if (s->graph_cycles > 1 && ncycles >= s->graph_cycles) {
-        if ((st = ensure_graph_k(s)) != LULESH_OK) return st;
-        for (; ncycles >= s->graph_cycles; ncycles -= s->graph_cycles)
-            LCHECK(cudaGraphLaunch(s->exec_k, s->stream));
+    const int k = cycles_per_launch(s, ncycles);
+    if (k > 1 && ncycles >= k) {
+        if ((st = ensure_graph_k(s, k)) != LULESH_OK) return st;
+        for (; ncycles >= k; ncycles -= k) LCHECK(cudaGraphLaunch(s->exec_k, s->stream));
     }
     for (int i = 0; i < ncycles; ++i) LCHECK(cudaGraphLaunch(s->exec, s->stream));
     return LULESH_OK;

@@ -87,6 +87,7 @@ struct lulesh_set {
     cudaGraph_t graph_k = nullptr;
     cudaGraphExec_t exec_k = nullptr;
     bool graph_k_ready = false;
+    long long cycles_run = 0;  // by one-cycle launches (cycles_per_launch, set.cu)
     // whole-run graph: a WHILE conditional node around one cycle
     // (rungraph.cu); run_ctl[0] counts cycles, run_ctl[1] is the cap
     cudaGraph_t graph_run = nullptr;
