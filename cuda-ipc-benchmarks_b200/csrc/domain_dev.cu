@@ -93,6 +93,8 @@ int upload_domain(const HostDomain &h, int tc, long comm_doubles, bool mixed, Ca
                   cudaStream_t st, DomDev *out, CornerF32 *c32, Carver *node_cv)
 {
     const DomSizes z = sizes_of(h, comm_doubles);
+    char *const lo = cv.base + cv.off;
+    char *const nlo = node_cv ? node_cv->base + node_cv->off : nullptr;
     DomDev D{};
     D.nx = h.nx;
     D.en = h.nx + 1;
@@ -160,22 +162,12 @@ int upload_domain(const HostDomain &h, int tc, long comm_doubles, bool mixed, Ca
         c32->fz = cv.take<float>(8 * z.Ep);
     }
 
-    // InitializeFields (lulesh.cu:432-451): zeros except v = 1
-    const size_t E = z.E, N = z.N;
-    double *edbl[16] = {D.e, D.p, D.q, D.ql, D.qq, D.v, D.volo, D.delv, D.vdov,
-                        D.arealg, D.ss, D.elemMass, D.vnew, D.delx_xi, D.delx_eta,
-                        D.delx_zeta};
-    for (double *p : edbl) DCHECK(cudaMemsetAsync(p, 0, 8 * E, st));
-    double *ndbl[13] = {D.x, D.y, D.z, D.xd, D.yd, D.zd, D.xdd, D.ydd, D.zdd,
-                        D.fx, D.fy, D.fz, D.nodalMass};
-    for (double *p : ndbl) DCHECK(cudaMemsetAsync(p, 0, 8 * N, st));
-    DCHECK(cudaMemsetAsync(D.delv_xi, 0, 8 * z.allElem, st));
-    DCHECK(cudaMemsetAsync(D.delv_eta, 0, 8 * z.allElem, st));
-    DCHECK(cudaMemsetAsync(D.delv_zeta, 0, 8 * z.allElem, st));
-    DCHECK(cudaMemsetAsync(D.fx_elem, 0, 8 * 8 * z.Ep, st));
-    DCHECK(cudaMemsetAsync(D.fy_elem, 0, 8 * 8 * z.Ep, st));
-    DCHECK(cudaMemsetAsync(D.fz_elem, 0, 8 * 8 * z.Ep, st));
-    if (z.comm) DCHECK(cudaMemsetAsync(D.commRecv, 0, 8 * z.comm, st));
+    // InitializeFields (lulesh.cu:432-451): zeros except v = 1; one clear of
+    // everything carved (and of the node region's share)
+    const size_t E = z.E;
+    DCHECK(cudaMemsetAsync(lo, 0, (size_t)(cv.base + cv.off - lo), st));
+    if (node_cv)
+        DCHECK(cudaMemsetAsync(nlo, 0, (size_t)(ncv.base + ncv.off - nlo), st));
     int su;
     if (h.device_geometry) {
         // single domain: geometry and the per-element region arrays on the
@@ -186,7 +178,6 @@ int upload_domain(const HostDomain &h, int tc, long comm_doubles, bool mixed, Ca
         int *rp[] = {D.regCSR, D.regReps, D.regSorted};
         for (size_t k = 0; k < sizeof(rp) / sizeof(rp[0]); ++k)
             if ((su = upload(rp[k], *rv[k], st)) != LULESH_OK) return su;
-        DCHECK(cudaStreamSynchronize(st));
         *out = D;
         return LULESH_OK;
     }

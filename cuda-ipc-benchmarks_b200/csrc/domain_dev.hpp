@@ -41,8 +41,9 @@ struct Carver {
 
 // Carve every array of host domain `h` from `cv`, initialise and upload it
 // on `st`, and fill the device record *D (and *c32 when mixed).  `tc` is
-// the TimeCtl slot of the domain's job.  Synchronises `st` before
-// returning, so `h` may be released afterwards.
+// the TimeCtl slot of the domain's job.  A host-built domain's upload
+// synchronises `st`, so `h` may be released afterwards; one whose geometry is
+// generated on the device (device_geometry) must live until `st` has passed.
 // With node_cv, x, y, z, xd, yd and zd come from node_cv (a set's node
 // region: every domain's six arrays one after the other) and cv carves the
 // rest; cv then advances by node_region_bytes(...) less than domain_bytes.

@@ -50,7 +50,6 @@ int ensure_run_graph(lulesh_set *s)
     if (s->exec_run) return LULESH_OK;
     int st = prepare_capture(s);
     if (st != LULESH_OK) return st;
-    if (!s->run_ctl) RCHECK(cudaMalloc(&s->run_ctl, 2 * sizeof(unsigned long long)));
     cudaGraph_t g = nullptr;
     RCHECK(cudaGraphCreate(&g, 0));
     cudaGraphConditionalHandle h;

@@ -103,11 +103,11 @@ int build_tables(lulesh_set *s)
     size_t bytes = sizeof(int2) * (eb.size() + nb.size() + gb.size() + sb.size() + 1);
     if (s->elem_blocks) {  // rebuilding: the old tables may still be in use
         LCHECK(cudaStreamSynchronize(s->stream));
-        LCHECK(cudaFree(s->elem_blocks));
+        block_put(&s->tables_block);
         s->elem_blocks = nullptr;
     }
-    int2 *t = nullptr;
-    LCHECK(cudaMalloc(&t, bytes));
+    LCHECK(block_get(&s->tables_block, bytes));
+    int2 *t = static_cast<int2 *>(s->tables_block.p);
     s->elem_blocks = t;
     s->node_blocks = t + eb.size();
     s->ghost_blocks = t + eb.size() + nb.size();
@@ -233,7 +233,8 @@ static int create_common(lulesh_set *s, const std::vector<DomPlace> &place, int 
         }
     }
     s->arena_bytes = total;
-    LCHECK(cudaMalloc(&s->arena, total));
+    LCHECK(block_get(&s->arena_block, total));
+    s->arena = s->arena_block.p;
     if (mixed) LCHECK(cudaMalloc(&s->dcorner32, sizeof(CornerF32) * s->ndom));
 
     // subdomain sets: every domain's x..zd side by side at the start of the
@@ -255,6 +256,8 @@ static int create_common(lulesh_set *s, const std::vector<DomPlace> &place, int 
     std::vector<CornerF32> hc32(s->ndom);
     std::vector<double> job_dt(s->njobs, 0.0);
 
+    std::vector<HostDomain> lights;  // until the stream has passed their uploads
+    lights.reserve(s->ndom);
     for (int d = 0; d < s->ndom; ++d) {
         const DomPlace &pl = place[d];
         const lulesh_job &j = s->jobs[pl.job];
@@ -281,6 +284,7 @@ static int create_common(lulesh_set *s, const std::vector<DomPlace> &place, int 
             s->job_origin[pl.job] = d;
             job_dt[pl.job] = h.deltatime;  // the origin domain's initial dt
         }
+        if (h.device_geometry) lights.push_back(std::move(h));
     }
     // a part of a problem split over GPUs: the job's dt starts from the
     // origin domain's even where that domain lives on another part
@@ -315,7 +319,14 @@ static int create_common(lulesh_set *s, const std::vector<DomPlace> &place, int 
                 }
     }
     const size_t ntab = s->hdoms.size() + s->hproxies.size();
-    LCHECK(cudaMalloc(&s->ddoms, sizeof(DomDev) * ntab));
+    // domain records, time control records and the run graph's counters
+    const size_t doms_bytes = align256(sizeof(DomDev) * ntab);
+    const size_t tc_bytes = align256(sizeof(TimeCtl) * 2 * s->njobs);
+    LCHECK(block_get(&s->ctl_block, doms_bytes + tc_bytes + 2 * sizeof(unsigned long long)));
+    char *ctl = static_cast<char *>(s->ctl_block.p);
+    s->ddoms = reinterpret_cast<DomDev *>(ctl);
+    s->dtc = reinterpret_cast<TimeCtl *>(ctl + doms_bytes);
+    s->run_ctl = reinterpret_cast<unsigned long long *>(ctl + doms_bytes + tc_bytes);
     LCHECK(cudaMemcpyAsync(s->ddoms, s->hdoms.data(), sizeof(DomDev) * s->ndom,
                            cudaMemcpyHostToDevice, s->stream));
     if (!s->hproxies.empty())
@@ -330,8 +341,8 @@ static int create_common(lulesh_set *s, const std::vector<DomPlace> &place, int 
     // time control blocks
     std::vector<TimeCtl> tc(s->njobs);
     for (int j = 0; j < s->njobs; ++j) tc[j] = initial_timectl(job_dt[j], s->jobs[j].its);
-    LCHECK(cudaMalloc(&s->dtc, sizeof(TimeCtl) * 2 * s->njobs));
-    LCHECK(cudaMallocHost(&s->htc_pinned, sizeof(TimeCtl) * s->njobs));
+    LCHECK(block_get(&s->pinned_block, sizeof(TimeCtl) * s->njobs, /*pinned=*/true));
+    s->htc_pinned = static_cast<TimeCtl *>(s->pinned_block.p);
     tc.insert(tc.end(), s->njobs, initial_timectl(0.0, 0));  // SetArgs::next
     LCHECK(cudaMemcpyAsync(s->dtc, tc.data(), sizeof(TimeCtl) * tc.size(),
                            cudaMemcpyHostToDevice, s->stream));
@@ -878,14 +889,10 @@ int lulesh_destroy(lulesh_set *s)
     clear_l2_window(s);
     comm_release(s);
     part_release(s);
-    if (s->elem_blocks) cudaFree(s->elem_blocks);
-    if (s->ddoms) cudaFree(s->ddoms);
-    if (s->dtc) cudaFree(s->dtc);
-    if (s->htc_pinned) cudaFreeHost(s->htc_pinned);
     if (s->dcorner32) cudaFree(s->dcorner32);
-    if (s->run_ctl) cudaFree(s->run_ctl);
     if (s->pack) cudaFree(s->pack);
-    if (s->arena) cudaFree(s->arena);
+    for (Block *b : {&s->tables_block, &s->ctl_block, &s->pinned_block, &s->arena_block})
+        block_put(b);
     if (s->own_stream && s->stream) cudaStreamDestroy(s->stream);
     delete s;
     return LULESH_OK;

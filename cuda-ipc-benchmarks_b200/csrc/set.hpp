@@ -6,6 +6,7 @@
 #include <string>
 #include <vector>
 
+#include "block_cache.hpp"
 #include "host_setup.hpp"
 #include "kernels.cuh"
 #include "lulesh_b200.h"
@@ -76,6 +77,8 @@ struct lulesh_set {
     // domain's x..zd, node_region_bytes), single domains carve in place
     void *arena = nullptr;
     size_t arena_bytes = 0;
+    // what the device pointers above and htc_pinned lie in
+    lulesh::Block arena_block, tables_block, ctl_block, pinned_block;
     void *pack = nullptr;  // nodePack and cornerPack of a scattered mesh
     size_t node_region_bytes = 0;
 
