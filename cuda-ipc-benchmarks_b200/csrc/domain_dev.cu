@@ -98,6 +98,8 @@ int upload_domain(const HostDomain &h, int tc, long comm_doubles, bool mixed, Ca
     DomDev D{};
     D.nx = h.nx;
     D.en = h.nx + 1;
+    D.by_nx = fast_div(D.nx);
+    D.by_en = fast_div(D.en);
     D.numElem = h.numElem;
     D.numNode = h.numNode;
     D.Ep = h.Ep;

@@ -47,11 +47,9 @@ __device__ __forceinline__ void elem_nodes(const DomDev &D, int el, int n[8])
         for (int k = 0; k < 8; ++k) n[k] = D.nodelist[(size_t)k * D.Ep + el];
         return;
     }
-    const int nx = D.nx, en = D.en;
-    const int ix = el % nx;
-    const int t = el / nx;
-    const int iy = t % nx;
-    const int iz = t / nx;
+    const int en = D.en;
+    int ix, iy, iz;
+    lattice(D.by_nx, el, ix, iy, iz);
     const int n0 = (iz * en + iy) * en + ix;
     n[0] = n0;
     n[1] = n0 + 1;

@@ -16,6 +16,14 @@ void lulesh_host_rand(unsigned seed, int n, int *out)
     for (int i = 0; i < n; ++i) out[i] = r.next();
 }
 
+// (a, b, c) of each of n[0..count) by lattice() for edge d (lulesh_dev.h).
+void lulesh_host_lattice(int d, const int *n, int count, int *out)
+{
+    const lulesh::FastDiv f = lulesh::fast_div(d);
+    for (int i = 0; i < count; ++i)
+        lulesh::lattice(f, n[i], out[3 * i], out[3 * i + 1], out[3 * i + 2]);
+}
+
 // Copy the named array of a built domain into out (capacity `cap` elements
 // of the array's type); returns the array length, -1 if unknown.
 static long copy_field(const lulesh::HostDomain &d, const char *name, void *out, long cap)

@@ -474,7 +474,11 @@ __device__ __forceinline__ void advance_node(const DomDev &D, double dt, const P
 // the others gather.
 template <int MODE, int BS, class W, bool INCR = false>
 __global__ void __launch_bounds__(INCR ? BS + 32 : BS,
-                                  min_blocks(INCR ? kNodalIncrMinBlocks : kNodalMinBlocks, BS))
+                                  min_blocks(INCR ? kNodalIncrMinBlocks
+                                             : std::is_same_v<W, FewDomains>
+                                                 ? kNodalFewMinBlocks
+                                                 : kNodalMinBlocks,
+                                             BS))
     k_nodal(const __grid_constant__ W w, Params P)
 {
     pdl_enter();
@@ -488,7 +492,8 @@ __global__ void __launch_bounds__(INCR ? BS + 32 : BS,
         const bool speaks = first_of_job(D, blk.y);
         if (W::kTable && !speaks && !increment_due(T, P)) return;
         const bool mine = threadIdx.x < BS && i < D.numNode;
-        const int en = D.en, px = i % en, t = i / en, py = t % en, pz = t / en;
+        int px, py, pz;
+        lattice(D.by_en, i, px, py, pz);
         double fx, fy, fz;
         if (threadIdx.x >= BS) {
             TimeCtl n = T;
@@ -511,11 +516,8 @@ __global__ void __launch_bounds__(INCR ? BS + 32 : BS,
     }
     if (W::kTable && !T.active) return;
     if (i >= D.numNode) return;
-    const int en = D.en;
-    const int px = i % en;
-    const int t = i / en;
-    const int py = t % en;
-    const int pz = t / en;
+    int px, py, pz;
+    lattice(D.by_en, i, px, py, pz);
 
     double fx, fy, fz;
     if (MODE == 0) {
@@ -815,7 +817,8 @@ __device__ __forceinline__ void elem_face_links(const DomDev &D, int z, int &bc,
                                                 int &xp, int &em, int &ep, int &zm, int &zp)
 {
     const int nx = D.nx, nn = nx * nx;
-    const int ix = z % nx, t = z / nx, iy = t % nx, iz = t / nx;
+    int ix, iy, iz;
+    lattice(D.by_nx, z, ix, iy, iz);
     bc = 0;
     xm = z - 1;
     xp = z + 1;
@@ -1091,7 +1094,8 @@ __global__ void __launch_bounds__(BS, min_blocks(kEosMinBlocks, BS))
             // comm faces: the mirrored element of the neighbour's opposite
             // face layer, where k_monoq_ghost would copy it from
             const int nx = D.nx;
-            const int ix = zidx % nx, t = zidx / nx, iy = t % nx, iz = t / nx;
+            int ix, iy, iz;
+            lattice(D.by_nx, zidx, ix, iy, iz);
             if (bcMask & XI_M_COMM) {
                 sm[0] = &w.doms()[D.nbr[0 + 3 + 9]];
                 lm[0] = (iz * nx + iy) * nx + (nx - 1);

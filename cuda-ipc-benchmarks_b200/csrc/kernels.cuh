@@ -46,12 +46,15 @@ constexpr int kNodeBlock = 128;  // threads per block, node kernels
 #ifndef LULESH_EOS_MINB
 #define LULESH_EOS_MINB 8
 #endif
-// nodal: 16 blocks (32 registers, every warp slot of the SM) for the
-// streaming corner gather, 60.2 -> 56.7 us
+// nodal: 12 blocks (40 registers) for the streaming corner gather, 41.6 us at
+// -s 100 and 188 at -s 160; 44.6 and 195 at 16 (32 registers, spills), 41.6 and
+// 187 at 10.  The subdomain gather, whose neighbour records add latency, wants
+// every warp slot: 54.8 us at 16, 56.6 at 12, 59.3 at 10 (2x2x2 of -s 50).
 #ifndef LULESH_NODAL_MINB
-#define LULESH_NODAL_MINB 16
+#define LULESH_NODAL_MINB 12
 #endif
 constexpr int kNodalMinBlocks = LULESH_NODAL_MINB;
+constexpr int kNodalFewMinBlocks = 16;
 // with the time increment's warp (small sets, one wave): registers for all
 // corner loads of a node at once
 #ifndef LULESH_NODAL_INCR_MINB

@@ -52,12 +52,62 @@ struct TimeCtl {
     int chk;         // checked builds: code of the first index out of range, 0 none
 };
 
+// n / d and n % d for 0 <= n < 2^31 by a multiplication (Granlund and
+// Montgomery, "Division by invariant integers using multiplication", 1994): the
+// first thing a kernel does with its element or node number, a chain of some
+// 40 instructions each before the first gather otherwise.  d = 1 divides only
+// n = 0, the one element of such a mesh.
+struct FastDiv {
+    unsigned mul, shift;
+    int d;
+};
+
+inline FastDiv fast_div(int d)
+{
+    FastDiv f{0, 0, d};
+    if (d <= 1) return f;
+    int l = 0;
+    while ((1ll << l) < d) ++l;
+    f.mul = (unsigned)((1ull << (31 + l)) / (unsigned)d + 1);
+    f.shift = (unsigned)(l - 1);
+    return f;
+}
+
+#ifdef __CUDACC__
+__host__ __device__ __forceinline__
+#else
+inline
+#endif
+int quotient(const FastDiv &f, int n)
+{
+#ifdef __CUDA_ARCH__
+    return (int)(__umulhi((unsigned)n, f.mul) >> f.shift);
+#else
+    return (int)((unsigned)(((unsigned long long)(unsigned)n * f.mul) >> 32) >> f.shift);
+#endif
+}
+
+// (a, b, c) of n = (c * d + b) * d + a
+#ifdef __CUDACC__
+__host__ __device__ __forceinline__
+#else
+inline
+#endif
+void lattice(const FastDiv &f, int n, int &a, int &b, int &c)
+{
+    const int t = quotient(f, n);
+    a = n - t * f.d;
+    c = quotient(f, t);
+    b = t - c * f.d;
+}
+
 // One domain.  Sizes follow lulesh.cu:783-798; node (px,py,pz) has index
 // (pz*en + py)*en + px and element (ix,iy,iz) index (iz*nx + iy)*nx + ix,
 // exactly the order BuildMesh (lulesh.cu:688-747) produces.
 struct DomDev {
     int nx, en, numElem, numNode, Ep, allElem;
     int col, row, plane, tp;
+    FastDiv by_nx, by_en;  // of element and node numbers
     int tc;        // TimeCtl index
     int numReg;
     int nbr[27];   // domain index of the neighbour at (dx,dy,dz)+1 (x fastest), -1 none

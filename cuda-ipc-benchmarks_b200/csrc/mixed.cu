@@ -40,8 +40,9 @@ namespace lulesh {
 
 __device__ __forceinline__ void elem_nodes_m(const DomDev &D, int el, int n[8])
 {
-    const int nx = D.nx, en = D.en;
-    const int ix = el % nx, t = el / nx, iy = t % nx, iz = t / nx;
+    const int en = D.en;
+    int ix, iy, iz;
+    lattice(D.by_nx, el, ix, iy, iz);
     const int n0 = (iz * en + iy) * en + ix;
     n[0] = n0;
     n[1] = n0 + 1;
@@ -176,8 +177,9 @@ __global__ void __launch_bounds__(kNodeBlock, min_blocks(LULESH_MIXED_NODAL_MINB
     const int i = blk.y + threadIdx.x;
     if (i >= D.numNode) return;
     const CornerF32 cf = corner_arrays(w, cfs, cf1, blk.x);
-    const int en = D.en, nx = D.nx;
-    const int px = i % en, t = i / en, py = t % en, pz = t / en;
+    const int nx = D.nx;
+    int px, py, pz;
+    lattice(D.by_en, i, px, py, pz);
     float sx = 0.f, sy = 0.f, sz = 0.f, cx = 0.f, cy = 0.f, cz = 0.f;
     const int ox[8] = {0, 1, 1, 0, 0, 1, 1, 0}, oy[8] = {0, 0, 1, 1, 0, 0, 1, 1},
               oz[8] = {0, 0, 0, 0, 1, 1, 1, 1};

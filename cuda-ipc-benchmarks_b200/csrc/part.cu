@@ -276,6 +276,8 @@ int part_build(lulesh_set *s)
         DomDev P{};
         P.nx = j.nx;
         P.en = j.nx + 1;
+        P.by_nx = fast_div(P.nx);
+        P.by_en = fast_div(P.en);
         P.numElem = (int)z.E;
         P.numNode = (int)z.N;
         P.Ep = (int)z.Ep;
