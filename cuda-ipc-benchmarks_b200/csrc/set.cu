@@ -459,8 +459,7 @@ static int l2_node_window_on_device(lulesh_set *s);
 // current for the call, whatever device the calling thread has
 static int l2_node_window(lulesh_set *s)
 {
-    if (!LULESH_L2_WINDOW || (s->ndom != 1 && !s->node_region_bytes) || s->l2_window)
-        return LULESH_OK;
+    if (!LULESH_L2_WINDOW || (s->ndom != 1 && !s->node_region_bytes)) return LULESH_OK;
     int prev = -1;
     LCHECK(cudaGetDevice(&prev));
     if (prev != s->device) LCHECK(cudaSetDevice(s->device));
@@ -501,9 +500,11 @@ static int l2_node_window_on_device(lulesh_set *s)
             LCHECK(cudaDeviceSetLimit(cudaLimitPersistingL2CacheSize, persist));
             g.now = persist;
         }
-        ++g.sets;
+        if (!s->l2_window) ++g.sets;
         s->l2_window = true;  // counted: clear_l2_window undoes it
     }
+    // at every capture: sets may share the caller's stream, and its attribute
+    // is then the window of the set prepared last, or none after one is closed
     cudaStreamAttrValue v{};
     v.accessPolicyWindow.base_ptr = const_cast<char *>(lo);
     v.accessPolicyWindow.num_bytes = bytes;
@@ -563,8 +564,8 @@ static int cycles_per_launch(lulesh_set *s, int n)
 static int ensure_graph_k(lulesh_set *s, int k)
 {
     if (s->graph_k_ready) return LULESH_OK;
-    int st = ensure_graph(s);  // prepares comm tables when staged
-    if (st != LULESH_OK) return st;
+    int st = ensure_graph(s);
+    if (st != LULESH_OK || (st = prepare_capture(s)) != LULESH_OK) return st;
     LCHECK(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
     for (int c = 0; c < k && st == LULESH_OK; ++c) st = enqueue_cycle(s);
     cudaGraph_t g = nullptr;
