@@ -1028,6 +1028,71 @@ __device__ __forceinline__ int eos_block(const DomDev &D, int b)
     return b % kEosMix == 0 ? b / kEosMix : heavy + b - b / kEosMix - 1;
 }
 
+// Lanes that share the reps of an element of a domain's costliest class: a
+// power of two, at most kRepLanes and the class's reps, while the kernel stays
+// one wave of blocks; 1 otherwise.  In one wave the costliest class's reps, 20
+// by default, are the kernel's longest chain while lanes stand idle.  Every rep
+// is still evaluated: lane k has reps k, k + lanes, ..., and the lane of the
+// last one writes.  Cycle on B200, us, 1 -> 4, 8, 16 lanes: -s 10 15.6 -> 14.6,
+// 14.6, 14.6; -s 20 16.9 -> 16.0, 16.0, 16.2; -s 30 17.7 -> 16.7, 18.7, 18.7;
+// -s 45 26.1 -> 25.3 (all); with cost 3 18.1 -> 15.5, 18.1 -> 15.1, 20.3 ->
+// 17.7, 28.3 -> 25.3 (4 lanes).  Past one wave the class's warps run beside the
+// others', and its loads would be made by more of them.
+#ifndef LULESH_REP_LANES
+#define LULESH_REP_LANES 4
+#endif
+constexpr int kRepLanes = LULESH_REP_LANES;
+
+// blocks of the costliest class with its reps shared, and of the other slots
+__host__ __device__ __forceinline__ int shared_blocks(const DomDev &D, int lanes, int bs)
+{
+    return (int)(((long long)D.eosClassEnd[0] * lanes + bs - 1) / bs);
+}
+__host__ __device__ __forceinline__ int other_blocks(const DomDev &D, int bs)
+{
+    return (D.numElem - D.eosClassEnd[0] + bs - 1) / bs;
+}
+
+static int rep_lanes(const DomDev &D, int bs)
+{
+    const int wave = 148 * min_blocks(kEosMinBlocks, bs);
+    int lanes = kRepLanes;
+    while (lanes > 1 && (lanes > D.eosClassRep[0] ||
+                         shared_blocks(D, lanes, bs) + other_blocks(D, bs) > wave))
+        lanes /= 2;
+    return lanes;
+}
+
+// A thread's place in the EOS kernel: its slot, the reps it evaluates, and
+// whether it writes the element's results (the thread that has the last rep).
+struct EosPlace {
+    int slot, rep;
+    bool writes;
+};
+
+template <int BS, bool SHARE>
+__device__ __forceinline__ EosPlace eos_place(const DomDev &D, int b, int lanes)
+{
+    EosPlace p{eos_block<BS>(D, b) * BS + (int)threadIdx.x, 0, true};
+    if (SHARE) {
+        const int shared = shared_blocks(D, lanes, BS), costly = D.eosClassEnd[0];
+        if (b < shared) {
+            const int t = b * BS + threadIdx.x, part = t & (lanes - 1);
+            const int rep = D.eosClassRep[0];
+            p.slot = t >> (31 - __clz(lanes));
+            if (p.slot >= costly) p.slot = D.numElem;  // past the class: none
+            p.rep = (rep - part + lanes - 1) >> (31 - __clz(lanes));
+            p.writes = part == ((rep - 1) & (lanes - 1));
+            return p;
+        }
+        p.slot = costly + (b - shared) * BS + threadIdx.x;
+    }
+    int cls = 0;
+    while (cls < D.eosNumClass - 1 && p.slot >= D.eosClassEnd[cls]) ++cls;
+    p.rep = D.eosClassRep[cls];
+    return p;
+}
+
 // SUB: a subdomain set's fused cycle, which reads a comm face's neighbour
 // element in the neighbouring subdomain (no MonoQ ghost copy)
 //
@@ -1041,28 +1106,26 @@ __device__ __forceinline__ int eos_block(const DomDev &D, int b)
 // Elements in natural order instead of class order: 57.8 us at 8 blocks,
 // 53.7 at 9, but 150 against 136 us at -s 133 with cost 4, where every warp
 // runs its costliest element's reps.
-template <int BS, bool U, bool SUB, class W>
+template <int BS, bool U, bool SUB, class W, bool SHARE = false>
 __global__ void __launch_bounds__(BS, min_blocks(kEosMinBlocks, BS))
-    k_eos(const __grid_constant__ W w, Params P)
+    k_eos(const __grid_constant__ W w, Params P, int lanes)
 {
     pdl_enter();
     const int2 blk = w.template block<BS, LULESH_EOS_REVERSE>();
     const DomDev &D = w.domain(blk.x);
     TimeCtl &T = w.time(D);
     if (!T.active) return;  // uniform per block
-    const int i = eos_block<BS>(D, blk.y / BS) * BS + threadIdx.x;
+    const EosPlace place = eos_place<BS, SHARE>(D, blk.y / BS, lanes);
     double dtc = 1.0e+20, vmax = 0.0;
-    if (i < D.numElem) {
+    if (place.slot < D.numElem) {
         // The element of this slot and its rep count.  The reference visits
         // regElemlist and finds the rep by region (giveMyRegion,
         // lulesh.cu:3976-3984); here slots are grouped by rep class
         // (HostDomain::eosOrder), which keeps the trip count uniform per warp
         // with denser loads (measured 98 us vs 99 us regElemlist order and
         // 108 us natural order at -s 100).
-        const int zidx = chk_index(D.eosOrder[i], D.numElem, &T, kChkSlot);
-        int cls = 0;
-        while (cls < D.eosNumClass - 1 && i >= D.eosClassEnd[cls]) ++cls;
-        const int rep = D.eosClassRep[cls];
+        const int zidx = chk_index(D.eosOrder[place.slot], D.numElem, &T, kChkSlot);
+        const int rep = place.rep;
 
         // Every array the element needs, before any arithmetic, branch or
         // store.  A face on the mesh boundary reads the element itself: its
@@ -1169,8 +1232,9 @@ __global__ void __launch_bounds__(BS, min_blocks(kEosMinBlocks, BS))
                      delvxeta * delvxeta * (1. - phieta * phieta) +
                      delvxzeta * delvxzeta * (1. - phizeta * phizeta));
         }
-        if (q_old_z > P.qstop) atomicMin(&T.bad_q, zidx);
-        if (w.materialize()) {
+        const bool writes = !SHARE || place.writes;
+        if (writes && q_old_z > P.qstop) atomicMin(&T.bad_q, zidx);
+        if (writes && w.materialize()) {
             D.qq[zidx] = qquad;
             D.ql[zidx] = qlin;
         }
@@ -1191,7 +1255,7 @@ __global__ void __launch_bounds__(BS, min_blocks(kEosMinBlocks, BS))
         if (eosvmax != 0.) {
             if (vc > eosvmax) vc = eosvmax;
         }
-        if (vc <= 0.) atomicMin(&T.bad_vol, zidx);
+        if (writes && vc <= 0.) atomicMin(&T.bad_vol, zidx);
 
         double p_new = 0., e_new = 0., q_new = 0., bvc = 0., pbvc = 0.;
         const double rho0 = P.refdens;
@@ -1203,9 +1267,11 @@ __global__ void __launch_bounds__(BS, min_blocks(kEosMinBlocks, BS))
         else
             eos_reps<false>(rep, e_temp, p_temp, q_old_z, qquad, qlin, delvc_temp, vnewc,
                             eosvmin, eosvmax, rho0, P, p_new, e_new, q_new, bvc, pbvc);
-        D.p[zidx] = p_new;
-        D.e[zidx] = e_new;
-        D.q[zidx] = q_new;
+        if (writes) {
+            D.p[zidx] = p_new;
+            D.e[zidx] = e_new;
+            D.q[zidx] = q_new;
+        }
 
         // CalcSoundSpeedForElems_device, lulesh.cu:3795-3809
         double ssTmp = pbvc * e_new + vnewc * vnewc * bvc * p_new;
@@ -1214,12 +1280,12 @@ __global__ void __launch_bounds__(BS, min_blocks(kEosMinBlocks, BS))
             ssTmp = .3333333e-18;
         else
             ssTmp = sqrt(ssTmp);
-        D.ss[zidx] = ssTmp;
+        if (writes) D.ss[zidx] = ssTmp;
 
         // UpdateVolumesForElems_device, lulesh.cu:3850-3861
         double tmpV = vnew_z;
         if (fabs(tmpV - 1.0) < P.v_cut) tmpV = 1.0;
-        D.v[zidx] = tmpV;
+        if (writes) D.v[zidx] = tmpV;
 
         // CalcTimeConstraintsForElems_kernel body, lulesh.cu:4246-4279
         const double qqc2 = 64.0 * P.qqc * P.qqc;
@@ -1229,7 +1295,7 @@ __global__ void __launch_bounds__(BS, min_blocks(kEosMinBlocks, BS))
         double dtf = ss_tmp * ss_tmp;
         dtf += ((vdov_tmp < 0.) ? qqc2 * area_tmp * area_tmp * vdov_tmp * vdov_tmp : 0.);
         dtf = area_tmp * rsqrt(dtf);
-        if (vdov_tmp != 0. && dtf < dtc) dtc = dtf;
+        if (writes && vdov_tmp != 0. && dtf < dtc) dtc = dtf;
     }
     // block minimum (exact, order-free), one atomic per block.  The hydro
     // limit dvovmax / (|vdov| + tiny) falls as |vdov| grows, also after
@@ -1259,31 +1325,43 @@ __global__ void __launch_bounds__(BS, min_blocks(kEosMinBlocks, BS))
     }
 }
 
-template <int BS, bool SUB>
+template <int BS, bool U, bool SUB>
 static void launch_eos_bs(const SetArgs &a, int nblocks, Params P, cudaStream_t s)
 {
-    launch_where<!SUB, SUB>(a, nblocks, [&](const auto &w) {
-        launch_k(k_eos<BS, false, SUB, std::decay_t<decltype(w)>>, nblocks, BS, s, a.pdl != 0, w,
-                 P);
-    });
+    const int lanes = !SUB && a.records && a.ndom == 1 ? rep_lanes(a.records[0], BS) : 1;
+    if constexpr (!SUB) {
+        if (lanes > 1) {
+            const int n = shared_blocks(a.records[0], lanes, BS) + other_blocks(a.records[0], BS);
+            launch_k(k_eos<BS, U, false, OneDomain, true>, n, BS, s, a.pdl != 0, by_value<1>(a, n),
+                     P, lanes);
+            return;
+        }
+    }
+    if constexpr (U)
+        launch_k(k_eos<BS, true, false, OneDomain>, nblocks, BS, s, a.pdl != 0,
+                 by_value<1>(a, nblocks), P, 1);
+    else
+        launch_where<!SUB, SUB>(a, nblocks, [&](const auto &w) {
+            launch_k(k_eos<BS, false, SUB, std::decay_t<decltype(w)>>, nblocks, BS, s, a.pdl != 0,
+                     w, P, 1);
+        });
 }
 
 void launch_eos(const SetArgs &a, int nblocks, Params P, cudaStream_t s, int bs, bool u,
                 bool sub)
 {
     if (u) {
-        launch_k(k_eos<kElemBlock, true, false, OneDomain>, nblocks, kElemBlock, s, a.pdl != 0,
-                 by_value<1>(a, nblocks), P);
+        launch_eos_bs<kElemBlock, true, false>(a, nblocks, P, s);
         return;
     }
     if (sub) {  // subdomain sets take 128-element blocks only
-        launch_eos_bs<kElemBlock, true>(a, nblocks, P, s);
+        launch_eos_bs<kElemBlock, false, true>(a, nblocks, P, s);
         return;
     }
     switch (bs) {
-        case 64: launch_eos_bs<64, false>(a, nblocks, P, s); break;
-        case 256: launch_eos_bs<256, false>(a, nblocks, P, s); break;
-        default: launch_eos_bs<kElemBlock, false>(a, nblocks, P, s); break;
+        case 64: launch_eos_bs<64, false, false>(a, nblocks, P, s); break;
+        case 256: launch_eos_bs<256, false, false>(a, nblocks, P, s); break;
+        default: launch_eos_bs<kElemBlock, false, false>(a, nblocks, P, s); break;
     }
 }
 
