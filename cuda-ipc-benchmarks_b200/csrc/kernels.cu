@@ -1,6 +1,7 @@
 // kernels.cu -- the per-cycle kernels of the LULESH Lagrange leapfrog step.
 //
-// One cycle is five launches (captured in one CUDA graph):
+// One cycle is five launches (captured in CUDA graphs), four in sets of one
+// wave, whose kernels make the time increment themselves:
 //   time_increment  TimeIncrement on the device (lulesh.cu:1400-1461)
 //   force           CalcVolumeForceForElems_kernel (lulesh.cu:2080-2259):
 //                   stress + FB hourglass corner forces per element
@@ -22,9 +23,10 @@
 // neither (every corner of every node is summed in single-domain order, and
 // k_eos<..., SUB> reads comm-face neighbours in place), and the parts of a
 // multi-GPU problem read their proxies in place after the MONOQ messages.
-// Unstructured (lmesh) domains run force, kinematics and EOS with U = true,
-// which reads nodelist, the face links and elemBC from memory instead of
-// computing them from the element index, and k_nodal_u for the nodal step.
+// Unstructured (lmesh) domains run force and kinematics with Mesh::kLists and
+// EOS with U = true, which read nodelist, the face links and elemBC from memory
+// instead of computing them from the element index, and k_nodal_u for the nodal
+// step; scattered ones Mesh::kPacked, k_begin_packed and k_nodal_packed.
 #include <climits>
 #include <cstdint>
 #include <type_traits>
@@ -257,10 +259,8 @@ void launch_begin_packed(const SetArgs &a, int nblocks, Params P, cudaStream_t s
 // and 312 against 272 us at -s 160.
 template <bool HG, Mesh M, bool TABLE>
 __device__ __forceinline__ void force_one(const DomDev &D, bool active, TimeCtl &E, const Params &P,
-                                          int elem)
+                                          int elem, int (&n)[8])
 {
-    int n[8];
-    elem_nodes<M != Mesh::kBox>(D, elem, n);
 #pragma unroll
     for (int i = 0; i < 8; ++i) n[i] = chk_index(n[i], D.numNode, &E, kChkNode);
     double vn[3][8], xn[8], yn[8], zn[8];
@@ -315,15 +315,22 @@ template <bool HG, int BS, Mesh M, class W>
 __global__ void __launch_bounds__(BS, min_blocks(kForceMinBlocks, BS))
     k_force(const __grid_constant__ W w, Params P)
 {
-    pdl_enter();
+    // an lmesh cycle begins with another kernel: the node ids may come early
+    if (M == Mesh::kBox) pdl_enter();
     const int2 blk = w.template block<BS, LULESH_FORCE_REVERSE>();
     const DomDev &D = w.domain(blk.x);
+    const int elem = blk.y + threadIdx.x;
+    int n[8];
+    if (M != Mesh::kBox) {
+        if (elem < D.numElem) elem_nodes<true>(D, elem, n);
+        pdl_enter();
+    }
     const TimeCtl &T = w.time(D);
     const bool active = w.increments() ? increment_due(T, P) : T.active != 0;
     if (W::kTable && !active) return;
-    const int elem = blk.y + threadIdx.x;
     if (elem >= D.numElem) return;
-    force_one<HG, M, W::kTable>(D, active, w.next(D), P, elem);
+    if (M == Mesh::kBox) elem_nodes<false>(D, elem, n);
+    force_one<HG, M, W::kTable>(D, active, w.next(D), P, elem, n);
 }
 
 template <int BS, Mesh M, class W>
@@ -420,15 +427,48 @@ __device__ __forceinline__ void gather_corners(const DomDev *doms, const DomDev 
     }
 }
 
+// Node i's state where the update reads it
+struct NodeNow {
+    const DomDev &D;
+    int i;
+    __device__ __forceinline__ double mass() const { return D.nodalMass[i]; }
+    __device__ __forceinline__ double x() const { return D.x[i]; }
+    __device__ __forceinline__ double y() const { return D.y[i]; }
+    __device__ __forceinline__ double z() const { return D.z[i]; }
+    __device__ __forceinline__ double xd() const { return D.xd[i]; }
+    __device__ __forceinline__ double yd() const { return D.yd[i]; }
+    __device__ __forceinline__ double zd() const { return D.zd[i]; }
+};
+
+// or before pdl_enter
+struct NodeEarly {
+    double vm, vx, vy, vz, vxd, vyd, vzd;
+    __device__ __forceinline__ void read(const DomDev &D, int i)
+    {
+        vm = __ldcg(D.nodalMass + i);
+        vxd = __ldcg(D.xd + i), vyd = __ldcg(D.yd + i), vzd = __ldcg(D.zd + i);
+        vx = __ldcg(D.x + i), vy = __ldcg(D.y + i), vz = __ldcg(D.z + i);
+    }
+    __device__ __forceinline__ double mass() const { return vm; }
+    __device__ __forceinline__ double x() const { return vx; }
+    __device__ __forceinline__ double y() const { return vy; }
+    __device__ __forceinline__ double z() const { return vz; }
+    __device__ __forceinline__ double xd() const { return vxd; }
+    __device__ __forceinline__ double yd() const { return vyd; }
+    __device__ __forceinline__ double zd() const { return vzd; }
+};
+
 // CalcAccelerationForNodes (lulesh.cu:2926-2939), the symmetry-plane zeroing
 // of ApplyAccelerationBoundaryConditionsForNodes (bc bits 0/1/2 zero the
 // x/y/z acceleration) and CalcPositionAndVelocityForNodes (lulesh.cu:
 // 2999-3028) for node i with the summed force (fx, fy, fz)
+template <class Node>
 __device__ __forceinline__ void advance_node(const DomDev &D, double dt, const Params &P, int i,
                                              int bc, double fx, double fy, double fz,
-                                             int materialize, bool write_f, bool pack = false)
+                                             int materialize, bool write_f, const Node &n,
+                                             bool pack = false)
 {
-    const double one_over_nMass = 1. / D.nodalMass[i];
+    const double one_over_nMass = 1. / n.mass();
     double xdd = fx * one_over_nMass;
     double ydd = fy * one_over_nMass;
     double zdd = fz * one_over_nMass;
@@ -437,15 +477,15 @@ __device__ __forceinline__ void advance_node(const DomDev &D, double dt, const P
     if (bc & 4) zdd = 0.0;
 
     const double u_cut = P.u_cut;
-    double xdtmp = D.xd[i] + xdd * dt;
-    double ydtmp = D.yd[i] + ydd * dt;
-    double zdtmp = D.zd[i] + zdd * dt;
+    double xdtmp = n.xd() + xdd * dt;
+    double ydtmp = n.yd() + ydd * dt;
+    double zdtmp = n.zd() + zdd * dt;
     if (fabs(xdtmp) < u_cut) xdtmp = 0.0;
     if (fabs(ydtmp) < u_cut) ydtmp = 0.0;
     if (fabs(zdtmp) < u_cut) zdtmp = 0.0;
-    const double x = D.x[i] + xdtmp * dt;
-    const double y = D.y[i] + ydtmp * dt;
-    const double z = D.z[i] + zdtmp * dt;
+    const double x = n.x() + xdtmp * dt;
+    const double y = n.y() + ydtmp * dt;
+    const double z = n.z() + zdtmp * dt;
     D.x[i] = x;
     D.y[i] = y;
     D.z[i] = z;
@@ -481,12 +521,15 @@ __global__ void __launch_bounds__(INCR ? BS + 32 : BS,
                                              BS))
     k_nodal(const __grid_constant__ W w, Params P)
 {
-    pdl_enter();
+    if (!INCR) pdl_enter();
     const int2 blk = w.template block<BS, LULESH_NODAL_REVERSE && !W::kTable>();
     const DomDev &D = w.domain(blk.x);
     TimeCtl &T = w.time(D);
     const int i = blk.y + threadIdx.x;
     if constexpr (INCR) {
+        NodeEarly node;
+        if (!W::kTable && threadIdx.x < BS && i < D.numNode) node.read(D, i);
+        pdl_enter();
         __shared__ double s_dt;
         __shared__ int s_active;
         const bool speaks = first_of_job(D, blk.y);
@@ -509,9 +552,10 @@ __global__ void __launch_bounds__(INCR ? BS + 32 : BS,
         }
         __syncthreads();
         if (!mine || !s_active) return;
+        if (W::kTable) node.read(D, i);
         const int bc = (D.col == 0 && px == 0 ? 1 : 0) | (D.row == 0 && py == 0 ? 2 : 0) |
                        (D.plane == 0 && pz == 0 ? 4 : 0);
-        advance_node(D, s_dt, P, i, bc, fx, fy, fz, w.materialize(), true);
+        advance_node(D, s_dt, P, i, bc, fx, fy, fz, w.materialize(), true, node);
         return;
     }
     if (W::kTable && !T.active) return;
@@ -539,7 +583,8 @@ __global__ void __launch_bounds__(INCR ? BS + 32 : BS,
     const int bc = (D.col == 0 && px == 0 ? 1 : 0) | (D.row == 0 && py == 0 ? 2 : 0) |
                    (D.plane == 0 && pz == 0 ? 4 : 0);
     if (!W::kTable && !T.active) return;
-    advance_node(D, T.deltatime, P, i, bc, fx, fy, fz, w.materialize(), MODE == 0);
+    advance_node(D, T.deltatime, P, i, bc, fx, fy, fz, w.materialize(), MODE == 0,
+                 NodeNow{D, i});
 }
 
 // Scattered meshes: the corner forces of a node, one sector each, summed in
@@ -547,14 +592,19 @@ __global__ void __launch_bounds__(INCR ? BS + 32 : BS,
 __global__ void __launch_bounds__(kNodeBlock)
     k_nodal_packed(const __grid_constant__ OneDomain w, Params P)
 {
-    pdl_enter();
     const DomDev &D = w.D[0];
     TimeCtl &T = *w.tc;
     const int i = blockIdx.x * kNodeBlock + threadIdx.x;
-    if (i >= D.numNode) return;
-    int k[8];
+    int k[8], bc = 0;
+    NodeEarly node;
+    if (i < D.numNode) {
 #pragma unroll
-    for (int j = 0; j < 8; ++j) k[j] = D.packedCornerEll[(size_t)j * D.numNode + i];
+        for (int j = 0; j < 8; ++j) k[j] = D.packedCornerEll[(size_t)j * D.numNode + i];
+        bc = D.nodeBC[i];
+        node.read(D, i);
+    }
+    pdl_enter();
+    if (i >= D.numNode) return;
     double vx[8], vy[8], vz[8], pad;
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
@@ -573,7 +623,7 @@ __global__ void __launch_bounds__(kNodeBlock)
             fz += vz[j];
         }
     }
-    advance_node(D, T.deltatime, P, i, D.nodeBC[i], fx, fy, fz, w.mat, true, /*pack=*/true);
+    advance_node(D, T.deltatime, P, i, bc, fx, fy, fz, w.mat, true, node, /*pack=*/true);
 }
 
 // Unstructured meshes: AddNodeForcesFromElems (lulesh.cu:1715-1751) over
@@ -587,23 +637,26 @@ template <int BS>
 __global__ void __launch_bounds__(BS, min_blocks(kNodalUMinBlocks, BS))
     k_nodal_u(const __grid_constant__ OneDomain w, Params P)
 {
-    pdl_enter();
     __shared__ int s_list[8 * BS];
     const int2 blk = w.template block<BS, LULESH_NODAL_REVERSE>();
     const DomDev &D = w.D[0];
     const TimeCtl &T = *w.tc;
-    if (!T.active) return;  // the whole block
     const int first = blk.y;
     const int last = min(first + BS, D.numNode) - 1;
+    int slot[8];
+    if (D.nodeCornerEll && first + (int)threadIdx.x <= last) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+            slot[j] = D.nodeCornerEll[(size_t)j * D.numNode + first + threadIdx.x];
+    }
+    pdl_enter();
+    if (!T.active) return;  // the whole block
     if (D.nodeCornerEll) {
         // the run slot-major (uniform per block: no staging, no barrier):
         // eight coalesced loads, then the corners, summed in run order
         const int i = first + threadIdx.x;
         if (i > last) return;
-        const int N = D.numNode;
-        int k[8];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) k[j] = D.nodeCornerEll[(size_t)j * N + i];
+        const int(&k)[8] = slot;
         double fx = 0.0, fy = 0.0, fz = 0.0;
 #pragma unroll
         for (int h = 0; h < 8; h += 4) {
@@ -627,7 +680,7 @@ __global__ void __launch_bounds__(BS, min_blocks(kNodalUMinBlocks, BS))
                     fz += vz[q];
                 }
         }
-        advance_node(D, T.deltatime, P, i, D.nodeBC[i], fx, fy, fz, w.mat, true);
+        advance_node(D, T.deltatime, P, i, D.nodeBC[i], fx, fy, fz, w.mat, true, NodeNow{D, i});
         return;
     }
     const long long list_len = 8LL * D.numElem;  // corner-list entries
@@ -679,7 +732,7 @@ __global__ void __launch_bounds__(BS, min_blocks(kNodalUMinBlocks, BS))
         fz += ld_corner(D.fz_elem + k);
     }
     // symmetry nodes of the mesh's X/Y/Z sets: nodeBC bits 0/1/2
-    advance_node(D, T.deltatime, P, i, D.nodeBC[i], fx, fy, fz, w.mat, true);
+    advance_node(D, T.deltatime, P, i, D.nodeBC[i], fx, fy, fz, w.mat, true, NodeNow{D, i});
 }
 
 template <int BS>
@@ -735,17 +788,19 @@ __global__ void __launch_bounds__(BS, min_blocks(M == Mesh::kPacked ? kKinPacked
                                                                     : kKinMinBlocks, BS))
     k_kinematics(const __grid_constant__ W w)
 {
-    pdl_enter();
     const int2 blk = w.template block<BS, LULESH_KIN_REVERSE>();
     const DomDev &D = w.domain(blk.x);
     TimeCtl &T = w.time(D), &N = w.next(D);
+    int n[8];
+    if (M != Mesh::kBox && blk.y + (int)threadIdx.x < D.numElem)
+        elem_nodes<true>(D, blk.y + threadIdx.x, n);
+    pdl_enter();
     if (w.increments() && threadIdx.x == 0 && first_of_job(D, blk.y)) commit_increment(T, N);
     if (W::kTable && !N.active) return;
     const int k = blk.y + threadIdx.x;
     if (k >= D.numElem) return;
 
-    int n[8];
-    elem_nodes<M != Mesh::kBox>(D, k, n);
+    if (M == Mesh::kBox) elem_nodes<false>(D, k, n);
 #pragma unroll
     for (int l = 0; l < 8; ++l) n[l] = chk_index(n[l], D.numNode, &T, kChkNode);
     double xn[8], yn[8], zn[8];
@@ -1110,12 +1165,24 @@ template <int BS, bool U, bool SUB, class W, bool SHARE = false>
 __global__ void __launch_bounds__(BS, min_blocks(kEosMinBlocks, BS))
     k_eos(const __grid_constant__ W w, Params P, int lanes)
 {
-    pdl_enter();
     const int2 blk = w.template block<BS, LULESH_EOS_REVERSE>();
     const DomDev &D = w.domain(blk.x);
     TimeCtl &T = w.time(D);
-    if (!T.active) return;  // uniform per block
     const EosPlace place = eos_place<BS, SHARE>(D, blk.y / BS, lanes);
+    // before pdl_enter: the element, and in a set of one wave what the
+    // kinematics kernel does not write
+    int zidx = 0;
+    double mass_z, volo_z, q_old_z, v_z, e_temp, p_temp;
+    if (place.slot < D.numElem) {
+        zidx = chk_index(D.eosOrder[place.slot], D.numElem, &T, kChkSlot);
+        if (SHARE) {
+            mass_z = __ldcg(D.elemMass + zidx), volo_z = __ldcg(D.volo + zidx);
+            q_old_z = __ldcg(D.q + zidx), v_z = __ldcg(D.v + zidx);
+            e_temp = __ldcg(D.e + zidx), p_temp = __ldcg(D.p + zidx);
+        }
+    }
+    pdl_enter();
+    if (!T.active) return;  // uniform per block
     double dtc = 1.0e+20, vmax = 0.0;
     if (place.slot < D.numElem) {
         // The element of this slot and its rep count.  The reference visits
@@ -1124,7 +1191,6 @@ __global__ void __launch_bounds__(BS, min_blocks(kEosMinBlocks, BS))
         // (HostDomain::eosOrder), which keeps the trip count uniform per warp
         // with denser loads (measured 98 us vs 99 us regElemlist order and
         // 108 us natural order at -s 100).
-        const int zidx = chk_index(D.eosOrder[place.slot], D.numElem, &T, kChkSlot);
         const int rep = place.rep;
 
         // Every array the element needs, before any arithmetic, branch or
@@ -1196,9 +1262,12 @@ __global__ void __launch_bounds__(BS, min_blocks(kEosMinBlocks, BS))
         const double vdov_z = D.vdov[zidx];
         const double vnew_z = D.vnew[zidx];
         const double xxi = D.delx_xi[zidx], xeta = D.delx_eta[zidx], xzeta = D.delx_zeta[zidx];
-        const double mass_z = D.elemMass[zidx], volo_z = D.volo[zidx];
-        const double q_old_z = D.q[zidx], v_z = D.v[zidx];
-        const double e_temp = D.e[zidx], p_temp = D.p[zidx], delvc_temp = D.delv[zidx];
+        if (!SHARE) {
+            mass_z = D.elemMass[zidx], volo_z = D.volo[zidx];
+            q_old_z = D.q[zidx], v_z = D.v[zidx];
+            e_temp = D.e[zidx], p_temp = D.p[zidx];
+        }
+        const double delvc_temp = D.delv[zidx];
         const double area_tmp = D.arealg[zidx];
 
         // ---- CalcMonotonicQRegionForElems_kernel, lulesh.cu:3586-3724

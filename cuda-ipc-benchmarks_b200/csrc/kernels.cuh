@@ -56,9 +56,10 @@ constexpr int kNodeBlock = 128;  // threads per block, node kernels
 constexpr int kNodalMinBlocks = LULESH_NODAL_MINB;
 constexpr int kNodalFewMinBlocks = 16;
 // with the time increment's warp (small sets, one wave): registers for all
-// corner loads of a node at once
+// corner loads of a node at once beside its state (55; 16 B of spills at 8
+// blocks, and -s 30 16.6 us per cycle against 16.1, -s 60 42.7 against 41.7)
 #ifndef LULESH_NODAL_INCR_MINB
-#define LULESH_NODAL_INCR_MINB 8
+#define LULESH_NODAL_INCR_MINB 7
 #endif
 constexpr int kNodalIncrMinBlocks = LULESH_NODAL_INCR_MINB;
 // unstructured nodal kernel: four corners x 3 components in flight
@@ -245,10 +246,23 @@ __device__ __forceinline__ int chk_index(long long i, long long n, TimeCtl *T, i
 //
 // The cycle kernels may be launched with programmatic stream serialisation
 // (SetArgs::pdl): the next kernel's blocks are then scheduled while this
-// one's last wave drains.  Every kernel launched that way starts with
-// pdl_enter(): it waits until the previous grid has completed and its
-// writes are visible, before touching any memory, then lets its own
-// dependents be scheduled.  Without the attribute both pass at once.
+// one's last wave drains.  Every kernel launched that way calls pdl_enter()
+// before it reads what the previous grid may write, or writes anything: it
+// waits until that grid has completed and its writes are visible, then lets
+// its own dependents be scheduled.  Without the attribute both pass at once.
+//
+// What the previous kernel cannot write may be read before pdl_enter(), while
+// that kernel runs: the mesh's tables (node ids, corner slots, the EOS order)
+// in every set, and in sets of one wave, whose kernels are chains of loads, the
+// node update's own node and the EOS's element values.  Their last writer is
+// several grids back: every kernel waits before it lets its dependents in, so
+// all grids but the previous one have ended, and __ldcg takes their values
+// from L2.  Only kernels that always follow another kernel of the set do this:
+// nothing of the caller's can lie between.  Measured on B200, us per cycle:
+// -s 10 15.0 -> 14.1, -s 30 16.6 -> 16.1, -s 45 25.3 -> 24.2, -s 60 42.5 ->
+// 41.3, a scattered -s 40 mesh 38.3 -> 37.3, -s 100 182.7 -> 181.4.  The force
+// kernel's gathers done the same way (past L1) gained 3% at -s 10 and lost 2%
+// at -s 60.
 
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger()
