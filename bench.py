@@ -88,9 +88,8 @@ BUILD_BYTES_STEP = bytes_model.step_bytes(bytes_model.THIS_BUILD)
 LAUNCHES_PER_CYCLE = 5  # time_increment, force, nodal, kinematics, eos
 # FP64 flops per element of each phase (an FMA counts 2), measured with
 # ncu's smsp__sass_thread_inst_executed_op_{dfma,dadd,dmul}_pred_on counters
-# at -s 64 (profiles/cycle_kernels_s64_full.md; the EOS after its
-# unit-density form, profiles/eos_unit_density_s64.md); nodal is per node.
-FP64_FLOPS = {"force": 1427.0, "nodal": 50.2, "kinematics": 814.0, "eos": 359.9}
+# at -s 64 (profiles/cycle_kernels_s64_modes.md); nodal is per node.
+FP64_FLOPS = {"force": 820.0, "nodal": 48.0, "kinematics": 499.0, "eos": 335.5}
 
 
 def fp64_peak_tflops(dev):

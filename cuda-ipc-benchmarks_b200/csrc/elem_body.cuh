@@ -1,7 +1,7 @@
 // elem_body.cuh -- per-element bodies of the FP64 force and kinematics
-// kernels.  Each body receives the element's eight gathered node values and
-// does the rest: element loads, arithmetic, stores.  The launch that
-// gathers (kernels.cu) issues all 48 node loads before any arithmetic.
+// kernels, in the modes of elem_modal.cuh.  Each body receives the element's
+// eight gathered node values and does the rest: element loads, arithmetic,
+// stores.
 #pragma once
 
 #include <climits>

@@ -10,7 +10,8 @@
 //      tables, writes the time state of newly admitted jobs and re-captures
 //      the cycle graph (updating the executable graph in place);
 //   3. launches the cycle graph cycles_per_step times: every resident job,
-//      whatever its size, advances in the same five launches per cycle;
+//      whatever its size, advances in the same launches of a cycle (five, or
+//      four while the resident jobs are small);
 //   4. while those cycles run, admits queued jobs in arrival order while a
 //      slot is free and the job's device footprint fits under the cap
 //      (stream-ordered allocations from a memory pool, uploaded on a side
@@ -218,7 +219,7 @@ static int rebuild(lulesh_server *s)
         launch_eos(s->args(s->elem_b), s->n_elem, s->P, s->stream, kServerElemBlock);
         cudaGraph_t g = nullptr;
         SCHECK(cudaStreamEndCapture(s->stream, &g));
-        // same five kernels every time, only their grids and tables change:
+        // same kernels every time, only their grids and tables change:
         // update the executable graph in place, instantiate only if that fails
         if (s->exec) {
             cudaGraphExecUpdateResultInfo info{};

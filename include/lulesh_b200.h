@@ -150,8 +150,9 @@ int lulesh_create_batch(const lulesh_job *jobs, int njobs, int flags,
 int lulesh_create_from_mesh(const char *path, const lulesh_job *job,
                             int flags, int device, lulesh_set **out);
 
-/* Frees the arena, graphs and streams (the reference's teardown,
- * lulesh.cu:4904-4944, minus MPI). */
+/* Frees the graphs and streams and gives the arena back (the reference's
+ * teardown, lulesh.cu:4904-4944, minus MPI).  Up to 512 MB of device and 1 MB
+ * of pinned memory per device are kept for the next set. */
 int lulesh_destroy(lulesh_set *set);
 
 /* Bytes of device memory a set of these jobs would hold (the admission
@@ -177,7 +178,7 @@ int lulesh_lagrange_leapfrog(lulesh_set *set);
 int lulesh_step(lulesh_set *set, int ncycles);
 
 /* The whole run in one CUDA graph launch: a WHILE conditional node repeats
- * the cycle until every job of the set is done (the reference's host loop,
+ * four cycles until every job of the set is done (the reference's host loop,
  * lulesh.cu:4858-4873, moved onto the device).  max_cycles bounds the loop
  * (<= 0: 1,000,000 cycles); jobs still running when it stops are left as
  * they are.  Synchronous; returns like lulesh_run. */
@@ -185,7 +186,8 @@ int lulesh_run_graph(lulesh_set *set, long long max_cycles);
 
 /* Capture k consecutive cycles in one CUDA graph (default 1): lulesh_step(n)
  * then issues n / k launches of the k-cycle graph and n % k of the
- * one-cycle graph, so a whole batch run can be a single graph launch. */
+ * one-cycle graph, so a whole batch run can be a single graph launch.  At
+ * the default, a set that has made 256 cycles takes four at a time. */
 int lulesh_set_graph_cycles(lulesh_set *set, int k);
 
 /* Checkpoint of a set's whole state: every device array of every domain
