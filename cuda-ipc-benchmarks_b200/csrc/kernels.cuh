@@ -165,6 +165,7 @@ struct ByValue {
     TimeCtl *tc, *tn;
     int mat;
     int per;  // blocks per domain of this launch
+    long long stride;  // doubles from one domain's corner forces to the next's
     template <int BS, bool REVERSE>
     __device__ __forceinline__ int2 block() const
     {
@@ -194,6 +195,7 @@ inline ByValue<N> by_value(const SetArgs &a, int nblocks)
     w.tn = a.next ? a.next : a.tcs;
     w.mat = a.materialize;
     w.per = nblocks / N;
+    w.stride = N > 1 ? a.records[1].fx_elem - a.records[0].fx_elem : 0;
     return w;
 }
 

@@ -139,6 +139,22 @@ struct lulesh_set {
         return nodes <= lulesh::kInlineIncrementNodes;
     }
 
+    // 2x2x2 subdomains in the order of their ranks, their corner forces at
+    // equal distances (one arena of equal parts)
+    bool even_records() const
+    {
+        if (ndom != lulesh::kFewDomains || tp != 2) return false;
+        const lulesh::DomDev &a = hdoms[0];
+        const auto step = hdoms[1].fx_elem - a.fx_elem;
+        for (int d = 0; d < ndom; ++d) {
+            const lulesh::DomDev &b = hdoms[d];
+            if (b.fx_elem != a.fx_elem + d * step || b.fy_elem != a.fy_elem + d * step ||
+                b.fz_elem != a.fz_elem + d * step || b.col + 2 * b.row + 4 * b.plane != d)
+                return false;
+        }
+        return true;
+    }
+
     lulesh::SetArgs args(const int2 *blocks) const
     {
         lulesh::SetArgs a;
@@ -149,9 +165,8 @@ struct lulesh_set {
         a.pdl = pdl ? 1 : 0;
         // not for parts: their records are followed by proxies
         a.ndom = ndom;
-        a.records = nparts == 1 && njobs == 1 && (ndom == 1 || ndom == lulesh::kFewDomains)
-                        ? hdoms.data()
-                        : nullptr;
+        a.records = nparts == 1 && njobs == 1 && (ndom == 1 || even_records()) ? hdoms.data()
+                                                                               : nullptr;
         if (inline_increment()) a.next = dtc + njobs;
         a.corner32 = hcorner32.empty() ? nullptr : hcorner32.data();
         return a;
