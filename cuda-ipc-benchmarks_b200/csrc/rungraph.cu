@@ -70,7 +70,8 @@ int ensure_run_graph(lulesh_set *s)
                          "capture loop body");
         if (st == LULESH_OK) {
             int est = LULESH_OK;
-            for (int c = 0; c < kCyclesPerTurn && est == LULESH_OK; ++c) est = enqueue_cycle(s);
+            for (int c = 0; c < kCyclesPerTurn && est == LULESH_OK; ++c)
+                est = enqueue_cycle(s, c > 0);
             k_run_continue<<<1, 128, 0, s->stream>>>(h, s->dtc, s->njobs, s->run_ctl);
             cudaGraph_t captured = nullptr;
             const int cst = cuda_status(cudaStreamEndCapture(s->stream, &captured), "end capture");

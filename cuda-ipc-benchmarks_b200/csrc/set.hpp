@@ -176,10 +176,11 @@ struct lulesh_set {
 namespace lulesh {
 void set_error(const std::string &msg);
 int cuda_status(cudaError_t e, const char *what);
-// enqueue one cycle (no graph)
-int enqueue_cycle(lulesh_set *s);
+// enqueue one cycle (no graph); follows: straight after another one, with
+// nothing of the caller's between
+int enqueue_cycle(lulesh_set *s, bool follows = false);
 // the start of a cycle: the time increment (and a scattered mesh's packing)
-void launch_begin(lulesh_set *s, cudaStream_t st);
+void launch_begin(lulesh_set *s, cudaStream_t st, bool follows = false);
 // the FP64 force phase of every domain of the set
 void launch_force_fp64(lulesh_set *s, cudaStream_t st);
 // staged comm path of one cycle (comm.cu)

@@ -54,3 +54,21 @@ def test_lmesh(lulesh, tmp_path, nx):
             nudge(a, k), nudge(b, k)
         a.step(4), b.step(4)
         same(a, b)
+
+
+@pytest.mark.parametrize("nx,k", [(2, 2), (6, 3), (13, 4)])
+def test_packed_nodes_in_longer_graphs(lulesh, tmp_path, nx, k):
+    """Only the first of a graph's cycles packs the nodes anew."""
+    rng = np.random.default_rng(nx)
+    path = str(tmp_path / "m.lmesh")
+    lmesh.write(path, lmesh.renumber(lmesh.box(nx), rng.permutation((nx + 1) ** 3),
+                                     rng.permutation(nx ** 3)))
+    with lulesh.LuleshSet.from_mesh(path) as a, \
+            lulesh.LuleshSet.from_mesh(path, flags=lulesh.FLAG_MATERIALIZE) as b:
+        a.set_graph_cycles(k)
+        for part, n in enumerate((k, 2 * k + 1, 3 * k)):
+            a.step(n), b.step(n)
+            same(a, b)
+            nudge(a, part), nudge(b, part)
+        assert a.run_graph(9) == b.run_graph(9)
+        same(a, b)
