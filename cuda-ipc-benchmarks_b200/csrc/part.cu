@@ -428,6 +428,8 @@ int lulesh_part_phase(lulesh_set *s, int phase)
     SetArgs ae = s->args(s->elem_blocks), an = s->args(s->node_blocks),
             ag = s->args(s->ghost_blocks), as = s->args(s->sync_blocks);
     ae.pdl = an.pdl = ag.pdl = as.pdl = 0;
+    // the increment is a phase of its own here, also for one part's small set
+    ae.next = an.next = ag.next = as.next = nullptr;
     cudaStream_t st = s->stream;
     switch (phase) {
         case LULESH_PHASE_TIME_INCREMENT: launch_time_increment(s->dtc, s->njobs, s->P, st, false); break;
