@@ -136,4 +136,10 @@ void block_put(Block *b)
     if (prev >= 0 && prev != was.device) cudaSetDevice(prev);
 }
 
+void block_free(Block *b)
+{
+    if (b->p) free_block(*b);
+    *b = Block{};
+}
+
 }  // namespace lulesh

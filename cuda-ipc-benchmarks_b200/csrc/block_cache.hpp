@@ -9,9 +9,13 @@
 // kCachePinnedBytes of pinned memory, in at most kCacheBlocks blocks each.
 // Larger or later blocks go back to the driver at once, and so does all that is
 // kept when an allocation on the device fails.  A block is put back only when
-// no work on it is pending (lulesh_destroy has synchronised the set's
-// stream), so any stream may have it next.  Blocks of a context that
-// cudaDeviceReset has ended are recognised and forgotten.  Thread-safe.
+// no work on it can be pending, so any stream may have it next: the set's
+// stream has been synchronised, and nobody else knows the memory.  A set whose
+// pointers a caller holds, or whose kernels a caller's graph holds, may still
+// be at work on a stream the library does not know; its blocks go to the
+// driver, whose cudaFree waits for the device (lulesh_set::handed_out).
+// Blocks of a context that cudaDeviceReset has ended are recognised and
+// forgotten.  Thread-safe.
 #pragma once
 
 #include <cstddef>
@@ -36,5 +40,7 @@ struct Block {
 cudaError_t block_get(Block *b, size_t bytes, bool pinned = false);
 // Nothing may be pending on the block; *b is emptied.  Any current device.
 void block_put(Block *b);
+// The block to the driver, after all work on its device; *b is emptied.
+void block_free(Block *b);
 
 }  // namespace lulesh

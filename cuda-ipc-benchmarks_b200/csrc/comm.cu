@@ -580,6 +580,7 @@ static int check_rank(lulesh_set *s, int rank)
         set_error("comm: rank out of range");
         return LULESH_INVALID_ARG;
     }
+    s->handed_out = true;  // a caller may be capturing the exchange's kernels
     return LULESH_OK;
 }
 

@@ -423,6 +423,7 @@ int lulesh_part_phase(lulesh_set *s, int phase)
         set_error("lulesh_part_phase: FP64 structured sets with the fused exchange only");
         return LULESH_INVALID_ARG;
     }
+    s->handed_out = true;  // a caller may be capturing the phases
     // plain stream order between phases: the transport's copies and
     // collectives sit between them on the same stream
     SetArgs ae = s->args(s->elem_blocks), an = s->args(s->node_blocks),
@@ -459,6 +460,7 @@ int lulesh_part_phase(lulesh_set *s, int phase)
 int lulesh_part_dt_pack(lulesh_set *s, long long *dev_buf)
 {
     if (!s || !dev_buf) return LULESH_INVALID_ARG;
+    s->handed_out = true;
     k_dt_pack<<<1, 1, 0, s->stream>>>(s->dtc, dev_buf);
     return cuda_status(cudaGetLastError(), "dt pack");
 }
@@ -466,6 +468,7 @@ int lulesh_part_dt_pack(lulesh_set *s, long long *dev_buf)
 int lulesh_part_dt_unpack(lulesh_set *s, const long long *dev_buf)
 {
     if (!s || !dev_buf) return LULESH_INVALID_ARG;
+    s->handed_out = true;
     k_dt_unpack<<<1, 1, 0, s->stream>>>(s->dtc, dev_buf);
     return cuda_status(cudaGetLastError(), "dt unpack");
 }
@@ -571,6 +574,7 @@ int lulesh_wait_flag(lulesh_set *s, const unsigned int *dev_flag, unsigned int e
         set_error("lulesh_wait_flag: need a flag and 0 < timeout_ms <= 60000");
         return LULESH_INVALID_ARG;
     }
+    s->handed_out = true;
     const unsigned long long ns = (unsigned long long)(timeout_ms * 1e6);
     // one poll per ~1 us of sleep: the cap ends the wait even if the device
     // timer stood still

@@ -103,7 +103,7 @@ int build_tables(lulesh_set *s)
     size_t bytes = sizeof(int2) * (eb.size() + nb.size() + gb.size() + sb.size() + 1);
     if (s->elem_blocks) {  // rebuilding: the old tables may still be in use
         LCHECK(cudaStreamSynchronize(s->stream));
-        block_put(&s->tables_block);
+        s->give_back(&s->tables_block);
         s->elem_blocks = nullptr;
     }
     LCHECK(block_get(&s->tables_block, bytes));
@@ -804,6 +804,7 @@ int lulesh_create_part(const lulesh_job *job, int tp, int nparts, int part, int 
     s->njobs = 1;
     s->nparts = nparts;
     s->part = part;
+    s->handed_out = true;  // phases and messages are the caller's to capture
     s->jobs.push_back(*job);
     // this part's run of consecutive ranks (halo_part_of)
     std::vector<DomPlace> place;
@@ -897,7 +898,7 @@ int lulesh_destroy(lulesh_set *s)
     if (s->dcorner32) cudaFree(s->dcorner32);
     if (s->pack) cudaFree(s->pack);
     for (Block *b : {&s->tables_block, &s->ctl_block, &s->pinned_block, &s->arena_block})
-        block_put(b);
+        s->give_back(b);
     if (s->own_stream && s->stream) cudaStreamDestroy(s->stream);
     delete s;
     return LULESH_OK;
@@ -939,6 +940,7 @@ int lulesh_step(lulesh_set *s, int ncycles)
             set_error("lulesh_step: call lulesh_step(set, 0) before capturing the set's stream");
             return LULESH_INVALID_ARG;
         }
+        s->handed_out = true;
         for (int i = 0; i < ncycles; ++i) {
             const int est = enqueue_cycle(s);
             if (est != LULESH_OK) return est;
@@ -1186,6 +1188,7 @@ int lulesh_set_field(lulesh_set *s, int d, const char *name, const void *src, si
 int lulesh_domain_view_get(lulesh_set *s, int d, lulesh_domain_view *o)
 {
     if (!s || !o || d < 0 || d >= s->ndom) return LULESH_INVALID_ARG;
+    s->handed_out = true;
     const DomDev &D = s->hdoms[d];
     std::memset(o, 0, sizeof *o);
     o->numElem = D.numElem;

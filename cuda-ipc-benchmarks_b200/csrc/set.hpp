@@ -79,6 +79,10 @@ struct lulesh_set {
     size_t arena_bytes = 0;
     // what the device pointers above and htc_pinned lie in
     lulesh::Block arena_block, tables_block, ctl_block, pinned_block;
+    // a caller has had pointers to the arena, or may have kernels of the set in
+    // a graph of its own: work on the set's memory may run on streams unknown
+    // here
+    bool handed_out = false;
     void *pack = nullptr;  // nodePack and cornerPack of a scattered mesh
     size_t node_region_bytes = 0;
 
@@ -127,6 +131,15 @@ struct lulesh_set {
     long com_buf_doubles = 0;
     int max_plane = 0, max_edge = 0;
     int posted_msg = 0, posted_fields = 0, posted_do_recv = 1, posted_plane_only = 0;
+
+    // memory of the set that is no longer used
+    void give_back(lulesh::Block *b) const
+    {
+        if (handed_out)
+            lulesh::block_free(b);
+        else
+            lulesh::block_put(b);
+    }
 
     // The cycle's kernels make the time increment (kernels.cu) in place of a
     // launch of its own.

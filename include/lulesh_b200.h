@@ -152,7 +152,11 @@ int lulesh_create_from_mesh(const char *path, const lulesh_job *job,
 
 /* Frees the graphs and streams and gives the arena back (the reference's
  * teardown, lulesh.cu:4904-4944, minus MPI).  Up to 512 MB of device and 1 MB
- * of pinned memory per device are kept for the next set. */
+ * of pinned memory per device are kept for the next set.  The memory of a set
+ * whose device pointers were asked for (lulesh_domain_view_get), or whose
+ * kernels the caller may have captured (lulesh_step on a capturing stream,
+ * the phases of a part, the Comm calls), is not kept: it is freed, which waits
+ * for the work of every stream of the device. */
 int lulesh_destroy(lulesh_set *set);
 
 /* Bytes of device memory a set of these jobs would hold (the admission
