@@ -558,7 +558,7 @@ constexpr int kStepCycles = 4;
 constexpr long long kStepAfter = 256;
 static int cycles_per_launch(lulesh_set *s, int n)
 {
-    if (s->graph_cycles > 1) return s->graph_cycles;
+    if (s->graph_cycles > 1 || s->tuning) return s->graph_cycles;
     const bool lived = s->cycles_run >= kStepAfter;
     if (!lived) s->cycles_run += n;
     return lived ? kStepCycles : 1;

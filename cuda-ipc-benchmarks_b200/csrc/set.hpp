@@ -95,6 +95,9 @@ struct lulesh_set {
     cudaGraphExec_t exec_k = nullptr;
     bool graph_k_ready = false;
     long long cycles_run = 0;  // by one-cycle launches (cycles_per_launch, set.cu)
+    // graph_cycles taken at its word, whatever the set has run (lulesh_autotune,
+    // whose trials do not count as cycles of the set)
+    bool tuning = false;
     // whole-run graph: a WHILE conditional node around one cycle
     // (rungraph.cu); run_ctl[0] counts cycles, run_ctl[1] is the cap
     cudaGraph_t graph_run = nullptr;

@@ -86,6 +86,16 @@ struct Snapshot {
     }
 };
 
+// One cycle per launch means one while candidates are timed: a longer graph of
+// its own accord (cycles_per_launch, set.cu) would be captured and instantiated
+// inside the timed cycles of the candidate that reaches 256 cycles, and of every
+// later one.
+struct Tuning {
+    lulesh_set *s;
+    explicit Tuning(lulesh_set *set) : s(set) { s->tuning = true; }
+    ~Tuning() { s->tuning = false; }
+};
+
 // Device time per cycle of `cycles` cycles of the current shape, started
 // from the saved state (after an untimed warm-up that builds the graphs).
 static int time_shape(lulesh_set *s, Snapshot &snap, int cycles, cudaEvent_t e0, cudaEvent_t e1,
@@ -141,6 +151,7 @@ int lulesh_autotune(lulesh_set *s, int trial_cycles, int rounds, lulesh_tuning *
     Snapshot snap;
     int st = snap.save(s);
     if (st != LULESH_OK) return st;
+    const Tuning tuning(s);
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     TCHECK(cudaEventCreate(&e0));
     TCHECK(cudaEventCreate(&e1));
