@@ -1,6 +1,8 @@
 // block_cache.cu -- see block_cache.hpp.
 #include "block_cache.hpp"
 
+#include <cuda.h>
+
 #include <map>
 #include <mutex>
 #include <vector>
@@ -9,27 +11,23 @@ namespace lulesh {
 
 namespace {
 
-// A mark in the module's own device memory.  A device reset loads the module
-// again with 0 here, so what carries an older mark belongs to an ended context.
-__device__ unsigned long long g_mark;
-
 struct Kept {
     std::vector<Block> blocks;
     size_t bytes = 0;
 };
 
 struct Store {
-    unsigned long long mark = 0;  // as written to the device's g_mark, 0 none
-    Kept kept[2];                 // device memory, pinned memory
+    Kept kept[2];  // device memory, pinned memory
 };
 
 std::mutex g_mu;
-unsigned long long g_marks = 0;
 
-// by device; never destroyed, as the driver may be gone at exit
-std::map<int, Store> &stores()
+// by context.  What is kept of a context that has ended (cudaDeviceReset) went
+// with it: its entry is never looked up again and holds a few host bytes.  Never
+// destroyed, as the driver may be gone at exit.
+std::map<unsigned long long, Store> &stores()
 {
-    static auto *s = new std::map<int, Store>;
+    static auto *s = new std::map<unsigned long long, Store>;
     return *s;
 }
 
@@ -39,29 +37,39 @@ void free_block(const Block &b)
     if (e != cudaSuccess) (void)cudaGetLastError();
 }
 
-// the mark on the current device; 0 also when it cannot be read
-unsigned long long read_mark()
+// The id of the current context, unique for the life of the process: a reset
+// device has a new one.  0 where it cannot be had, and nothing is kept then.  No
+// stream is touched, so that a caller may be capturing any of its own.
+unsigned long long context_id()
 {
-    unsigned long long mark = 0;
-    if (cudaMemcpyFromSymbolAsync(&mark, g_mark, sizeof mark, 0, cudaMemcpyDeviceToHost,
-                                  cudaStreamPerThread) != cudaSuccess ||
-        cudaStreamSynchronize(cudaStreamPerThread) != cudaSuccess) {
-        (void)cudaGetLastError();
-        return 0;
+    using GetCurrent = CUresult (*)(CUcontext *);
+    using GetId = CUresult (*)(CUcontext, unsigned long long *);
+    struct Entry {
+        GetCurrent current = nullptr;
+        GetId id = nullptr;
+        Entry()
+        {
+            void *f = nullptr;
+            cudaDriverEntryPointQueryResult q;
+            if (cudaGetDriverEntryPoint("cuCtxGetCurrent", &f, cudaEnableDefault, &q) ==
+                    cudaSuccess && q == cudaDriverEntryPointSuccess)
+                current = reinterpret_cast<GetCurrent>(f);
+            if (cudaGetDriverEntryPoint("cuCtxGetId", &f, cudaEnableDefault, &q) == cudaSuccess &&
+                q == cudaDriverEntryPointSuccess)
+                id = reinterpret_cast<GetId>(f);
+            (void)cudaGetLastError();
+        }
+    };
+    static const Entry entry;
+    if (!entry.current || !entry.id) return 0;
+    for (int attempt = 0; attempt < 2; ++attempt) {
+        CUcontext c = nullptr;
+        unsigned long long id = 0;
+        if (entry.current(&c) == CUDA_SUCCESS && c && entry.id(c, &id) == CUDA_SUCCESS) return id;
+        // none yet on this thread, or ended by a reset: the runtime's own
+        if (attempt == 0 && cudaFree(nullptr) != cudaSuccess) (void)cudaGetLastError();
     }
-    return mark;
-}
-
-unsigned long long write_mark()
-{
-    const unsigned long long mark = ++g_marks;
-    if (cudaMemcpyToSymbolAsync(g_mark, &mark, sizeof mark, 0, cudaMemcpyHostToDevice,
-                                cudaStreamPerThread) != cudaSuccess ||
-        cudaStreamSynchronize(cudaStreamPerThread) != cudaSuccess) {
-        (void)cudaGetLastError();
-        return 0;
-    }
-    return mark;
+    return 0;
 }
 
 void release(Kept &k)
@@ -77,12 +85,12 @@ cudaError_t block_get(Block *b, size_t bytes, bool pinned)
     Block n;
     cudaError_t e = cudaGetDevice(&n.device);
     if (e != cudaSuccess) return e;
+    n.bytes = bytes;
+    n.context = context_id();
+    n.pinned = pinned;
     std::lock_guard<std::mutex> lock(g_mu);
-    Store &s = stores()[n.device];
-    if (s.mark == 0 || read_mark() != s.mark) {
-        s = Store{};  // nothing kept, or gone with its context
-        s.mark = write_mark();
-    }
+    Store none;
+    Store &s = n.context ? stores()[n.context] : none;
     Kept &k = s.kept[pinned];
     // the smallest block that is large enough and not twice too large
     size_t best = k.blocks.size();
@@ -96,9 +104,6 @@ cudaError_t block_get(Block *b, size_t bytes, bool pinned)
         k.blocks.erase(k.blocks.begin() + (long)best);
         return cudaSuccess;
     }
-    n.bytes = bytes;
-    n.mark = s.mark;
-    n.pinned = pinned;
     for (int attempt = 0; attempt < 2; ++attempt) {
         e = pinned ? cudaMallocHost(&n.p, bytes) : cudaMalloc(&n.p, bytes);
         if (e != cudaErrorMemoryAllocation || (s.kept[0].blocks.empty() && s.kept[1].blocks.empty()))
@@ -120,13 +125,11 @@ void block_put(Block *b)
     cudaGetDevice(&prev);
     if (prev != was.device) cudaSetDevice(was.device);
     bool keep = false;
-    {
+    if (was.context != 0 && context_id() == was.context) {
         std::lock_guard<std::mutex> lock(g_mu);
-        Store &s = stores()[was.device];
-        Kept &k = s.kept[was.pinned];
-        keep = was.mark != 0 && was.mark == s.mark && k.blocks.size() < kCacheBlocks &&
-               k.bytes + was.bytes <= (was.pinned ? kCachePinnedBytes : kCacheDeviceBytes) &&
-               read_mark() == was.mark;
+        Kept &k = stores()[was.context].kept[was.pinned];
+        keep = k.blocks.size() < kCacheBlocks &&
+               k.bytes + was.bytes <= (was.pinned ? kCachePinnedBytes : kCacheDeviceBytes);
         if (keep) {
             k.blocks.push_back(was);
             k.bytes += was.bytes;

@@ -14,8 +14,8 @@
 // pointers a caller holds, or whose kernels a caller's graph holds, may still
 // be at work on a stream the library does not know; its blocks go to the
 // driver, whose cudaFree waits for the device (lulesh_set::handed_out).
-// Blocks of a context that cudaDeviceReset has ended are recognised and
-// forgotten.  Thread-safe.
+// Blocks are kept by context, and those of a context that cudaDeviceReset has
+// ended are never looked at again.  Thread-safe.
 #pragma once
 
 #include <cstddef>
@@ -30,8 +30,8 @@ constexpr size_t kCacheBlocks = 64;
 
 struct Block {
     void *p = nullptr;
-    size_t bytes = 0;              // of the block, at least what was asked for
-    unsigned long long mark = 0;   // of the context it lives in, 0 not known
+    size_t bytes = 0;                // of the block, at least what was asked for
+    unsigned long long context = 0;  // id of the context it lives in, 0 not known
     int device = 0;
     bool pinned = false;
 };
