@@ -5,7 +5,10 @@
 
 #include <map>
 #include <mutex>
+#include <utility>
 #include <vector>
+
+#include "lulesh_b200.h"
 
 namespace lulesh {
 
@@ -72,12 +75,6 @@ unsigned long long context_id()
     return 0;
 }
 
-void release(Kept &k)
-{
-    for (const Block &b : k.blocks) free_block(b);
-    k = Kept{};
-}
-
 }  // namespace
 
 cudaError_t block_get(Block *b, size_t bytes, bool pinned)
@@ -88,30 +85,23 @@ cudaError_t block_get(Block *b, size_t bytes, bool pinned)
     n.bytes = bytes;
     n.context = context_id();
     n.pinned = pinned;
-    std::lock_guard<std::mutex> lock(g_mu);
-    Store none;
-    Store &s = n.context ? stores()[n.context] : none;
-    Kept &k = s.kept[pinned];
-    // the smallest block that is large enough and not twice too large
-    size_t best = k.blocks.size();
-    for (size_t i = 0; i < k.blocks.size(); ++i)
-        if (k.blocks[i].bytes >= bytes && k.blocks[i].bytes <= 2 * bytes + 4096 &&
-            (best == k.blocks.size() || k.blocks[i].bytes < k.blocks[best].bytes))
-            best = i;
-    if (best < k.blocks.size()) {
-        *b = k.blocks[best];
-        k.bytes -= b->bytes;
-        k.blocks.erase(k.blocks.begin() + (long)best);
-        return cudaSuccess;
+    if (n.context != 0) {
+        std::lock_guard<std::mutex> lock(g_mu);
+        Kept &k = stores()[n.context].kept[pinned];
+        // the smallest block that is large enough and not twice too large
+        size_t best = k.blocks.size();
+        for (size_t i = 0; i < k.blocks.size(); ++i)
+            if (k.blocks[i].bytes >= bytes && k.blocks[i].bytes <= 2 * bytes + 4096 &&
+                (best == k.blocks.size() || k.blocks[i].bytes < k.blocks[best].bytes))
+                best = i;
+        if (best < k.blocks.size()) {
+            *b = k.blocks[best];
+            k.bytes -= b->bytes;
+            k.blocks.erase(k.blocks.begin() + (long)best);
+            return cudaSuccess;
+        }
     }
-    for (int attempt = 0; attempt < 2; ++attempt) {
-        e = pinned ? cudaMallocHost(&n.p, bytes) : cudaMalloc(&n.p, bytes);
-        if (e != cudaErrorMemoryAllocation || (s.kept[0].blocks.empty() && s.kept[1].blocks.empty()))
-            break;
-        (void)cudaGetLastError();
-        release(s.kept[0]);
-        release(s.kept[1]);
-    }
+    e = retry_trimmed([&] { return pinned ? cudaMallocHost(&n.p, bytes) : cudaMalloc(&n.p, bytes); });
     if (e == cudaSuccess) *b = n;
     return e;
 }
@@ -145,4 +135,24 @@ void block_free(Block *b)
     *b = Block{};
 }
 
+bool block_trim()
+{
+    const unsigned long long context = context_id();
+    Store was;
+    {
+        std::lock_guard<std::mutex> lock(g_mu);
+        const auto it = stores().find(context);
+        if (it != stores().end()) std::swap(was, it->second);
+    }
+    for (const Kept &k : was.kept)
+        for (const Block &b : k.blocks) free_block(b);
+    return !was.kept[0].blocks.empty() || !was.kept[1].blocks.empty();
+}
+
 }  // namespace lulesh
+
+extern "C" int lulesh_release_memory(void)
+{
+    lulesh::block_trim();
+    return LULESH_OK;
+}

@@ -8,7 +8,8 @@
 // Kept, per device: at most kCacheDeviceBytes of device memory and
 // kCachePinnedBytes of pinned memory, in at most kCacheBlocks blocks each.
 // Larger or later blocks go back to the driver at once, and so does all that is
-// kept when an allocation on the device fails.  A block is put back only when
+// kept when an allocation of the library's on the device fails (retry_trimmed)
+// or the program asks (lulesh_release_memory).  A block is put back only when
 // no work on it can be pending, so any stream may have it next: the set's
 // stream has been synchronised, and nobody else knows the memory.  A set whose
 // pointers a caller holds, or whose kernels a caller's graph holds, may still
@@ -42,5 +43,23 @@ cudaError_t block_get(Block *b, size_t bytes, bool pinned = false);
 void block_put(Block *b);
 // The block to the driver, after all work on its device; *b is emptied.
 void block_free(Block *b);
+// All that is kept in the current context to the driver; false if nothing was.
+bool block_trim();
+
+// alloc(), and once more without the kept blocks where it was short of memory
+template <class Alloc>
+inline cudaError_t retry_trimmed(const Alloc &alloc)
+{
+    const cudaError_t e = alloc();
+    if (e != cudaErrorMemoryAllocation || !block_trim()) return e;
+    (void)cudaGetLastError();
+    return alloc();
+}
+
+template <class T>
+inline cudaError_t device_malloc(T **p, size_t bytes)
+{
+    return retry_trimmed([&] { return cudaMalloc(reinterpret_cast<void **>(p), bytes); });
+}
 
 }  // namespace lulesh

@@ -344,9 +344,9 @@ static int build_msgs(lulesh_set *s, int rank, int xferFields, bool doSend, bool
     out->nmsg = (int)msgs.size();
     out->nblocks = (int)blocks.size();
     if (msgs.empty()) return LULESH_OK;
-    int st = cuda_status(cudaMalloc(&out->msgs, sizeof(Msg) * msgs.size()), "comm table");
+    int st = cuda_status(device_malloc(&out->msgs, sizeof(Msg) * msgs.size()), "comm table");
     if (st != LULESH_OK) return st;
-    st = cuda_status(cudaMalloc(&out->blocks, sizeof(int2) * blocks.size()), "comm table");
+    st = cuda_status(device_malloc(&out->blocks, sizeof(int2) * blocks.size()), "comm table");
     if (st != LULESH_OK) return st;
     st = cuda_status(cudaMemcpy(out->msgs, msgs.data(), sizeof(Msg) * msgs.size(),
                                 cudaMemcpyHostToDevice),
@@ -400,7 +400,7 @@ static int node_blocks_for(lulesh_set *s, int rank, int2 **blocks, int *n)
         MsgTable t;
         t.nblocks = (int)b.size();
         if (!b.empty()) {
-            int st = cuda_status(cudaMalloc(&t.blocks, sizeof(int2) * b.size()), "comm table");
+            int st = cuda_status(device_malloc(&t.blocks, sizeof(int2) * b.size()), "comm table");
             if (st != LULESH_OK) return st;
             st = cuda_status(cudaMemcpy(t.blocks, b.data(), sizeof(int2) * b.size(),
                                         cudaMemcpyHostToDevice),
@@ -542,7 +542,7 @@ int comm_monoq_impl(lulesh_set *s, int rank, int gate)
         }
         if (gb.empty()) return LULESH_OK;
         int2 *tmp = nullptr;
-        int st = cuda_status(cudaMalloc(&tmp, sizeof(int2) * gb.size()), "monoq table");
+        int st = cuda_status(device_malloc(&tmp, sizeof(int2) * gb.size()), "monoq table");
         if (st != LULESH_OK) return st;
         cudaMemcpy(tmp, gb.data(), sizeof(int2) * gb.size(), cudaMemcpyHostToDevice);
         k_unpack_monoq<<<(int)gb.size(), kElemBlock, 0, s->stream>>>(s->ddoms, s->dtc, tmp, gate);

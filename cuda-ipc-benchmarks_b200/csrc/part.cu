@@ -126,7 +126,7 @@ int upload_table(const std::vector<double *> &ptrs, lulesh_set::HaloTable *t)
 {
     t->n = (long long)ptrs.size();
     if (ptrs.empty()) return LULESH_OK;
-    int st = cuda_status(cudaMalloc(&t->ptrs, sizeof(double *) * ptrs.size()), "halo table");
+    int st = cuda_status(device_malloc(&t->ptrs, sizeof(double *) * ptrs.size()), "halo table");
     if (st != LULESH_OK) return st;
     return cuda_status(cudaMemcpy(t->ptrs, ptrs.data(), sizeof(double *) * ptrs.size(),
                                   cudaMemcpyHostToDevice),
@@ -263,7 +263,7 @@ int part_build(lulesh_set *s)
     const DomSizes z = sizes_of(j.nx, j.numReg, 0);
     const size_t per = proxy_bytes(z);
     if (!s->proxy_rank.empty()) {
-        int st = cuda_status(cudaMalloc(&s->proxy_arena, per * s->proxy_rank.size()),
+        int st = cuda_status(device_malloc(&s->proxy_arena, per * s->proxy_rank.size()),
                              "proxy arena");
         if (st != LULESH_OK) return st;
         st = cuda_status(cudaMemsetAsync(s->proxy_arena, 0, per * s->proxy_rank.size(), s->stream),
@@ -341,7 +341,7 @@ int part_build(lulesh_set *s)
     // can be exported to the peers' processes with cudaIpcGetMemHandle)
     const MailboxLayout L = mailbox_layout(j.nx, tp, s->nparts, s->part);
     s->mailbox_bytes = L.bytes;
-    int st = cuda_status(cudaMalloc(&s->mailbox, L.bytes), "mailbox");
+    int st = cuda_status(device_malloc(&s->mailbox, L.bytes), "mailbox");
     if (st != LULESH_OK) return st;
     st = cuda_status(cudaMemsetAsync(s->mailbox, 0, L.bytes, s->stream), "mailbox");
     if (st != LULESH_OK) return st;

@@ -180,7 +180,9 @@ static int rebuild(lulesh_server *s)
     if (need > s->blocks_cap) {
         if (s->dblocks) SCHECK(cudaFreeAsync(s->dblocks, s->stream));
         size_t cap = need + need / 2 + 1024;
-        SCHECK(cudaMallocAsync(&s->dblocks, sizeof(int2) * cap, s->stream));
+        SCHECK(retry_trimmed([&] {
+            return cudaMallocAsync(&s->dblocks, sizeof(int2) * cap, s->stream);
+        }));
         s->blocks_cap = cap;
     }
     s->node_b = s->dblocks;
@@ -269,12 +271,12 @@ int lulesh_server_create(const lulesh_server_config *cfg, lulesh_server **out)
     unsigned long long keep = ~0ull;  // keep freed job memory cached in the pool
     cudaMemPoolSetAttribute(s->pool, cudaMemPoolAttrReleaseThreshold, &keep);
     const int M = cfg->max_jobs;
-    if ((st = cuda_status(cudaMalloc(&s->dtc, sizeof(TimeCtl) * 2 * M), "slots"))) return fail(st);
+    if ((st = cuda_status(device_malloc(&s->dtc, sizeof(TimeCtl) * 2 * M), "slots"))) return fail(st);
     if ((st = cuda_status(cudaMallocHost(&s->htc, sizeof(TimeCtl) * M), "slots"))) return fail(st);
-    if ((st = cuda_status(cudaMalloc(&s->denergy, sizeof(double) * M), "slots"))) return fail(st);
+    if ((st = cuda_status(device_malloc(&s->denergy, sizeof(double) * M), "slots"))) return fail(st);
     if ((st = cuda_status(cudaMallocHost(&s->henergy, sizeof(double) * M), "slots")))
         return fail(st);
-    if ((st = cuda_status(cudaMalloc(&s->ddoms, sizeof(DomDev) * M), "slots"))) return fail(st);
+    if ((st = cuda_status(device_malloc(&s->ddoms, sizeof(DomDev) * M), "slots"))) return fail(st);
     if ((st = cuda_status(cudaEventCreateWithFlags(&s->step_done, cudaEventDisableTiming), "event")))
         return fail(st);
     // every slot starts empty: done, so the time-increment kernel skips it
@@ -410,7 +412,7 @@ int lulesh_server_step(lulesh_server *s, int *n_active, int *n_queued)
         if (s->free_slots.empty() || s->used_bytes + j->bytes > s->cfg.hbm_cap_bytes) break;
         const int slot = s->free_slots.back();
         void *mem = nullptr;
-        SCHECK(cudaMallocAsync(&mem, j->bytes, s->upload));
+        SCHECK(retry_trimmed([&] { return cudaMallocAsync(&mem, j->bytes, s->upload); }));
         Carver cv{static_cast<char *>(mem)};
         int st = upload_domain(*j->host, slot, 0, false, cv, s->upload, &j->dom, nullptr);
         if (st != LULESH_OK) {

@@ -169,7 +169,7 @@ static int pack_scattered_mesh(lulesh_set *s, const HostDomain &h, DomDev &D)
         gather_sectors(h) < LULESH_PACK_SECTORS)
         return LULESH_OK;
     const size_t N = D.numNode, nodes = 8 * N, corners = 32 * (size_t)D.Ep;  // doubles
-    if (cudaMalloc(&s->pack, sizeof(double) * (nodes + corners) + sizeof(int) * 8 * N) !=
+    if (device_malloc(&s->pack, sizeof(double) * (nodes + corners) + sizeof(int) * 8 * N) !=
         cudaSuccess) {
         (void)cudaGetLastError();  // not enough memory for both: run from the lists
         s->pack = nullptr;
@@ -235,7 +235,7 @@ static int create_common(lulesh_set *s, const std::vector<DomPlace> &place, int 
     s->arena_bytes = total;
     LCHECK(block_get(&s->arena_block, total));
     s->arena = s->arena_block.p;
-    if (mixed) LCHECK(cudaMalloc(&s->dcorner32, sizeof(CornerF32) * s->ndom));
+    if (mixed) LCHECK(device_malloc(&s->dcorner32, sizeof(CornerF32) * s->ndom));
 
     // subdomain sets: every domain's x..zd side by side at the start of the
     // arena (the node region), so one L2 window can cover them all; the

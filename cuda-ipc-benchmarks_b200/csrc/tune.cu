@@ -67,8 +67,8 @@ struct Snapshot {
     }
     int save(const lulesh_set *s)
     {
-        TCHECK(cudaMalloc(&arena, s->arena_bytes));
-        TCHECK(cudaMalloc(&tc, sizeof(TimeCtl) * s->njobs));
+        TCHECK(device_malloc(&arena, s->arena_bytes));
+        TCHECK(device_malloc(&tc, sizeof(TimeCtl) * s->njobs));
         return restore_into(s, true);
     }
     int restore(const lulesh_set *s) { return restore_into(s, false); }

@@ -61,7 +61,8 @@ INT_FIELDS = {
 # every symbol include/lulesh_b200.h declares
 EXPORTED = [
     "lulesh_create", "lulesh_create_batch", "lulesh_create_from_mesh", "lulesh_destroy",
-    "lulesh_footprint_bytes", "lulesh_set_stream", "lulesh_lagrange_leapfrog",
+    "lulesh_footprint_bytes", "lulesh_release_memory", "lulesh_set_stream",
+    "lulesh_lagrange_leapfrog",
     "lulesh_step", "lulesh_run", "lulesh_host_cycle", "lulesh_sync",
     "lulesh_num_jobs", "lulesh_num_domains", "lulesh_job_state_get",
     "lulesh_origin_energy", "lulesh_symmetry", "lulesh_field_bytes",
@@ -164,6 +165,7 @@ def load_library(path: str | None = None) -> ctypes.CDLL:
         "lulesh_create_from_mesh": (ip, [ctypes.c_char_p, ctypes.POINTER(Job), ip, ip,
                                          ctypes.POINTER(vp)]),
         "lulesh_destroy": (ip, [vp]),
+        "lulesh_release_memory": (ip, []),
         "lulesh_footprint_bytes": (ctypes.c_size_t, [ctypes.POINTER(Job), ip, ip]),
         "lulesh_set_stream": (ip, [vp, vp]),
         "lulesh_lagrange_leapfrog": (ip, [vp]),
@@ -266,6 +268,12 @@ def footprint_bytes(jobs: list[JobSpec], tp: int = 1) -> int:
     lib = load_library()
     arr = (Job * len(jobs))(*[j.c() for j in jobs])
     return int(lib.lulesh_footprint_bytes(arr, len(jobs), tp))
+
+
+def release_memory() -> None:
+    """Memory kept from closed sets on the current device back to the driver."""
+    lib = load_library()
+    _check(lib, lib.lulesh_release_memory(), "lulesh_release_memory")
 
 
 class LuleshSet:

@@ -159,6 +159,11 @@ int lulesh_create_from_mesh(const char *path, const lulesh_job *job,
  * for the work of every stream of the device. */
 int lulesh_destroy(lulesh_set *set);
 
+/* Gives the memory kept from closed sets on the current device back to the
+ * driver, for another allocator of the program's.  The library's own
+ * allocations do so by themselves where memory is short. */
+int lulesh_release_memory(void);
+
 /* Bytes of device memory a set of these jobs would hold (the admission
  * model of the serving loop). */
 size_t lulesh_footprint_bytes(const lulesh_job *jobs, int njobs, int tp);
