@@ -88,10 +88,11 @@ cudaError_t block_get(Block *b, size_t bytes, bool pinned)
     if (n.context != 0) {
         std::lock_guard<std::mutex> lock(g_mu);
         Kept &k = stores()[n.context].kept[pinned];
-        // the smallest block that is large enough and not twice too large
+        // the smallest block that is large enough and not an eighth too large:
+        // what a set holds stays what lulesh_footprint_bytes says, nearly
         size_t best = k.blocks.size();
         for (size_t i = 0; i < k.blocks.size(); ++i)
-            if (k.blocks[i].bytes >= bytes && k.blocks[i].bytes <= 2 * bytes + 4096 &&
+            if (k.blocks[i].bytes >= bytes && k.blocks[i].bytes <= bytes + bytes / 8 + 4096 &&
                 (best == k.blocks.size() || k.blocks[i].bytes < k.blocks[best].bytes))
                 best = i;
         if (best < k.blocks.size()) {

@@ -744,9 +744,9 @@ size_t lulesh_footprint_bytes(const lulesh_job *jobs, int njobs, int tp)
         const size_t E = (size_t)jobs[j].nx * jobs[j].nx * jobs[j].nx;
         const size_t N = (size_t)(jobs[j].nx + 1) * (jobs[j].nx + 1) * (jobs[j].nx + 1);
         total += tp * tp * tp * (8 * (E / kElemBlock + N / kNodeBlock + 2) + sizeof(DomDev)) +
-                 sizeof(TimeCtl);
+                 2 * sizeof(TimeCtl);
     }
-    return total;
+    return total + 2 * sizeof(unsigned long long);  // the run graph's counters
 }
 
 int lulesh_create(const lulesh_job *job, int tp, int flags, int device, lulesh_set **out)

@@ -106,6 +106,11 @@ int main()
     block_put(&a);
     block_put(&b);
     CHECK(g_used[0] == 300 * MB);
+    // a smaller set gets it only where it is not an eighth too large
+    CHECK(block_get(&a, 250 * MB) == cudaSuccess && a.p != p);
+    block_free(&a);
+    CHECK(block_get(&a, 270 * MB) == cudaSuccess && a.p == p && a.bytes == 300 * MB);
+    block_put(&a);
     // block_free keeps nothing
     CHECK(block_get(&a, 300 * MB) == cudaSuccess && a.p == p);
     block_free(&a);
