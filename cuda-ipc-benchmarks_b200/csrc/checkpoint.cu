@@ -80,6 +80,8 @@ int lulesh_checkpoint_save(lulesh_set *s, void *buf, size_t bytes)
         set_error("lulesh_checkpoint_save: buffer smaller than lulesh_checkpoint_bytes");
         return LULESH_INVALID_ARG;
     }
+    const int st = show_corners(s);
+    if (st != LULESH_OK) return st;
     const CkptHeader h = header_of(s);
     char *p = static_cast<char *>(buf);
     std::memcpy(p, &h, sizeof h);
@@ -122,6 +124,8 @@ int lulesh_checkpoint_load(lulesh_set *s, const void *buf, size_t bytes)
                            s->stream));
     CCHECK(cudaMemcpyAsync(s->dtc, p + sizeof h + s->arena_bytes, h.tc_bytes,
                            cudaMemcpyHostToDevice, s->stream));
+    const int st = hide_corners(s);
+    if (st != LULESH_OK) return st;
     CCHECK(cudaStreamSynchronize(s->stream));
     return LULESH_OK;
 }

@@ -243,6 +243,37 @@ void launch_begin_packed(const SetArgs &a, int nblocks, Params P, cudaStream_t s
     launch_k(k_begin_packed, nblocks, kNodeBlock, s, a.pdl != 0, by_value<1>(a, nblocks), P);
 }
 
+// The fourth value of a corner's sector: kNewCorner where fx_elem, fy_elem and
+// fz_elem do not have the corner force yet, else 0.
+constexpr double kNewCorner = 1.0;
+
+// An element's packed corner forces to the arrays that callers read
+__device__ __forceinline__ void show_element(const DomDev &D, int e)
+{
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        double *p = D.cornerPack + 4 * (8 * (size_t)e + k);
+        double fx, fy, fz, state;
+        ld4(p, fx, fy, fz, state);
+        if (state != kNewCorner) continue;
+        D.fx_elem[e + D.Ep * k] = fx;
+        D.fy_elem[e + D.Ep * k] = fy;
+        D.fz_elem[e + D.Ep * k] = fz;
+        p[3] = 0.0;
+    }
+}
+
+__global__ void __launch_bounds__(kElemBlock) k_show_corners(const __grid_constant__ OneDomain w)
+{
+    const int e = blockIdx.x * kElemBlock + threadIdx.x;
+    if (e < w.D[0].numElem) show_element(w.D[0], e);
+}
+
+void launch_show_corners(const SetArgs &a, int nblocks, cudaStream_t s)
+{
+    launch_k(k_show_corners, nblocks, kElemBlock, s, /*pdl=*/false, by_value<1>(a, nblocks));
+}
+
 // ---------------------------------------------------------------------------
 // force: CalcVolumeForceForElems_kernel, lulesh.cu:2080-2259
 
@@ -259,7 +290,7 @@ void launch_begin_packed(const SetArgs &a, int nblocks, Params P, cudaStream_t s
 // and 312 against 272 us at -s 160.
 template <bool HG, Mesh M, bool TABLE>
 __device__ __forceinline__ void force_one(const DomDev &D, bool active, TimeCtl &E, const Params &P,
-                                          int elem, int (&n)[8])
+                                          int elem, int (&n)[8], bool show)
 {
 #pragma unroll
     for (int i = 0; i < 8; ++i) n[i] = chk_index(n[i], D.numNode, &E, kChkNode);
@@ -286,7 +317,11 @@ __device__ __forceinline__ void force_one(const DomDev &D, bool active, TimeCtl 
 #pragma unroll
         for (int i = 0; i < 8; ++i) zn[i] = D.z[n[i]];
     }
-    if (!TABLE && !active) return;
+    if (!TABLE && !active) {
+        // the graph's last cycle with work was an earlier one
+        if (M == Mesh::kPacked && show) show_element(D, elem);
+        return;
+    }
     double fx[8], fy[8];  // held for cornerPack, whose corners take all three
     force_modal<HG>(
         xn, yn, zn, D.volo[elem], D.v[elem], D.p[elem], D.q[elem], D.ss[elem], D.elemMass[elem],
@@ -302,11 +337,11 @@ __device__ __forceinline__ void force_one(const DomDev &D, bool active, TimeCtl 
                 for (int k = 0; k < 8; ++k) {
                     if (c == 0) fx[k] = f[k];
                     if (c == 1) fy[k] = f[k];
-                    if (c == 2) st4(p + 4 * k, fx[k], fy[k], f[k], 0.0);
+                    if (c == 2) st4(p + 4 * k, fx[k], fy[k], f[k], show ? 0.0 : kNewCorner);
                 }
-            } else {
-                CornerStore{D.fx_elem, D.fy_elem, D.fz_elem, elem, D.Ep}(c, f);
             }
+            if (M != Mesh::kPacked || show)
+                CornerStore{D.fx_elem, D.fy_elem, D.fz_elem, elem, D.Ep}(c, f);
         },
         [&] { atomicMin(&E.bad_vol, elem); });
 }
@@ -330,7 +365,7 @@ __global__ void __launch_bounds__(BS, min_blocks(kForceMinBlocks, BS))
     if (W::kTable && !active) return;
     if (elem >= D.numElem) return;
     if (M == Mesh::kBox) elem_nodes<false>(D, elem, n);
-    force_one<HG, M, W::kTable>(D, active, w.next(D), P, elem, n);
+    force_one<HG, M, W::kTable>(D, active, w.next(D), P, elem, n, w.show());
 }
 
 template <int BS, Mesh M, class W>

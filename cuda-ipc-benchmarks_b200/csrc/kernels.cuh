@@ -120,6 +120,7 @@ struct SetArgs {
     // k_time_increment launch
     TimeCtl *next = nullptr;
     const CornerF32 *corner32 = nullptr;  // a mixed set's first domain (host side only)
+    int show = 0;  // a scattered mesh's corner forces to fx_elem ... too (force)
 };
 
 // Where a block of a cycle kernel works: its domain's record, the time state
@@ -153,6 +154,7 @@ struct ManyDomains {
     __device__ __forceinline__ bool increments() const { return a.next != nullptr; }
     __device__ __forceinline__ const DomDev *doms() const { return a.doms; }
     __device__ __forceinline__ int materialize() const { return a.materialize; }
+    __device__ __forceinline__ bool show() const { return true; }
     // The node block table is already laid out last to first.  A job that is
     // done skips its gathers: the time state is read first.
     static constexpr bool kTable = true;
@@ -163,7 +165,7 @@ template <int N>
 struct ByValue {
     DomDev D[N];
     TimeCtl *tc, *tn;
-    int mat;
+    int mat, shows;
     int per;  // blocks per domain of this launch
     long long stride;  // doubles from one domain's corner forces to the next's
     template <int BS, bool REVERSE>
@@ -179,6 +181,7 @@ struct ByValue {
     __device__ __forceinline__ bool increments() const { return tn != tc; }
     __device__ __forceinline__ const DomDev *doms() const { return D; }
     __device__ __forceinline__ int materialize() const { return mat; }
+    __device__ __forceinline__ bool show() const { return shows != 0; }
     // the time state is read beside the gathers, and checked before any store
     static constexpr bool kTable = false;
 };
@@ -194,6 +197,7 @@ inline ByValue<N> by_value(const SetArgs &a, int nblocks)
     w.tc = a.tcs;
     w.tn = a.next ? a.next : a.tcs;
     w.mat = a.materialize;
+    w.shows = a.show;
     w.per = nblocks / N;
     w.stride = N > 1 ? a.records[1].fx_elem - a.records[0].fx_elem : 0;
     return w;
@@ -296,6 +300,8 @@ inline void launch_k(void (*kernel)(KArgs...), int grid, int block, cudaStream_t
 
 // start of a scattered mesh's cycle: time increment and node packing (node blocks)
 void launch_begin_packed(const SetArgs &a, int nblocks, Params P, cudaStream_t s);
+// a scattered mesh's corner forces to fx_elem, fy_elem, fz_elem (element blocks)
+void launch_show_corners(const SetArgs &a, int nblocks, cudaStream_t s);
 void launch_time_increment(TimeCtl *tcs, int ntc, Params P, cudaStream_t s, bool pdl = false);
 // u: the set's domains are unstructured (lmesh): 128-wide blocks, mesh
 // arrays read instead of structured indexing

@@ -145,8 +145,9 @@ struct DomDev {
     int *nodeCornerEll;
     // scattered unstructured meshes (pack_scattered_mesh, set.cu), else null:
     // node i's x, y, z, xd, yd, zd at nodePack + 8*i (two 32-byte sectors),
-    // packed at the start of every cycle; corner k of element e's force at
-    // cornerPack + 4*(8*e + k) (one sector); packedCornerEll is nodeCornerEll
+    // packed at the start of a graph's first cycle; corner k of element e's
+    // force at cornerPack + 4*(8*e + k) (one sector, its fourth value telling
+    // whether fx_elem has it, k_show_corners); packedCornerEll is nodeCornerEll
     // with 8*e + k in place of e + Ep*k
     double *nodePack, *cornerPack;
     int *packedCornerEll;

@@ -47,8 +47,9 @@ __global__ void k_run_continue(cudaGraphConditionalHandle h, const TimeCtl *tcs,
 
 int ensure_run_graph(lulesh_set *s)
 {
-    if (s->exec_run) return LULESH_OK;
-    int st = prepare_capture(s);
+    int st = refresh_graphs(s);
+    if (st != LULESH_OK || s->exec_run) return st;
+    st = prepare_capture(s);
     if (st != LULESH_OK) return st;
     cudaGraph_t g = nullptr;
     RCHECK(cudaGraphCreate(&g, 0));
@@ -71,7 +72,7 @@ int ensure_run_graph(lulesh_set *s)
         if (st == LULESH_OK) {
             int est = LULESH_OK;
             for (int c = 0; c < kCyclesPerTurn && est == LULESH_OK; ++c)
-                est = enqueue_cycle(s, c > 0);
+                est = enqueue_cycle(s, c > 0, c + 1 == kCyclesPerTurn);
             k_run_continue<<<1, 128, 0, s->stream>>>(h, s->dtc, s->njobs, s->run_ctl);
             cudaGraph_t captured = nullptr;
             const int cst = cuda_status(cudaStreamEndCapture(s->stream, &captured), "end capture");

@@ -183,6 +183,7 @@ static int pack_scattered_mesh(lulesh_set *s, const HostDomain &h, DomDev &D)
         if (c >= 0) c = 8 * (c % D.Ep) + c / D.Ep;
     LCHECK(cudaMemcpyAsync(D.packedCornerEll, at.data(), sizeof(int) * at.size(),
                            cudaMemcpyHostToDevice, s->stream));
+    LCHECK(cudaMemsetAsync(D.cornerPack, 0, sizeof(double) * corners, s->stream));
     LCHECK(cudaStreamSynchronize(s->stream));
     return LULESH_OK;
 }
@@ -374,12 +375,44 @@ void launch_begin(lulesh_set *s, cudaStream_t st, bool follows)
         launch_time_increment(s->dtc, s->njobs, s->P, st, s->pdl);
 }
 
-void launch_force_fp64(lulesh_set *s, cudaStream_t st)
+int show_corners(lulesh_set *s)
 {
-    launch_force(s->args(s->elem_blocks), s->n_elem_blocks, s->P, st, s->eb, s->unstructured);
+    if (!s->pack) return LULESH_OK;
+    launch_show_corners(s->args(s->elem_blocks), s->n_elem_blocks, s->stream);
+    return cuda_status(cudaGetLastError(), "corner forces");
 }
 
-int enqueue_cycle(lulesh_set *s, bool follows)
+int hide_corners(lulesh_set *s)
+{
+    if (!s->pack) return LULESH_OK;
+    const DomDev &D = s->hdoms[0];
+    return cuda_status(cudaMemsetAsync(D.cornerPack, 0, sizeof(double) * 32 * D.Ep, s->stream),
+                       "corner forces");
+}
+
+int refresh_graphs(lulesh_set *s)
+{
+    if (!s->pack || s->graphs_show == s->handed_out) return LULESH_OK;
+    LCHECK(cudaStreamSynchronize(s->stream));
+    drop_graph(s);
+    s->graphs_show = s->handed_out;
+    return LULESH_OK;
+}
+
+static bool is_corner_field(const char *name)
+{
+    return std::strcmp(name, "fx_elem") == 0 || std::strcmp(name, "fy_elem") == 0 ||
+           std::strcmp(name, "fz_elem") == 0;
+}
+
+void launch_force_fp64(lulesh_set *s, cudaStream_t st, bool last)
+{
+    SetArgs a = s->args(s->elem_blocks);
+    a.show = s->pack && s->handed_out && last;
+    launch_force(a, s->n_elem_blocks, s->P, st, s->eb, s->unstructured);
+}
+
+int enqueue_cycle(lulesh_set *s, bool follows, bool last)
 {
     if (s->flags & LULESH_FLAG_COMM_STAGED) return enqueue_cycle_staged(s);
     cudaStream_t st = s->stream;
@@ -388,7 +421,7 @@ int enqueue_cycle(lulesh_set *s, bool follows)
     if (mixed)
         launch_force_mixed(s->args(s->elem_blocks), s->n_elem_blocks, s->P, s->dcorner32, st);
     else
-        launch_force_fp64(s, st);
+        launch_force_fp64(s, st, last);
     if (mixed)
         launch_nodal_mixed(s->args(s->node_blocks), s->n_node_blocks, s->P, s->dcorner32, st);
     else
@@ -525,6 +558,8 @@ static int l2_node_window_on_device(lulesh_set *s)
 
 static int ensure_graph(lulesh_set *s)
 {
+    const int rst = refresh_graphs(s);
+    if (rst != LULESH_OK) return rst;
     if (s->graph_ready) return LULESH_OK;
     if (s->nparts > 1) {
         set_error("a part of a multi-GPU problem has no one-GPU cycle graph");
@@ -571,7 +606,7 @@ static int ensure_graph_k(lulesh_set *s, int k)
     int st = ensure_graph(s);
     if (st != LULESH_OK || (st = prepare_capture(s)) != LULESH_OK) return st;
     LCHECK(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
-    for (int c = 0; c < k && st == LULESH_OK; ++c) st = enqueue_cycle(s, c > 0);
+    for (int c = 0; c < k && st == LULESH_OK; ++c) st = enqueue_cycle(s, c > 0, c + 1 == k);
     cudaGraph_t g = nullptr;
     cudaError_t e = cudaStreamEndCapture(s->stream, &g);
     if (st != LULESH_OK) {
@@ -942,7 +977,7 @@ int lulesh_step(lulesh_set *s, int ncycles)
         }
         s->handed_out = true;
         for (int i = 0; i < ncycles; ++i) {
-            const int est = enqueue_cycle(s);
+            const int est = enqueue_cycle(s, /*follows=*/false, i + 1 == ncycles);
             if (est != LULESH_OK) return est;
         }
         return LULESH_OK;
@@ -1167,6 +1202,8 @@ int lulesh_get_field(lulesh_set *s, int d, const char *name, void *dst, size_t n
         set_error(std::string("field size/name mismatch: ") + name);
         return LULESH_INVALID_ARG;
     }
+    const int st = is_corner_field(name) ? show_corners(s) : LULESH_OK;
+    if (st != LULESH_OK) return st;
     LCHECK(cudaStreamSynchronize(s->stream));
     LCHECK(cudaMemcpy(dst, f.ptr, nbytes, cudaMemcpyDeviceToHost));
     return LULESH_OK;
@@ -1180,6 +1217,8 @@ int lulesh_set_field(lulesh_set *s, int d, const char *name, const void *src, si
         set_error(std::string("field size/name mismatch: ") + name);
         return LULESH_INVALID_ARG;
     }
+    const int st = is_corner_field(name) ? show_corners(s) : LULESH_OK;
+    if (st != LULESH_OK) return st;
     LCHECK(cudaStreamSynchronize(s->stream));
     LCHECK(cudaMemcpy(f.ptr, src, nbytes, cudaMemcpyHostToDevice));
     return LULESH_OK;
@@ -1189,6 +1228,13 @@ int lulesh_domain_view_get(lulesh_set *s, int d, lulesh_domain_view *o)
 {
     if (!s || !o || d < 0 || d >= s->ndom) return LULESH_INVALID_ARG;
     s->handed_out = true;
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    if (s->pack) LCHECK(cudaStreamIsCapturing(s->stream, &cs));
+    if (s->pack && cs == cudaStreamCaptureStatusNone) {  // up to date from here on
+        const int st = show_corners(s);
+        if (st != LULESH_OK) return st;
+        LCHECK(cudaStreamSynchronize(s->stream));
+    }
     const DomDev &D = s->hdoms[d];
     std::memset(o, 0, sizeof *o);
     o->numElem = D.numElem;

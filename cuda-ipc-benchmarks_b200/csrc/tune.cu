@@ -65,13 +65,19 @@ struct Snapshot {
         if (arena) cudaFree(arena);
         if (tc) cudaFree(tc);
     }
-    int save(const lulesh_set *s)
+    int save(lulesh_set *s)
     {
+        const int st = show_corners(s);
+        if (st != LULESH_OK) return st;
         TCHECK(device_malloc(&arena, s->arena_bytes));
         TCHECK(device_malloc(&tc, sizeof(TimeCtl) * s->njobs));
         return restore_into(s, true);
     }
-    int restore(const lulesh_set *s) { return restore_into(s, false); }
+    int restore(lulesh_set *s)
+    {
+        const int st = restore_into(s, false);
+        return st == LULESH_OK ? hide_corners(s) : st;
+    }
 
    private:
     int restore_into(const lulesh_set *s, bool save_dir)
