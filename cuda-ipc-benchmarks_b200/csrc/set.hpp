@@ -12,6 +12,23 @@
 #include "lulesh_b200.h"
 #include "lulesh_dev.h"
 
+// The fused subdomain cycle needs no PosVel sync (CommSyncPosVel,
+// lulesh-comms.cu:115-168).  The reference syncs because each rank sums a
+// shared node's forces as its own partial sum plus the neighbour's, in its
+// own order, so the two copies of the node can differ in the last bits.
+// Here every subdomain gathers every corner of its nodes, the neighbours'
+// included, in the single-domain corner order, and the node masses are the
+// single-domain sums: both copies of a shared node take the same operations
+// on the same values and stay equal bit for bit (checked against the single
+// domain, every field, 2^3, 3^3 and 4^3 subdomains, up to 400 cycles).
+// Leaving the copy out takes 2x2x2 of -s 50 from 349.5 to 343.9 us per
+// cycle.  1 puts the k_posvel_sync launch back in the fused cycle.  The
+// staged Comm* path keeps the reference's exchange; the parts of a
+// multi-GPU problem exchange POSVEL only when their driver asks for it.
+#ifndef LULESH_FUSED_POSVEL_SYNC
+#define LULESH_FUSED_POSVEL_SYNC 0
+#endif
+
 // The EOS of a subdomain set's fused cycle, and of a part of a multi-GPU
 // problem, reads a comm face's neighbour element in the neighbouring
 // subdomain or its proxy (k_eos<..., SUB>): the value k_monoq_ghost would
@@ -151,6 +168,8 @@ struct lulesh_set {
     {
         if (nparts > 1 || unstructured || (flags & (LULESH_FLAG_COMM_STAGED | LULESH_FLAG_MIXED)))
             return false;
+        // k_posvel_sync reads the job's time state before kinematics commits it
+        if (LULESH_FUSED_POSVEL_SYNC && tp > 1) return false;
         long long nodes = 0;
         for (const lulesh::DomDev &D : hdoms) nodes += D.numNode;
         return nodes <= lulesh::kInlineIncrementNodes;
