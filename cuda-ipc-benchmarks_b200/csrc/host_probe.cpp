@@ -139,4 +139,14 @@ long lulesh_host_lmesh_field(const char *path, int numReg, int balance, int cost
     return copy_field(d, name, out, cap);
 }
 
+// gather_sectors of an lmesh file, and whether the library runs it packed
+// (device memory permitting); -2 if the file is unreadable or malformed
+double lulesh_host_lmesh_sectors(const char *path, int *packed)
+{
+    lulesh::HostDomain d;
+    if (!lulesh::build_domain_lmesh(d, path, 1, 1, 1, nullptr)) return -2.0;
+    *packed = lulesh::scattered_mesh(d) && !d.nodeCornerEll.empty();
+    return lulesh::gather_sectors(d);
+}
+
 }  // extern "C"

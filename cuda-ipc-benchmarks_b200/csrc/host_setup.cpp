@@ -762,6 +762,25 @@ void build_domain_light(HostDomain &d, int nx, int numReg, int balance, int cost
     build_region_runs(d, numReg, balance);
 }
 
+double gather_sectors(const HostDomain &d)
+{
+    // sectors by the last gather that touched them
+    std::vector<long long> last((size_t)d.numNode / 4 + 1, -1);
+    long long sectors = 0, gathers = 0;
+    for (int k = 0; k < 8; ++k)
+        for (int e = 0; e < d.numElem; e += 32) {
+            for (int i = e; i < std::min(e + 32, d.numElem); ++i) {
+                long long &l = last[d.nodelist[(size_t)k * d.Ep + i] / 4];
+                sectors += l != gathers;
+                l = gathers;
+            }
+            ++gathers;
+        }
+    return gathers ? (double)sectors / (double)gathers : 0.0;
+}
+
+bool scattered_mesh(const HostDomain &d) { return gather_sectors(d) >= LULESH_PACK_SECTORS; }
+
 double origin_deltatime(int nx, int tp)
 {
     // the origin domain's volo[0] and einit, as build_domain computes them

@@ -97,6 +97,28 @@ void build_domain_light(HostDomain &d, int nx, int numReg, int balance, int cost
 bool build_domain_lmesh(HostDomain &d, const char *path, int numReg, int balance, int cost,
                         std::string *err);
 
+// Distinct 32-byte sectors a warp's gather of one corner of 32 elements
+// touches in a node array, on average: 9 in a box's own numbering, 32 when
+// neighbouring elements' nodes lie anywhere.
+double gather_sectors(const HostDomain &d);
+
+// A mesh whose gathers are scattered moves a 32-byte sector for every 8-byte
+// node or corner value; packed (DomDev::nodePack), two sectors hold a node's
+// six values and one a corner's three.  The line lies at 28 sectors a gather,
+// measured on B200 (us per cycle, lists against packed):
+//    9 sectors, a box's own order        -s 40 30.8 / 36.9   -s 64 63.6 / 96.3
+//   25, nodes shuffled in runs of 256    -s 40 39.2 / 39.1   -s 64 82.0 / 106.5
+//   30, all shuffled in runs of 1024     -s 40 56.6 / 41.2   -s 64 128 / 113
+//   32, random nodes                     -s 40 59.5 / 39.1   -s 64 152 / 107
+//   32, random nodes and elements        -s 40 74.0 / 42.9   -s 64 192 / 116
+// (near neighbours still meet in L1, so few shuffled meshes gain below it).  A
+// mesh of fewer than 28 elements is never scattered, one shuffled throughout is
+// from 343 elements (nx 7) up.
+#ifndef LULESH_PACK_SECTORS
+#define LULESH_PACK_SECTORS 28.0
+#endif
+bool scattered_mesh(const HostDomain &d);
+
 // The initial dt of a tp^3 problem of nx^3 subdomains: that of the domain
 // holding the origin (lulesh.cu:1189-1205), which every subdomain starts
 // from.

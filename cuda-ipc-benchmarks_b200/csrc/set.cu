@@ -114,42 +114,12 @@ struct DomPlace {
     int job, tp, col, row, plane, rank;
 };
 
-// Distinct 32-byte sectors a warp's gather of one corner of 32 elements
-// touches in a node array, on average: 9 in a box's own numbering, 32 when
-// neighbouring elements' nodes lie anywhere.
-static double gather_sectors(const HostDomain &h)
-{
-    long long sectors = 0, gathers = 0;
-    for (int k = 0; k < 8; ++k)
-        for (int e = 0; e < h.numElem; e += 32) {
-            int seen[32], n = 0;
-            for (int i = e; i < std::min(e + 32, h.numElem); ++i) {
-                const int s = h.nodelist[(size_t)k * h.Ep + i] / 4;
-                if (std::find(seen, seen + n, s) == seen + n) seen[n++] = s;
-            }
-            sectors += n;
-            ++gathers;
-        }
-    return gathers ? (double)sectors / (double)gathers : 0.0;
-}
-
-// A mesh whose gathers are scattered moves a 32-byte sector for every 8-byte
-// node or corner value; packed (DomDev::nodePack), two sectors hold a node's
-// six values and one a corner's three.  The line lies at 28 sectors a gather,
-// measured on B200 (us per cycle, lists against packed):
-//    9 sectors, a box's own order        -s 40 30.8 / 36.9   -s 64 63.6 / 96.3
-//   25, nodes shuffled in runs of 256    -s 40 39.2 / 39.1   -s 64 82.0 / 106.5
-//   30, all shuffled in runs of 1024     -s 40 56.6 / 41.2   -s 64 128 / 113
-//   32, random nodes                     -s 40 59.5 / 39.1   -s 64 152 / 107
-//   32, random nodes and elements        -s 40 74.0 / 42.9   -s 64 192 / 116
-// (near neighbours still meet in L1, so few shuffled meshes gain below it).
-#ifndef LULESH_PACK_SECTORS
-#define LULESH_PACK_SECTORS 28.0
-#endif
+// The packed copies of a mesh that gathers from scattered nodes (scattered_mesh,
+// host_setup.hpp)
 static int pack_scattered_mesh(lulesh_set *s, const HostDomain &h, DomDev &D)
 {
     if (!D.nodeCornerEll || (s->flags & LULESH_FLAG_MATERIALIZE) ||
-        gather_sectors(h) < LULESH_PACK_SECTORS)
+        !scattered_mesh(h))
         return LULESH_OK;
     const size_t N = D.numNode, nodes = 8 * N, corners = 32 * (size_t)D.Ep;  // doubles
     if (device_malloc(&s->pack, sizeof(double) * (nodes + corners) + sizeof(int) * 8 * N) !=
