@@ -83,13 +83,25 @@ constexpr int min_blocks(int minb, int bs)
     return (minb * 128 / bs) > 0 ? (minb * 128 / bs) : 1;
 }
 
-// Largest set (nodes) whose cycle kernels make the time increment: one wave of
-// the node update, 16 blocks of 128 on each of 148 SMs.  Beyond it every later
-// wave would make it again, to save a launch of 1% of the cycle.
-#ifndef LULESH_INLINE_NODES
-#define LULESH_INLINE_NODES (148 * 16 * 128)
-#endif
-constexpr long long kInlineIncrementNodes = LULESH_INLINE_NODES;
+// Largest set (nodes) whose cycle kernels make the time increment.  Every block
+// of the node update then makes it, to save a launch: 1 to 2 us of a cycle while
+// the blocks run in one wave, less and less beyond it.  B200, graphs of four
+// cycles, us per cycle, launch -> inside:
+//   one domain        -s 36 23.1 -> 21.7   50 31.0 -> 28.3   51 32.2 -> 31.6
+//                     60 44.8 -> 43.3   66 56.9 -> 56.0   70 66.2 -> 65.6
+//                     80 97.1 -> 97.0   90 137.2 -> 137.1   100 183.9 -> 185.0
+//   2x2x2 of          -s 18 27.2 -> 25.5   24 36.1 -> 32.7   25 38.0 -> 38.0
+//                     26 39.8 -> 40.3   28 46.6 -> 46.0   30 52.5 -> 52.8
+//                     32 58.9 -> 62.6
+//   3x3x3 of          -s 14 33.8 -> 32.5   18 45.7 -> 50.2   20 61.3 -> 60.4
+//   batches of -s 28  2 jobs 26.6 -> 25.5   4 32.8 -> 31.6   6 39.9 -> 41.4
+//                     8 47.2 -> 48.6   12 67.8 -> 69.4
+// One domain's line is past its gains of more than 1% (-s 66).  Sets of several
+// domains read neighbours' or their own records in those blocks as well; theirs
+// is where the first wave of that kernel ends, kNodalIncrMinBlocks blocks of 128
+// nodes on each of 148 SMs (2x2x2 of -s 24, five jobs of -s 28).
+constexpr long long kInlineIncrementNodes = 148 * 16 * 128;
+constexpr long long kInlineIncrementNodesMany = 148 * kNodalIncrMinBlocks * 128;
 
 // Block shapes the FP64 element kernels (force, kinematics, EOS) and the
 // nodal kernel are compiled for; a set's block tables use one of each.

@@ -207,7 +207,7 @@ static int rebuild(lulesh_server *s)
         long long nodes = 0;
         for (const DomDev &D : hd) nodes += D.numNode;
         const bool was_inline = s->inline_increment;
-        s->inline_increment = nodes <= kInlineIncrementNodes;
+        s->inline_increment = nodes <= kInlineIncrementNodesMany;
         if (s->exec && was_inline != s->inline_increment) {  // another kernel sequence
             cudaGraphExecDestroy(s->exec);
             s->exec = nullptr;

@@ -172,7 +172,8 @@ struct lulesh_set {
         if (LULESH_FUSED_POSVEL_SYNC && tp > 1) return false;
         long long nodes = 0;
         for (const lulesh::DomDev &D : hdoms) nodes += D.numNode;
-        return nodes <= lulesh::kInlineIncrementNodes;
+        return nodes <= (ndom == 1 ? lulesh::kInlineIncrementNodes
+                                   : lulesh::kInlineIncrementNodesMany);
     }
 
     // 2x2x2 subdomains in the order of their ranks, their corner forces at

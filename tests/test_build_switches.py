@@ -11,24 +11,31 @@ from conftest import PKG, REPO
 _PROBE = r"""
 #include <cstdio>
 #include "set.hpp"
-int main()
+static int rule(int tp, int ndom, int nx)
 {
     lulesh_set s;
     lulesh::DomDev D{};
-    D.numNode = 343;
-    s.hdoms.assign(1, D);
-    std::printf("%d", (int)s.inline_increment());
-    s.tp = 2;
-    s.hdoms.assign(8, D);
-    std::printf("%d\n", (int)s.inline_increment());
+    D.numNode = (nx + 1) * (nx + 1) * (nx + 1);
+    s.tp = tp;
+    s.ndom = ndom;
+    s.hdoms.assign(ndom, D);
+    return s.inline_increment();
+}
+int main()
+{
+    std::printf("%d%d %d%d %d%d %d%d %d%d\n", rule(1, 1, 6), rule(2, 8, 6), rule(1, 1, 66),
+                rule(1, 1, 67), rule(2, 8, 24), rule(2, 8, 25), rule(3, 27, 15), rule(3, 27, 16),
+                rule(1, 5, 28), rule(1, 6, 28));
     return 0;
 }
 """
 
 
-@pytest.mark.parametrize("flags,want", [((), "11"), (("-DLULESH_FUSED_POSVEL_SYNC=1",), "10")])
+@pytest.mark.parametrize("flags,want", [
+    ((), "11 10 10 10 10"), (("-DLULESH_FUSED_POSVEL_SYNC=1",), "10 10 00 00 10")])
 def test_increment_inside_the_kernels(tmp_path, flags, want):
-    """The PosVel sync kernel gates on the time state that the increment inside
+    """Which sets' kernels make the time increment: single domains to -s 66, sets
+    of several domains to one wave.  The PosVel sync kernel gates on the time state that the increment inside
     the kernels commits only after it: a build with that kernel keeps the
     increment's own launch in subdomain sets."""
     nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
