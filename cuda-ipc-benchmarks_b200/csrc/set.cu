@@ -573,13 +573,55 @@ static int ensure_graph_k(lulesh_set *s, int k)
     return LULESH_OK;
 }
 
-void drop_graph(lulesh_set *s)
+// Graph of k cycles none of which is the last of its call (launch_force_fp64)
+static int ensure_quiet(lulesh_set *s, lulesh_set::Quiet *q, int k)
 {
+    if (q->exec) return LULESH_OK;
+    int st = prepare_capture(s);
+    if (st != LULESH_OK) return st;
+    LCHECK(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
+    for (int c = 0; c < k && st == LULESH_OK; ++c) st = enqueue_cycle(s, c > 0, /*last=*/false);
+    cudaGraph_t g = nullptr;
+    const cudaError_t e = cudaStreamEndCapture(s->stream, &g);
+    if (st == LULESH_OK) st = cuda_status(e, "end capture");
+    if (st == LULESH_OK)
+        st = cuda_status(cudaGraphInstantiate(&q->exec, g, 0), "cudaGraphInstantiate");
+    if (g) cudaGraphDestroy(g);
+    return st;
+}
+
+// n launches of a graph of k cycles, the call's last ones where `last`
+static int launch_graphs(lulesh_set *s, cudaGraphExec_t exec, lulesh_set::Quiet *q, int k, int n,
+                         bool last)
+{
+    const bool quiet = s->pack && s->handed_out && n - last > 0;
+    const int st = quiet ? ensure_quiet(s, q, k) : LULESH_OK;
+    if (st != LULESH_OK) return st;
+    for (int i = 0; i < n; ++i)
+        LCHECK(cudaGraphLaunch(quiet && !(last && i + 1 == n) ? q->exec : exec, s->stream));
+    return LULESH_OK;
+}
+
+static void drop_quiet(lulesh_set::Quiet *q)
+{
+    if (q->exec) cudaGraphExecDestroy(q->exec);
+    q->exec = nullptr;
+}
+
+static void drop_graph_k(lulesh_set *s)
+{
+    drop_quiet(&s->quiet_k);
     if (s->exec_k) cudaGraphExecDestroy(s->exec_k);
     if (s->graph_k) cudaGraphDestroy(s->graph_k);
     s->exec_k = nullptr;
     s->graph_k = nullptr;
     s->graph_k_ready = false;
+}
+
+void drop_graph(lulesh_set *s)
+{
+    drop_graph_k(s);
+    drop_quiet(&s->quiet);
     if (s->exec) cudaGraphExecDestroy(s->exec);
     if (s->graph) cudaGraphDestroy(s->graph);
     s->exec = nullptr;
@@ -940,10 +982,11 @@ int lulesh_step(lulesh_set *s, int ncycles)
     const int k = cycles_per_launch(s, ncycles);
     if (k > 1 && ncycles >= k) {
         if ((st = ensure_graph_k(s, k)) != LULESH_OK) return st;
-        for (; ncycles >= k; ncycles -= k) LCHECK(cudaGraphLaunch(s->exec_k, s->stream));
+        st = launch_graphs(s, s->exec_k, &s->quiet_k, k, ncycles / k, ncycles % k == 0);
+        if (st != LULESH_OK) return st;
+        ncycles %= k;
     }
-    for (int i = 0; i < ncycles; ++i) LCHECK(cudaGraphLaunch(s->exec, s->stream));
-    return LULESH_OK;
+    return launch_graphs(s, s->exec, &s->quiet, 1, ncycles, true);
 }
 
 int lulesh_set_graph_cycles(lulesh_set *s, int k)
@@ -951,11 +994,7 @@ int lulesh_set_graph_cycles(lulesh_set *s, int k)
     if (!s || k < 1 || k > 100000) return LULESH_INVALID_ARG;
     if (k != s->graph_cycles) {
         LCHECK(cudaStreamSynchronize(s->stream));
-        if (s->exec_k) cudaGraphExecDestroy(s->exec_k);
-        if (s->graph_k) cudaGraphDestroy(s->graph_k);
-        s->exec_k = nullptr;
-        s->graph_k = nullptr;
-        s->graph_k_ready = false;
+        drop_graph_k(s);
         s->graph_cycles = k;
     }
     return LULESH_OK;

@@ -112,6 +112,11 @@ struct lulesh_set {
     cudaGraph_t graph_k = nullptr;
     cudaGraphExec_t exec_k = nullptr;
     bool graph_k_ready = false;
+    // the same for launches with others of the call after them, where that
+    // makes a difference (show_corners)
+    struct Quiet {
+        cudaGraphExec_t exec = nullptr;
+    } quiet, quiet_k;
     long long cycles_run = 0;  // by one-cycle launches (cycles_per_launch, set.cu)
     // graph_cycles taken at its word, whatever the set has run (lulesh_autotune,
     // whose trials do not count as cycles of the set)
@@ -222,11 +227,11 @@ void launch_begin(lulesh_set *s, cudaStream_t st, bool follows = false);
 // them into fx_elem, fy_elem and fz_elem, where callers read them, before the
 // library reads these itself; hide_corners: fx_elem ... are the newest, written
 // by the library.  Both on the set's stream.  Once a caller may read them without
-// the library's doing (handed_out) the force kernel of each graph's last cycle
-// writes both forms, a -s 40 mesh 35.3 -> 35.8 us per cycle on B200 in graphs of
-// four and 41.3 -> 42.9 a cycle by itself (a launch of show_corners after each
-// step: 41 -> 71, and 567 -> 590 for 16 cycles).  refresh_graphs drops the graphs
-// that were captured without.
+// the library's doing (handed_out) the force kernel of a call's last cycle writes
+// both forms: a -s 40 mesh on B200 goes from 564 to 568 us per call of 16 cycles
+// and from 41.4 to 42.7 for one cycle (with a launch of show_corners after each
+// call 590 and 71; both forms in each graph of four 575).  refresh_graphs drops the
+// graphs that were captured without.
 int show_corners(lulesh_set *s);
 int hide_corners(lulesh_set *s);
 int refresh_graphs(lulesh_set *s);

@@ -108,3 +108,29 @@ def test_captured_before_any_pointer(lulesh, sets):
     b.step(4)
     same(a, b)
     del g
+
+
+@pytest.mark.parametrize("k", [1, 3])
+def test_pointers_with_longer_graphs(lulesh, tmp_path, k):
+    """Several graph launches a call, whole or with a rest, before and after the
+    set takes four cycles a graph by itself, and a cap inside a graph."""
+    torch = pytest.importorskip("torch")
+    path = str(tmp_path / "m.lmesh")
+    rng = np.random.default_rng(9)
+    lmesh.write(path, lmesh.renumber(lmesh.box(9), rng.permutation(1000), rng.permutation(729)))
+    with lulesh.LuleshSet.from_mesh(path, its=320) as a, \
+            lulesh.LuleshSet.from_mesh(path, its=320, flags=lulesh.FLAG_MATERIALIZE) as b:
+        stream = torch.cuda.Stream()
+        a.set_stream(stream.cuda_stream)
+        w, n = _view(lulesh, a), b.field("fx_elem").size
+        views = [torch.as_tensor(_Array(getattr(w, f), n), device="cuda") for f in CORNERS]
+        a.set_graph_cycles(k)
+        for cycles in (7, 9, 2, 250, 8, 9, 1, 31, 7, 4):
+            a.step(cycles), b.step(cycles)
+            with torch.cuda.stream(stream):
+                got = [v.cpu().numpy() for v in views]
+            for f, g in zip(CORNERS, got):
+                assert np.array_equal(g, b.field(f)), (cycles, f)
+        assert a.state() == b.state() and a.state()["cycle"] == 320
+        del views
+        torch.cuda.synchronize()
