@@ -927,8 +927,8 @@ int lulesh_destroy(lulesh_set *s)
     part_release(s);
     if (s->dcorner32) cudaFree(s->dcorner32);
     if (s->pack) cudaFree(s->pack);
-    for (Block *b : {&s->tables_block, &s->ctl_block, &s->pinned_block, &s->arena_block})
-        s->give_back(b);
+    for (Block *b : {&s->tables_block, &s->ctl_block, &s->arena_block}) s->give_back(b);
+    block_put(&s->pinned_block);  // read back on the set's stream only
     if (s->own_stream && s->stream) cudaStreamDestroy(s->stream);
     delete s;
     return LULESH_OK;
