@@ -1,7 +1,7 @@
 // kernels.cu -- the per-cycle kernels of the LULESH Lagrange leapfrog step.
 //
-// One cycle is five launches (captured in CUDA graphs), four in sets of one
-// wave, whose kernels make the time increment themselves:
+// One cycle is five launches (captured in CUDA graphs), four in small sets,
+// whose kernels make the time increment themselves:
 //   time_increment  TimeIncrement on the device (lulesh.cu:1400-1461)
 //   force           CalcVolumeForceForElems_kernel (lulesh.cu:2080-2259):
 //                   stress + FB hourglass corner forces per element
@@ -120,9 +120,8 @@ __device__ __forceinline__ void time_increment(TimeCtl &T, const Params &P)
 //               force's errors
 //   EOS         as after a k_time_increment launch
 // Measured on B200 in graphs of 4 cycles, us per cycle with a launch -> inside:
-// -s 10 17.5 -> 16.7, -s 30 20.1 -> 18.6, -s 45 28.5 -> 26.7, -s 64 55.3 -> 54.7,
-// 2x2x2 of -s 12 23.1 -> 21.6; past one wave of the node update it costs more
-// than the launch (-s 100 188.8 -> 192.6, a 24-job batch 187 -> 196).
+// -s 10 17.5 -> 16.7, -s 30 20.1 -> 18.6, 2x2x2 of -s 12 23.1 -> 21.6; the sizes
+// around the lines up to which it is done: kInlineIncrementNodes, kernels.cuh.
 __device__ __forceinline__ bool increment_due(const TimeCtl &T, const Params &P)
 {
 #if LULESH_CHECKED
@@ -226,8 +225,8 @@ __device__ __forceinline__ void store_node(const DomDev &D, int n, double x, dou
 }
 
 // Start of a scattered mesh's cycle: the time increment, and every node's six
-// values side by side.  Packed anew each cycle, so what the caller wrote to
-// the node arrays between cycles counts.
+// values side by side.  The first cycle of a graph: what the caller wrote to the
+// node arrays before it counts, and the node update keeps both forms from there.
 __global__ void __launch_bounds__(kNodeBlock)
     k_begin_packed(const __grid_constant__ OneDomain w, Params P)
 {
@@ -282,9 +281,9 @@ void launch_show_corners(const SetArgs &a, int nblocks, cudaStream_t s)
 // Bound by the corner stores (192 B of the 290 B an element moves) and by
 // FP64 issue, about evenly: 63 us at -s 100 (1.0e6 elements) on B200, where
 // the stores and loads take 44 us at the measured copy rate and the 588
-// operations 32 us at the FP64 peak (70 us with the records read from memory).  The form that evaluated the reference's
-// expressions corner by corner took 125 us (934 operations, 254 registers,
-// 8 warps per SM).  All 48 gathers go out before any arithmetic: with the
+// operations 32 us at the FP64 peak (70 us with the records read from memory).
+// The form that evaluated the reference's expressions corner by corner took
+// 125 us (934 operations, 254 registers, 8 warps per SM).  All 48 gathers go out before any arithmetic: with the
 // velocities gathered component by component, where force_modal asks for
 // them, the kernel fits 128 registers (16 warps) but took 73 against 70 us,
 // and 312 against 272 us at -s 160.
@@ -859,7 +858,8 @@ void launch_nodal_update(const SetArgs &a, int nblocks, Params P, cudaStream_t s
 // Bound by latency and FP64 issue at 20 warps per SM: 43 us at -s 100
 // (1.0e6 elements) on B200, against 22 us for its 144 B per element at the
 // measured copy rate and 20 us for its 367 operations (51.6 us with the
-// records read from memory); 80 us with the reference's corner-by-corner expressions (649 operations, 168 registers).
+// records read from memory); 80 us with the reference's corner-by-corner
+// expressions (649 operations, 168 registers).
 // The velocities are gathered where kin_modal asks for them, after the volume
 // and length stores, at 96 registers (5 blocks); 6 us more at 4 blocks.  Up
 // front took 8 us more at 3 blocks, and between the coordinates and the volume
@@ -1250,7 +1250,7 @@ __global__ void __launch_bounds__(BS, min_blocks(kEosMinBlocks, BS))
     const DomDev &D = w.domain(blk.x);
     TimeCtl &T = w.time(D);
     const EosPlace place = eos_place<BS, SHARE>(D, blk.y / BS, lanes);
-    // before pdl_enter: the element, and in a set of one wave what the
+    // before pdl_enter: the element, and where the kernel is one wave what the
     // kinematics kernel does not write
     int zidx = 0;
     double mass_z, volo_z, q_old_z, v_z, e_temp, p_temp;

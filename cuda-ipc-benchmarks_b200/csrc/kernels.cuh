@@ -55,7 +55,7 @@ constexpr int kNodeBlock = 128;  // threads per block, node kernels
 #endif
 constexpr int kNodalMinBlocks = LULESH_NODAL_MINB;
 constexpr int kNodalFewMinBlocks = 16;
-// with the time increment's warp (small sets, one wave): registers for all
+// with the time increment's warp (small sets): registers for all
 // corner loads of a node at once beside its state (55; 16 B of spills at 8
 // blocks, and -s 30 16.6 us per cycle against 16.1, -s 60 42.7 against 41.7)
 #ifndef LULESH_NODAL_INCR_MINB
@@ -198,6 +198,8 @@ struct ByValue {
     static constexpr bool kTable = false;
 };
 using OneDomain = ByValue<1>;
+// (3x3x3, 27 records of 21 KB, would fit the 32,764 B a kernel may take; it reads
+// the table, not measured the other way)
 constexpr int kFewDomains = 8;
 using FewDomains = ByValue<kFewDomains>;
 
@@ -271,8 +273,8 @@ __device__ __forceinline__ int chk_index(long long i, long long n, TimeCtl *T, i
 //
 // What the previous kernel cannot write may be read before pdl_enter(), while
 // that kernel runs: the mesh's tables (node ids, corner slots, the EOS order)
-// in every set, and in sets of one wave, whose kernels are chains of loads, the
-// node update's own node and the EOS's element values.  Their last writer is
+// in every set, and in small sets, whose kernels are chains of loads, the node
+// update's own node and the EOS's element values.  Their last writer is
 // several grids back: every kernel waits before it lets its dependents in, so
 // all grids but the previous one have ended, and __ldcg takes their values
 // from L2.  Only kernels that always follow another kernel of the set do this:

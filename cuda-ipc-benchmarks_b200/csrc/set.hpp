@@ -121,8 +121,8 @@ struct lulesh_set {
     // graph_cycles taken at its word, whatever the set has run (lulesh_autotune,
     // whose trials do not count as cycles of the set)
     bool tuning = false;
-    // whole-run graph: a WHILE conditional node around one cycle
-    // (rungraph.cu); run_ctl[0] counts cycles, run_ctl[1] is the cap
+    // whole-run graph: a WHILE conditional node around a few cycles
+    // (rungraph.cu); run_ctl[0] counts its turns, run_ctl[1] is their cap
     cudaGraph_t graph_run = nullptr;
     cudaGraphExec_t exec_run = nullptr;
     unsigned long long *run_ctl = nullptr;
