@@ -287,9 +287,9 @@ void launch_show_corners(const SetArgs &a, int nblocks, cudaStream_t s)
 // velocities gathered component by component, where force_modal asks for
 // them, the kernel fits 128 registers (16 warps) but took 73 against 70 us,
 // and 312 against 272 us at -s 160.
-template <bool HG, Mesh M, bool TABLE>
+template <bool HG, Mesh M, bool TABLE, bool SHOW>
 __device__ __forceinline__ void force_one(const DomDev &D, bool active, TimeCtl &E, const Params &P,
-                                          int elem, int (&n)[8], bool show)
+                                          int elem, int (&n)[8])
 {
 #pragma unroll
     for (int i = 0; i < 8; ++i) n[i] = chk_index(n[i], D.numNode, &E, kChkNode);
@@ -318,7 +318,7 @@ __device__ __forceinline__ void force_one(const DomDev &D, bool active, TimeCtl 
     }
     if (!TABLE && !active) {
         // the graph's last cycle with work was an earlier one
-        if (M == Mesh::kPacked && show) show_element(D, elem);
+        if (SHOW) show_element(D, elem);
         return;
     }
     double fx[8], fy[8];  // held for cornerPack, whose corners take all three
@@ -336,16 +336,17 @@ __device__ __forceinline__ void force_one(const DomDev &D, bool active, TimeCtl 
                 for (int k = 0; k < 8; ++k) {
                     if (c == 0) fx[k] = f[k];
                     if (c == 1) fy[k] = f[k];
-                    if (c == 2) st4(p + 4 * k, fx[k], fy[k], f[k], show ? 0.0 : kNewCorner);
+                    if (c == 2) st4(p + 4 * k, fx[k], fy[k], f[k], SHOW ? 0.0 : kNewCorner);
                 }
             }
-            if (M != Mesh::kPacked || show)
+            if (M != Mesh::kPacked || SHOW)
                 CornerStore{D.fx_elem, D.fy_elem, D.fz_elem, elem, D.Ep}(c, f);
         },
         [&] { atomicMin(&E.bad_vol, elem); });
 }
 
-template <bool HG, int BS, Mesh M, class W>
+// SHOW (kPacked): the corner forces in both forms
+template <bool HG, int BS, Mesh M, class W, bool SHOW = false>
 __global__ void __launch_bounds__(BS, min_blocks(kForceMinBlocks, BS))
     k_force(const __grid_constant__ W w, Params P)
 {
@@ -364,16 +365,16 @@ __global__ void __launch_bounds__(BS, min_blocks(kForceMinBlocks, BS))
     if (W::kTable && !active) return;
     if (elem >= D.numElem) return;
     if (M == Mesh::kBox) elem_nodes<false>(D, elem, n);
-    force_one<HG, M, W::kTable>(D, active, w.next(D), P, elem, n, w.show());
+    force_one<HG, M, W::kTable, SHOW>(D, active, w.next(D), P, elem, n);
 }
 
-template <int BS, Mesh M, class W>
+template <int BS, Mesh M, bool SHOW = false, class W>
 static void launch_force_w(const W &w, bool pdl, int nblocks, Params P, cudaStream_t s)
 {
     if (P.hgcoef > 0.0)
-        launch_k(k_force<true, BS, M, W>, nblocks, BS, s, pdl, w, P);
+        launch_k(k_force<true, BS, M, W, SHOW>, nblocks, BS, s, pdl, w, P);
     else
-        launch_k(k_force<false, BS, M, W>, nblocks, BS, s, pdl, w, P);
+        launch_k(k_force<false, BS, M, W, SHOW>, nblocks, BS, s, pdl, w, P);
 }
 
 template <int BS>
@@ -388,7 +389,9 @@ void launch_force(const SetArgs &a, int nblocks, Params P, cudaStream_t s, int b
 {
     if (u) {  // an lmesh set is one domain
         const OneDomain w = by_value<1>(a, nblocks);
-        if (w.D[0].nodePack)
+        if (w.D[0].nodePack && a.show)
+            launch_force_w<kElemBlock, Mesh::kPacked, true>(w, a.pdl != 0, nblocks, P, s);
+        else if (w.D[0].nodePack)
             launch_force_w<kElemBlock, Mesh::kPacked>(w, a.pdl != 0, nblocks, P, s);
         else
             launch_force_w<kElemBlock, Mesh::kLists>(w, a.pdl != 0, nblocks, P, s);

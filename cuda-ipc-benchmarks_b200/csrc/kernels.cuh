@@ -132,7 +132,7 @@ struct SetArgs {
     // k_time_increment launch
     TimeCtl *next = nullptr;
     const CornerF32 *corner32 = nullptr;  // a mixed set's first domain (host side only)
-    int show = 0;  // a scattered mesh's corner forces to fx_elem ... too (force)
+    int show = 0;  // a scattered mesh's corner forces to fx_elem ... too (host side only)
 };
 
 // Where a block of a cycle kernel works: its domain's record, the time state
@@ -166,7 +166,6 @@ struct ManyDomains {
     __device__ __forceinline__ bool increments() const { return a.next != nullptr; }
     __device__ __forceinline__ const DomDev *doms() const { return a.doms; }
     __device__ __forceinline__ int materialize() const { return a.materialize; }
-    __device__ __forceinline__ bool show() const { return true; }
     // The node block table is already laid out last to first.  A job that is
     // done skips its gathers: the time state is read first.
     static constexpr bool kTable = true;
@@ -177,7 +176,7 @@ template <int N>
 struct ByValue {
     DomDev D[N];
     TimeCtl *tc, *tn;
-    int mat, shows;
+    int mat;
     int per;  // blocks per domain of this launch
     long long stride;  // doubles from one domain's corner forces to the next's
     template <int BS, bool REVERSE>
@@ -193,7 +192,6 @@ struct ByValue {
     __device__ __forceinline__ bool increments() const { return tn != tc; }
     __device__ __forceinline__ const DomDev *doms() const { return D; }
     __device__ __forceinline__ int materialize() const { return mat; }
-    __device__ __forceinline__ bool show() const { return shows != 0; }
     // the time state is read beside the gathers, and checked before any store
     static constexpr bool kTable = false;
 };
@@ -211,7 +209,6 @@ inline ByValue<N> by_value(const SetArgs &a, int nblocks)
     w.tc = a.tcs;
     w.tn = a.next ? a.next : a.tcs;
     w.mat = a.materialize;
-    w.shows = a.show;
     w.per = nblocks / N;
     w.stride = N > 1 ? a.records[1].fx_elem - a.records[0].fx_elem : 0;
     return w;

@@ -573,10 +573,10 @@ static int ensure_graph_k(lulesh_set *s, int k)
     return LULESH_OK;
 }
 
-// Graph of k cycles none of which is the last of its call (launch_force_fp64)
-static int ensure_quiet(lulesh_set *s, lulesh_set::Quiet *q, int k)
+// The same with no last cycle of a call in it (launch_force_fp64)
+static int ensure_quiet_k(lulesh_set *s, int k)
 {
-    if (q->exec) return LULESH_OK;
+    if (s->exec_quiet_k) return LULESH_OK;
     int st = prepare_capture(s);
     if (st != LULESH_OK) return st;
     LCHECK(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
@@ -585,32 +585,31 @@ static int ensure_quiet(lulesh_set *s, lulesh_set::Quiet *q, int k)
     const cudaError_t e = cudaStreamEndCapture(s->stream, &g);
     if (st == LULESH_OK) st = cuda_status(e, "end capture");
     if (st == LULESH_OK)
-        st = cuda_status(cudaGraphInstantiate(&q->exec, g, 0), "cudaGraphInstantiate");
+        st = cuda_status(cudaGraphInstantiate(&s->exec_quiet_k, g, 0), "cudaGraphInstantiate");
     if (g) cudaGraphDestroy(g);
     return st;
 }
 
-// n launches of a graph of k cycles, the call's last ones where `last`
-static int launch_graphs(lulesh_set *s, cudaGraphExec_t exec, lulesh_set::Quiet *q, int k, int n,
-                         bool last)
+// n launches of the k-cycle graph, the call's last ones where `last`.  The
+// difference is worth graphs of several cycles only: their second graph is
+// captured once in 256 cycles, the one-cycle graph's would be in a set's first
+// call (100 us, against 1.6 a cycle at -s 40 and none at -s 14).
+static int launch_graphs_k(lulesh_set *s, int k, int n, bool last)
 {
-    const bool quiet = s->pack && s->handed_out && n - last > 0;
-    const int st = quiet ? ensure_quiet(s, q, k) : LULESH_OK;
+    int st = ensure_graph_k(s, k);
+    const bool quiet = s->pack && s->handed_out && n > (last ? 1 : 0);
+    if (st == LULESH_OK && quiet) st = ensure_quiet_k(s, k);
     if (st != LULESH_OK) return st;
     for (int i = 0; i < n; ++i)
-        LCHECK(cudaGraphLaunch(quiet && !(last && i + 1 == n) ? q->exec : exec, s->stream));
+        LCHECK(cudaGraphLaunch(quiet && !(last && i + 1 == n) ? s->exec_quiet_k : s->exec_k,
+                               s->stream));
     return LULESH_OK;
-}
-
-static void drop_quiet(lulesh_set::Quiet *q)
-{
-    if (q->exec) cudaGraphExecDestroy(q->exec);
-    q->exec = nullptr;
 }
 
 static void drop_graph_k(lulesh_set *s)
 {
-    drop_quiet(&s->quiet_k);
+    if (s->exec_quiet_k) cudaGraphExecDestroy(s->exec_quiet_k);
+    s->exec_quiet_k = nullptr;
     if (s->exec_k) cudaGraphExecDestroy(s->exec_k);
     if (s->graph_k) cudaGraphDestroy(s->graph_k);
     s->exec_k = nullptr;
@@ -621,7 +620,6 @@ static void drop_graph_k(lulesh_set *s)
 void drop_graph(lulesh_set *s)
 {
     drop_graph_k(s);
-    drop_quiet(&s->quiet);
     if (s->exec) cudaGraphExecDestroy(s->exec);
     if (s->graph) cudaGraphDestroy(s->graph);
     s->exec = nullptr;
@@ -981,12 +979,12 @@ int lulesh_step(lulesh_set *s, int ncycles)
     if (st != LULESH_OK) return st;
     const int k = cycles_per_launch(s, ncycles);
     if (k > 1 && ncycles >= k) {
-        if ((st = ensure_graph_k(s, k)) != LULESH_OK) return st;
-        st = launch_graphs(s, s->exec_k, &s->quiet_k, k, ncycles / k, ncycles % k == 0);
+        st = launch_graphs_k(s, k, ncycles / k, ncycles % k == 0);
         if (st != LULESH_OK) return st;
         ncycles %= k;
     }
-    return launch_graphs(s, s->exec, &s->quiet, 1, ncycles, true);
+    for (int i = 0; i < ncycles; ++i) LCHECK(cudaGraphLaunch(s->exec, s->stream));
+    return LULESH_OK;
 }
 
 int lulesh_set_graph_cycles(lulesh_set *s, int k)

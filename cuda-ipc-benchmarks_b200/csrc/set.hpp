@@ -112,11 +112,9 @@ struct lulesh_set {
     cudaGraph_t graph_k = nullptr;
     cudaGraphExec_t exec_k = nullptr;
     bool graph_k_ready = false;
-    // the same for launches with others of the call after them, where that
-    // makes a difference (show_corners)
-    struct Quiet {
-        cudaGraphExec_t exec = nullptr;
-    } quiet, quiet_k;
+    // exec_k for launches with others of the call after them, where that makes a
+    // difference (show_corners)
+    cudaGraphExec_t exec_quiet_k = nullptr;
     long long cycles_run = 0;  // by one-cycle launches (cycles_per_launch, set.cu)
     // graph_cycles taken at its word, whatever the set has run (lulesh_autotune,
     // whose trials do not count as cycles of the set)
@@ -227,11 +225,11 @@ void launch_begin(lulesh_set *s, cudaStream_t st, bool follows = false);
 // them into fx_elem, fy_elem and fz_elem, where callers read them, before the
 // library reads these itself; hide_corners: fx_elem ... are the newest, written
 // by the library.  Both on the set's stream.  Once a caller may read them without
-// the library's doing (handed_out) the force kernel of a call's last cycle writes
-// both forms: a -s 40 mesh on B200 goes from 564 to 568 us per call of 16 cycles
-// and from 41.4 to 42.7 for one cycle (with a launch of show_corners after each
-// call 590 and 71; both forms in each graph of four 575).  refresh_graphs drops the
-// graphs that were captured without.
+// the library's doing (handed_out) the last cycle of a graph runs the force kernel
+// that writes both forms, but not in launches of longer graphs with others of
+// the call after them.  A -s 40 mesh on B200, us per call of 16 cycles: 614, 618
+// this way, 624 with both forms in each graph; a launch of show_corners after
+// each call adds 25.  refresh_graphs drops the graphs that were captured without.
 int show_corners(lulesh_set *s);
 int hide_corners(lulesh_set *s);
 int refresh_graphs(lulesh_set *s);
