@@ -6,7 +6,9 @@
 // creates set after set gets the blocks of the sets it has closed.
 //
 // Kept, per device: at most kCacheDeviceBytes of device memory and
-// kCachePinnedBytes of pinned memory, in at most kCacheBlocks blocks each.
+// kCachePinnedBytes of pinned memory, in at most kCacheBlocks blocks each.  A
+// set may get a block up to an eighth larger than it needs, or up to twice while
+// all that is in use beyond the need stays within kCacheSlackBytes.
 // Larger or later blocks go back to the driver at once, and so does all that is
 // kept when an allocation of the library's on the device fails (retry_trimmed)
 // or the program asks (lulesh_release_memory).  A block is put back only when
@@ -28,10 +30,11 @@ namespace lulesh {
 constexpr size_t kCacheDeviceBytes = size_t(512) << 20;
 constexpr size_t kCachePinnedBytes = size_t(1) << 20;
 constexpr size_t kCacheBlocks = 64;
+constexpr size_t kCacheSlackBytes = size_t(128) << 20;  // of blocks over an eighth too large
 
 struct Block {
     void *p = nullptr;
-    size_t bytes = 0;                // of the block, at least what was asked for
+    size_t bytes = 0, asked = 0;     // of the block, and of it what was asked for
     unsigned long long context = 0;  // id of the context it lives in, 0 not known
     int device = 0;
     bool pinned = false;

@@ -166,7 +166,8 @@ int lulesh_release_memory(void);
 
 /* Bytes of device memory a set of these jobs would hold (the admission
  * model of the serving loop).  A set made from the memory of a closed one may
- * hold up to an eighth and 4 KB a block more. */
+ * hold up to an eighth more, and up to twice as much while all sets on the
+ * device hold at most 128 MB more than this together. */
 size_t lulesh_footprint_bytes(const lulesh_job *jobs, int njobs, int tp);
 
 /* ---- stepping -------------------------------------------------------- */

@@ -106,10 +106,28 @@ int main()
     block_put(&a);
     block_put(&b);
     CHECK(g_used[0] == 300 * MB);
-    // a smaller set gets it only where it is not an eighth too large
-    CHECK(block_get(&a, 250 * MB) == cudaSuccess && a.p != p);
-    block_free(&a);
+    // a smaller set gets it, but never half empty
     CHECK(block_get(&a, 270 * MB) == cudaSuccess && a.p == p && a.bytes == 300 * MB);
+    block_put(&a);
+    CHECK(block_get(&a, 140 * MB) == cudaSuccess && a.p != p);
+    block_free(&a);
+    // and beyond an eighth only while all in use waste 128 MB at most
+    CHECK(block_get(&a, 170 * MB) == cudaSuccess && a.p != p);
+    block_free(&a);
+    CHECK(block_get(&a, 200 * MB) == cudaSuccess && a.p == p);
+    CHECK(block_get(&b, 200 * MB) == cudaSuccess);
+    block_put(&b);
+    CHECK(block_get(&b, 150 * MB) == cudaSuccess && b.bytes == 150 * MB);
+    block_put(&b);
+    CHECK(block_get(&b, 185 * MB) == cudaSuccess && b.bytes == 200 * MB);
+    block_free(&b);
+    lulesh_release_memory();
+    block_put(&a);
+    CHECK(g_used[0] == 300 * MB);
+    CHECK(block_get(&a, 200 * MB) == cudaSuccess && a.p == p);
+    block_put(&a);
+    // a block from the driver instead of the cache wastes nothing
+    CHECK(block_get(&a, 172 * MB) == cudaSuccess && a.p == p);
     block_put(&a);
     // block_free keeps nothing
     CHECK(block_get(&a, 300 * MB) == cudaSuccess && a.p == p);
