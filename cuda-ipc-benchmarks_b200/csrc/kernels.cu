@@ -283,10 +283,10 @@ void launch_show_corners(const SetArgs &a, int nblocks, cudaStream_t s)
 // the stores and loads take 44 us at the measured copy rate and the 588
 // operations 32 us at the FP64 peak (70 us with the records read from memory).
 // The form that evaluated the reference's expressions corner by corner took
-// 125 us (934 operations, 254 registers, 8 warps per SM).  All 48 gathers go out before any arithmetic: with the
-// velocities gathered component by component, where force_modal asks for
-// them, the kernel fits 128 registers (16 warps) but took 73 against 70 us,
-// and 312 against 272 us at -s 160.
+// 125 us (934 operations, 254 registers, 8 warps per SM).  All 48 gathers go out
+// before any arithmetic: with the velocities gathered component by component,
+// where force_modal asks for them, the kernel fits 128 registers (16 warps) but
+// took 73 against 70 us, and 312 against 272 us at -s 160.
 template <bool HG, Mesh M, bool TABLE, bool SHOW>
 __device__ __forceinline__ void force_one(const DomDev &D, bool active, TimeCtl &E, const Params &P,
                                           int elem, int (&n)[8])

@@ -328,9 +328,26 @@ void launch_begin(lulesh_set *s, cudaStream_t st, bool follows)
         launch_time_increment(s->dtc, s->njobs, s->P, st, s->pdl);
 }
 
+// The set's device for a call that may come with another one current: reading a
+// field and the like only copy otherwise.
+struct OnDevice {
+    int prev = -1;
+    explicit OnDevice(int device)
+    {
+        if (cudaGetDevice(&prev) != cudaSuccess || prev == device ||
+            cudaSetDevice(device) != cudaSuccess)
+            prev = -1;
+    }
+    ~OnDevice()
+    {
+        if (prev >= 0) cudaSetDevice(prev);
+    }
+};
+
 int show_corners(lulesh_set *s)
 {
     if (!s->pack) return LULESH_OK;
+    const OnDevice on(s->device);
     launch_show_corners(s->args(s->elem_blocks), s->n_elem_blocks, s->stream);
     return cuda_status(cudaGetLastError(), "corner forces");
 }
@@ -338,6 +355,7 @@ int show_corners(lulesh_set *s)
 int hide_corners(lulesh_set *s)
 {
     if (!s->pack) return LULESH_OK;
+    const OnDevice on(s->device);
     const DomDev &D = s->hdoms[0];
     return cuda_status(cudaMemsetAsync(D.cornerPack, 0, sizeof(double) * 32 * D.Ep, s->stream),
                        "corner forces");
